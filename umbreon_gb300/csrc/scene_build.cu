@@ -938,25 +938,85 @@ __device__ __forceinline__ float halfArea(float3 lo, float3 hi) {
   return ex * ey + ey * ez + ez * ex;
 }
 
-// Power-of-two scale s >= ext/255 (with slack) as its biased exponent.
-__device__ __forceinline__ uint32_t scaleExp(float ext) {
-  float x = ext * (1.0f / 255.0f) * (1.0f + 0x1.0p-20f);
-  if (!(x > 0x1.0p-126f)) x = 0x1.0p-126f;
-  const uint32_t bits = __float_as_uint(x);
-  uint32_t ex = bits >> 23;
-  if (bits & 0x7FFFFFu) ++ex;
-  return ex;
+// The 8-bit code of a plane stands for the float whose bits are 0x43, code,
+// 0, 0: 128 + code below 128, 2 code from 128 on (steps of 1, then 2, over
+// [128, 510]), so traversal decodes a plane with one byte permute.
+__device__ __forceinline__ float planeValue(int q) { return q < 128 ? float(128 + q) : float(2 * q); }
+
+// One axis of a wide node: origin p and scale s such that the codes 0 and 255
+// lie outside [lo, hi] with the padding that covers the rounding of the
+// traversal's plane distances (a few ulps of the coordinates).  The low byte
+// of s is `low`.
+__device__ __forceinline__ float axisPad(float lo, float hi) {
+  return fmaxf(fabsf(lo), fabsf(hi)) * 0x1.0p-22f;
+}
+__device__ __forceinline__ void axisScale(float lo, float hi, float& p, float& s, uint32_t low) {
+  const float pad = axisPad(lo, hi);
+  float x = (hi - lo + 8.0f * pad) * (1.0f / 381.0f);
+  if (!(x > 0x1.0p-100f)) x = 0x1.0p-100f;
+  s = __uint_as_float(((__float_as_uint(x) + 0x1FFu) & ~0xFFu) | low);
+  p = fmaf(-128.0f, s, lo - 3.0f * pad);
 }
 
-__device__ __forceinline__ void quantize(float lo, float hi, float p, float sc, uint32_t& qlo, uint32_t& qhi) {
-  int a = int(floorf((lo - p) / sc)), b = int(ceilf((hi - p) / sc));
-  a = max(0, min(255, a));
-  b = max(0, min(255, b));
-  while (a > 0 && fmaf(float(a), sc, p) > lo) --a;
-  while (b < 255 && fmaf(float(b), sc, p) < hi) ++b;
+// Codes of a child's [lo, hi] on an axis, rounded outward.  Evaluated with
+// fmaf as traversal does; lo and hi come padded.
+__device__ __forceinline__ void quantize(float lo, float hi, float p, float s, uint32_t& qlo, uint32_t& qhi) {
+  auto code = [](float x) { return int(x < 256.0f ? x - 128.0f : 0.5f * x); };
+  int a = max(0, min(255, code(floorf((lo - p) / s)))), b = max(0, min(255, code(ceilf((hi - p) / s))));
+  while (a > 0 && fmaf(planeValue(a), s, p) > lo) --a;
+  while (b < 255 && fmaf(planeValue(b), s, p) < hi) ++b;
   qlo = uint32_t(a);
   qhi = uint32_t(b);
 }
+
+// A wide node being written: child slots are added in order, the internal
+// children first.
+struct NodePack {
+  float3 p, s, pad;
+  uint32_t ql[6], qh[6];  // per axis two words of four codes
+  int count;
+
+  // lo, hi: the union of the children's boxes; imask, lmask: the slots of the
+  // internal and of the leaf children
+  __device__ __forceinline__ NodePack(float3 lo, float3 hi, uint32_t lmask) : count(0) {
+    axisScale(lo.x, hi.x, p.x, s.x, 0u);
+    axisScale(lo.y, hi.y, p.y, s.y, 0u);
+    axisScale(lo.z, hi.z, p.z, s.z, lmask);
+    pad = make_float3(axisPad(lo.x, hi.x), axisPad(lo.y, hi.y), axisPad(lo.z, hi.z));
+    for (int w = 0; w < 6; ++w) {  // empty slots: inverted boxes, left out by the masks
+      ql[w] = 0xFFFFFFFFu;
+      qh[w] = 0u;
+    }
+  }
+  __device__ __forceinline__ void put(int axis, uint32_t a, uint32_t b) {
+    const int sh = (count & 3) * 8;
+    const uint32_t hi = count >> 2, m = 0xFFu << sh;
+    for (int w = 0; w < 2; ++w) {
+      const bool here = uint32_t(w) == hi;
+      uint32_t &l = ql[2 * axis + w], &h = qh[2 * axis + w];
+      l = here ? (l & ~m) | (a << sh) : l;
+      h = here ? h | (b << sh) : h;
+    }
+  }
+  __device__ __forceinline__ void add(float3 lo, float3 hi) {
+    uint32_t a, b;
+    quantize(lo.x - pad.x, hi.x + pad.x, p.x, s.x, a, b);
+    put(0, a, b);
+    quantize(lo.y - pad.y, hi.y + pad.y, p.y, s.y, a, b);
+    put(1, a, b);
+    quantize(lo.z - pad.z, hi.z + pad.z, p.z, s.z, a, b);
+    put(2, a, b);
+    ++count;
+  }
+  __device__ __forceinline__ void store(float4* o, int childBase, uint32_t imask, int primBase) const {
+    auto f = [](uint32_t u) { return __uint_as_float(u); };
+    o[0] = make_float4(p.x, p.y, p.z, f((uint32_t(childBase) << 8) | imask));
+    o[1] = make_float4(s.x, s.y, s.z, __int_as_float(primBase));
+    o[2] = make_float4(f(ql[0]), f(ql[1]), f(ql[2]), f(ql[3]));
+    o[3] = make_float4(f(ql[4]), f(ql[5]), f(qh[0]), f(qh[1]));
+    o[4] = make_float4(f(qh[2]), f(qh[3]), f(qh[4]), f(qh[5]));
+  }
+};
 
 // SAH-optimal collapse of the binary tree into 8-wide nodes (the dynamic
 // programme of Ylitie, Karras and Laine, "Efficient Incoherent Ray Traversal
@@ -1082,17 +1142,20 @@ __device__ __forceinline__ int subtreePrims(const float4* nodes, int code, int* 
 // that becomes a wide node of the next level.
 __global__ void k_collapse_sah(const float4* bnodes, const uint8_t* dec, const int* workCode, const int* workWide,
                                int workCount, int* nextCode, int* nextWide, int* cursors, float4* wnodes,
-                               const uint32_t* srcRef, const float4* srcGeo, uint32_t* dstRef, float4* dstGeo) {
+                               uint2* wmeta, const uint32_t* srcRef, const float4* srcGeo, uint32_t* dstRef, float4* dstGeo) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= workCount) return;
   const int code = workCode[i];
   const int w = workWide[i];
-  int ec[8], et[8];  // child code, type: 0 leaf, 1 wide node
+  // child code, type: 0 leaf, 1 wide node.  Every element is set: an index the
+  // compiler evaluates ahead of its guard must not come from a value never written
+  int ec[8] = {}, et[8] = {};
   float3 elo[8], ehi[8];
   int en = 0;
+  for (int k = 0; k < 8; ++k) elo[k] = ehi[k] = make_float3(0.0f, 0.0f, 0.0f);
   // stack of (binary parent, side, slots)
   int sp = 0;
-  int stP[16], stS[16], stJ[16];
+  int stP[16] = {}, stS[16] = {}, stJ[16] = {};
   const int k8 = dec[8 * code + 7];
   stP[sp] = code; stS[sp] = 1; stJ[sp] = 8 - k8; ++sp;
   stP[sp] = code; stS[sp] = 0; stJ[sp] = k8; ++sp;
@@ -1118,7 +1181,7 @@ __global__ void k_collapse_sah(const float4* bnodes, const uint8_t* dec, const i
     stP[sp] = c; stS[sp] = 0; stJ[sp] = k; ++sp;
   }
   int nInt = 0, nLeaf = 0;
-  int prims[8][kWideLeafMax], pc[8];
+  int prims[8][kWideLeafMax] = {}, pc[8] = {};
   for (int k = 0; k < en; ++k) {
     if (et[k] == 1) {
       ++nInt;
@@ -1131,72 +1194,38 @@ __global__ void k_collapse_sah(const float4* bnodes, const uint8_t* dec, const i
   const int childBase = nInt ? atomicAdd(&cursors[0], nInt) : 0;
   const int primBase = nLeaf ? atomicAdd(&cursors[1], nLeaf) : 0;
   const int pushBase = nInt ? atomicAdd(&cursors[2], nInt) : 0;
-  float3 p = elo[0], hmax = ehi[0];
+  float3 lo = elo[0], hi = ehi[0];
   for (int k = 1; k < en; ++k) {
-    p = make_float3(fminf(p.x, elo[k].x), fminf(p.y, elo[k].y), fminf(p.z, elo[k].z));
-    hmax = make_float3(fmaxf(hmax.x, ehi[k].x), fmaxf(hmax.y, ehi[k].y), fmaxf(hmax.z, ehi[k].z));
+    lo = make_float3(fminf(lo.x, elo[k].x), fminf(lo.y, elo[k].y), fminf(lo.z, elo[k].z));
+    hi = make_float3(fmaxf(hi.x, ehi[k].x), fmaxf(hi.y, ehi[k].y), fmaxf(hi.z, ehi[k].z));
   }
-  const uint32_t exX = scaleExp(hmax.x - p.x), exY = scaleExp(hmax.y - p.y), exZ = scaleExp(hmax.z - p.z);
-  const float scX = __uint_as_float(exX << 23), scY = __uint_as_float(exY << 23), scZ = __uint_as_float(exZ << 23);
-  uint32_t meta[2] = {0u, 0u}, qlx[2] = {0u, 0u}, qly[2] = {0u, 0u}, qlz[2] = {0u, 0u};
-  uint32_t qhx[2] = {0u, 0u}, qhy[2] = {0u, 0u}, qhz[2] = {0u, 0u};
-  int order[8];
-  {
-    int o = 0;
-    for (int k = 0; k < en; ++k)
-      if (et[k] == 1) order[o++] = k;
-    for (int k = 0; k < en; ++k)
-      if (et[k] == 0) order[o++] = k;
+  const uint32_t imask = (1u << nInt) - 1u, lmask = ((1u << en) - 1u) & ~imask;
+  NodePack np(lo, hi, lmask);
+  // slots: internal children first (slot k -> node childBase + k), then leaves
+  for (int k = 0; k < en; ++k) {
+    if (!(et[k] == 1)) continue;
+    nextCode[pushBase + np.count] = ec[k];
+    nextWide[pushBase + np.count] = childBase + np.count;
+    np.add(elo[k], ehi[k]);
   }
-  int kInt = 0, off = 0;
-  for (int slot = 0; slot < en; ++slot) {
-    const int k = order[slot];
-    uint32_t a, b;
-    const int wd = slot >> 2, sh = (slot & 3) * 8;
-    quantize(elo[k].x, ehi[k].x, p.x, scX, a, b);
-    qlx[wd] |= a << sh;
-    qhx[wd] |= b << sh;
-    quantize(elo[k].y, ehi[k].y, p.y, scY, a, b);
-    qly[wd] |= a << sh;
-    qhy[wd] |= b << sh;
-    quantize(elo[k].z, ehi[k].z, p.z, scZ, a, b);
-    qlz[wd] |= a << sh;
-    qhz[wd] |= b << sh;
-    uint32_t m;
-    if (et[k] == 1) {
-      m = 0x80u | uint32_t(kInt);
-      nextCode[pushBase + kInt] = ec[k];
-      nextWide[pushBase + kInt] = childBase + kInt;
-      ++kInt;
-    } else {
-      const int cnt = pc[k];
-      m = (uint32_t(cnt) << 5) | uint32_t(off);
-      for (int q = 0; q < cnt; ++q) {
-        const int d = primBase + off + q, sidx = prims[k][q];
-        dstRef[d] = srcRef[sidx];
-        for (int f = 0; f < kLeafF4; ++f) dstGeo[kLeafF4 * d + f] = srcGeo[kLeafF4 * sidx + f];
-      }
-      off += cnt;
+  int off = 0;
+  uint32_t meta[2] = {0u, 0u};
+  for (int k = 0; k < en; ++k) {
+    if (et[k] == 1) continue;
+    const int cnt = pc[k];
+    const uint32_t m = ((uint32_t(cnt) << 5) | uint32_t(off)) << ((np.count & 3) * 8);
+    meta[0] |= np.count < 4 ? m : 0u;
+    meta[1] |= np.count < 4 ? 0u : m;
+    np.add(elo[k], ehi[k]);
+    for (int q = 0; q < cnt; ++q) {
+      const int d = primBase + off + q, sidx = prims[k][q];
+      dstRef[d] = srcRef[sidx];
+      for (int f = 0; f < kLeafF4; ++f) dstGeo[kLeafF4 * d + f] = srcGeo[kLeafF4 * sidx + f];
     }
-    meta[wd] |= m << sh;
+    off += cnt;
   }
-  for (int k = en; k < 8; ++k) {
-    const int wd = k >> 2, sh = (k & 3) * 8;
-    qlx[wd] |= 255u << sh;
-    qly[wd] |= 255u << sh;
-    qlz[wd] |= 255u << sh;
-  }
-  float4* o = wnodes + kWideF4 * w;
-  o[0] = make_float4(p.x, p.y, p.z,
-                     __uint_as_float(exX | (exY << 8) | (exZ << 16) | (uint32_t(nInt) << 24) | (uint32_t(en) << 28)));
-  o[1] = make_float4(__int_as_float(childBase), __int_as_float(primBase), __uint_as_float(meta[0]),
-                     __uint_as_float(meta[1]));
-  o[2] = make_float4(__uint_as_float(qlx[0]), __uint_as_float(qlx[1]), __uint_as_float(qly[0]),
-                     __uint_as_float(qly[1]));
-  o[3] = make_float4(__uint_as_float(qlz[0]), __uint_as_float(qlz[1]), __uint_as_float(qhx[0]),
-                     __uint_as_float(qhx[1]));
-  o[4] = make_float4(__uint_as_float(qhy[0]), __uint_as_float(qhy[1]), __uint_as_float(qhz[0]),
-                     __uint_as_float(qhz[1]));
+  np.store(wnodes + kWideF4 * w, childBase, imask, wmeta ? primBase : primBase - nInt);
+  if (wmeta) wmeta[w] = make_uint2(meta[0], meta[1]);
 }
 
 // Top-down collapse of the binary LBVH into 8-wide nodes, one level of wide
@@ -1209,7 +1238,7 @@ __global__ void k_collapse_sah(const float4* bnodes, const uint8_t* dec, const i
 __global__ void k_collapse(const float4* bnodes, const int2* brange, const float4* rootLo, const float4* rootHi,
                            const int* workCode, const int* workWide, int workCount, int leafMax, int* nextCode,
                            int* nextWide,
-                           int* cursors, float4* wnodes, const uint32_t* srcRef, const float4* srcGeo,
+                           int* cursors, float4* wnodes, uint2* wmeta, const uint32_t* srcRef, const float4* srcGeo,
                            uint32_t* dstRef, float4* dstGeo) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= workCount) return;
@@ -1255,75 +1284,39 @@ __global__ void k_collapse(const float4* bnodes, const int2* brange, const float
   const int childBase = nInt ? atomicAdd(&cursors[0], nInt) : 0;
   const int primBase = nLeaf ? atomicAdd(&cursors[1], nLeaf) : 0;
   const int pushBase = nInt ? atomicAdd(&cursors[2], nInt) : 0;
-  float3 p = elo[0], hmax = ehi[0];
+  float3 lo = elo[0], hi = ehi[0];
   for (int k = 1; k < en; ++k) {
-    p = make_float3(fminf(p.x, elo[k].x), fminf(p.y, elo[k].y), fminf(p.z, elo[k].z));
-    hmax = make_float3(fmaxf(hmax.x, ehi[k].x), fmaxf(hmax.y, ehi[k].y), fmaxf(hmax.z, ehi[k].z));
+    lo = make_float3(fminf(lo.x, elo[k].x), fminf(lo.y, elo[k].y), fminf(lo.z, elo[k].z));
+    hi = make_float3(fmaxf(hi.x, ehi[k].x), fmaxf(hi.y, ehi[k].y), fmaxf(hi.z, ehi[k].z));
   }
-  const uint32_t exX = scaleExp(hmax.x - p.x), exY = scaleExp(hmax.y - p.y), exZ = scaleExp(hmax.z - p.z);
-  const float scX = __uint_as_float(exX << 23), scY = __uint_as_float(exY << 23), scZ = __uint_as_float(exZ << 23);
-  uint32_t meta[2] = {0u, 0u}, qlx[2] = {0u, 0u}, qly[2] = {0u, 0u}, qlz[2] = {0u, 0u};
-  uint32_t qhx[2] = {0u, 0u}, qhy[2] = {0u, 0u}, qhz[2] = {0u, 0u};
-  // slot order: internal children first (slot k -> node childBase + k), then leaves
-  int order[8];
-  {
-    int o = 0;
-    for (int k = 0; k < en; ++k)
-      if (ec[k] >= 0 && countOf(ec[k]) > leafMax) order[o++] = k;
-    for (int k = 0; k < en; ++k)
-      if (!(ec[k] >= 0 && countOf(ec[k]) > leafMax)) order[o++] = k;
+  const uint32_t imask = (1u << nInt) - 1u, lmask = ((1u << en) - 1u) & ~imask;
+  NodePack np(lo, hi, lmask);
+  // slots: internal children first (slot k -> node childBase + k), then leaves
+  for (int k = 0; k < en; ++k) {
+    if (!(ec[k] >= 0 && countOf(ec[k]) > leafMax)) continue;
+    nextCode[pushBase + np.count] = ec[k];
+    nextWide[pushBase + np.count] = childBase + np.count;
+    np.add(elo[k], ehi[k]);
   }
-  int kInt = 0, off = 0;
-  for (int slot = 0; slot < en; ++slot) {
-    const int k = order[slot];
-    uint32_t a, b;
-    const int wd = slot >> 2, sh = (slot & 3) * 8;
-    quantize(elo[k].x, ehi[k].x, p.x, scX, a, b);
-    qlx[wd] |= a << sh;
-    qhx[wd] |= b << sh;
-    quantize(elo[k].y, ehi[k].y, p.y, scY, a, b);
-    qly[wd] |= a << sh;
-    qhy[wd] |= b << sh;
-    quantize(elo[k].z, ehi[k].z, p.z, scZ, a, b);
-    qlz[wd] |= a << sh;
-    qhz[wd] |= b << sh;
-    uint32_t m;
-    if (ec[k] >= 0 && countOf(ec[k]) > leafMax) {
-      m = 0x80u | uint32_t(kInt);
-      nextCode[pushBase + kInt] = ec[k];
-      nextWide[pushBase + kInt] = childBase + kInt;
-      ++kInt;
-    } else {
-      const int cnt = countOf(ec[k]);
-      const int first = ec[k] < 0 ? ~ec[k] : brange[ec[k]].x;
-      m = (uint32_t(cnt) << 5) | uint32_t(off);
-      for (int q = 0; q < cnt; ++q) {
-        const int d = primBase + off + q, sidx = first + q;
-        dstRef[d] = srcRef[sidx];
-        for (int f = 0; f < kLeafF4; ++f) dstGeo[kLeafF4 * d + f] = srcGeo[kLeafF4 * sidx + f];
-      }
-      off += cnt;
+  int off = 0;
+  uint32_t meta[2] = {0u, 0u};
+  for (int k = 0; k < en; ++k) {
+    if (ec[k] >= 0 && countOf(ec[k]) > leafMax) continue;
+    const int cnt = countOf(ec[k]);
+    const int first = ec[k] < 0 ? ~ec[k] : brange[ec[k]].x;
+    const uint32_t m = ((uint32_t(cnt) << 5) | uint32_t(off)) << ((np.count & 3) * 8);
+    meta[0] |= np.count < 4 ? m : 0u;
+    meta[1] |= np.count < 4 ? 0u : m;
+    np.add(elo[k], ehi[k]);
+    for (int q = 0; q < cnt; ++q) {
+      const int d = primBase + off + q, sidx = first + q;
+      dstRef[d] = srcRef[sidx];
+      for (int f = 0; f < kLeafF4; ++f) dstGeo[kLeafF4 * d + f] = srcGeo[kLeafF4 * sidx + f];
     }
-    meta[wd] |= m << sh;
+    off += cnt;
   }
-  // empty slots: qlo = 255 > qhi = 0 and meta 0 (never tested)
-  for (int k = en; k < 8; ++k) {
-    const int wd = k >> 2, sh = (k & 3) * 8;
-    qlx[wd] |= 255u << sh;
-    qly[wd] |= 255u << sh;
-    qlz[wd] |= 255u << sh;
-  }
-  float4* o = wnodes + kWideF4 * w;
-  o[0] = make_float4(p.x, p.y, p.z,
-                     __uint_as_float(exX | (exY << 8) | (exZ << 16) | (uint32_t(nInt) << 24) | (uint32_t(en) << 28)));
-  o[1] = make_float4(__int_as_float(childBase), __int_as_float(primBase), __uint_as_float(meta[0]),
-                     __uint_as_float(meta[1]));
-  o[2] = make_float4(__uint_as_float(qlx[0]), __uint_as_float(qlx[1]), __uint_as_float(qly[0]),
-                     __uint_as_float(qly[1]));
-  o[3] = make_float4(__uint_as_float(qlz[0]), __uint_as_float(qlz[1]), __uint_as_float(qhx[0]),
-                     __uint_as_float(qhx[1]));
-  o[4] = make_float4(__uint_as_float(qhy[0]), __uint_as_float(qhy[1]), __uint_as_float(qhz[0]),
-                     __uint_as_float(qhz[1]));
+  np.store(wnodes + kWideF4 * w, childBase, imask, wmeta ? primBase : primBase - nInt);
+  if (wmeta) wmeta[w] = make_uint2(meta[0], meta[1]);
 }
 
 template <class T>
@@ -1483,6 +1476,11 @@ ubr_status buildScene(Context* c, const ubr_scene_desc& d, Scene** out) {
     // the scene keeps the 8-wide nodes and the leaf records in wide order;
     // the binary tree and the Morton-ordered leaves are build temporaries
     if ((st = allocOwned(c, sc, sizeof(float4) * kWideF4 * nn, &pWide)) != UBR_OK) return fail(st);
+    // leaves of several primitives need their runs within a node's block; a
+    // tree of one-primitive leaves has slot k's primitive at primBase + k
+    void* pMeta = nullptr;
+    if (c->leafMax > 1 || c->collapse == 2)
+      if ((st = allocOwned(c, sc, sizeof(uint2) * nn, &pMeta)) != UBR_OK) return fail(st);
     if ((st = allocOwned(c, sc, sizeof(uint32_t) * n, &pRef2)) != UBR_OK) return fail(st);
     if ((st = allocOwned(c, sc, sizeof(float4) * kLeafF4 * n, &pGeo2)) != UBR_OK) return fail(st);
     if ((st = scratchGet(c, 50, sizeof(float4) * kNodeF4 * nn, &pNodes)) != UBR_OK) return fail(st);
@@ -1624,13 +1622,13 @@ ubr_status buildScene(Context* c, const ubr_scene_desc& d, Scene** out) {
         if (sah)
           k_collapse_sah<<<(count + 127) / 128, 128, 0, c->stream>>>(
               (const float4*)pNodes, (const uint8_t*)pDec, (const int*)pWc[cur], (const int*)pWw[cur], count,
-              (int*)pWc[cur ^ 1], (int*)pWw[cur ^ 1], (int*)pCur, (float4*)pWide, (const uint32_t*)pRef,
+              (int*)pWc[cur ^ 1], (int*)pWw[cur ^ 1], (int*)pCur, (float4*)pWide, (uint2*)pMeta, (const uint32_t*)pRef,
               (const float4*)pGeo, (uint32_t*)pRef2, (float4*)pGeo2);
         else
           k_collapse<<<(count + 127) / 128, 128, 0, c->stream>>>(
               (const float4*)pNodes, (const int2*)pRange, (const float4*)pLo, (const float4*)pHi,
               (const int*)pWc[cur], (const int*)pWw[cur], count, c->leafMax, (int*)pWc[cur ^ 1],
-              (int*)pWw[cur ^ 1], (int*)pCur, (float4*)pWide, (const uint32_t*)pRef, (const float4*)pGeo,
+              (int*)pWw[cur ^ 1], (int*)pCur, (float4*)pWide, (uint2*)pMeta, (const uint32_t*)pRef, (const float4*)pGeo,
               (uint32_t*)pRef2, (float4*)pGeo2);
         UBR_CUDA(c, cudaGetLastError());
         UBR_CUDA(c, cudaMemcpyAsync(hostCur, pCur, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -1646,6 +1644,7 @@ ubr_status buildScene(Context* c, const ubr_scene_desc& d, Scene** out) {
         return fail(setError(c, UBR_INVALID_ARGUMENT, "scene too large: more than 2^24 wide BVH nodes"));
     }
     v.wnodes = (const float4*)pWide;
+    v.wmeta = (const uint2*)pMeta;
     v.nodes = nullptr;
     v.leafRef = (const uint32_t*)pRef2;
     v.leafGeo = (const float4*)pGeo2;

@@ -157,10 +157,10 @@ UBR_D bool anyHitPhase(const TravScene& s, const Ray& r, const TriPre& pre, int 
 // (geomID, primID).
 constexpr float kSlabGrow = 1.0f + 0x1.0p-19f;
 
-// Byte b of word q as a float, without an integer->float conversion: place
-// the byte in the mantissa of 2^23 (byte permute) and subtract 2^23 (exact).
-UBR_D float byteToFloat(uint32_t q, int b) {
-  return __uint_as_float(__byte_perm(q, 0x4B000000u, 0x7540u + uint32_t(b))) - 8388608.0f;
+// Bound code b of word q as the float it stands for (ubr_internal.h): the
+// byte under the top byte 0x43, the low bytes zero.
+UBR_D float boundValue(uint32_t q, int b) {
+  return __uint_as_float(__byte_perm(q, 0x43000000u, 0x7044u | (uint32_t(b) << 8)));
 }
 
 // Packed pairs of floats for the slab test of two children at once:
@@ -189,12 +189,8 @@ UBR_D f2x mul2(f2x a, f2x b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
-// Bytes b and b+1 of q as a float pair (byteToFloat on both).
-UBR_D f2x bytePairToFloat2(uint32_t q, int b, f2x bias) {
-  return add2(pk2(__uint_as_float(__byte_perm(q, 0x4B000000u, 0x7540u + uint32_t(b))),
-                  __uint_as_float(__byte_perm(q, 0x4B000000u, 0x7540u + uint32_t(b + 1)))),
-              bias);
-}
+// Bounds b and b+1 of q as a float pair.
+UBR_D f2x boundPair(uint32_t q, int b) { return pk2(boundValue(q, b), boundValue(q, b + 1)); }
 
 // Slot of the nearest hit internal child (-1: none): the smallest key among
 // the hit slots, a key being the entry distance's bits with the slot in the
@@ -211,6 +207,77 @@ UBR_D int nearestChild(const float (&tmin)[8], uint32_t hitInt) {
     best = ((hitInt >> k) & 1u) ? min(best, key) : best;
   }
   return hitInt ? int(best & 7u) : -1;
+}
+
+// Slab test of a wide node's eight slots over [tnear, tmax]: the entry
+// distances, and the slots missed as the low eight bits (empty slots may
+// read as hit: the node's masks leave them out).
+UBR_D uint32_t nodeMisses(const float4& n0, const float4& n1, const float4& n2, const float4& n3, const float4& n4,
+                          const f3& org, const f3& inv, float tnear, float tmax, float (&tminP)[8]) {
+  const float sx = n1.x * inv.x, sy = n1.y * inv.y, sz = n1.z * inv.z;
+  const float ox = (n0.x - org.x) * inv.x, oy = (n0.y - org.y) * inv.y, oz = (n0.z - org.z) * inv.z;
+  // near/far planes per axis by the sign of the direction (swap lo/hi words)
+  const bool nx = inv.x < 0.0f, ny = inv.y < 0.0f, nz = inv.z < 0.0f;
+  const uint32_t qnx[2] = {nx ? __float_as_uint(n3.z) : __float_as_uint(n2.x),
+                           nx ? __float_as_uint(n3.w) : __float_as_uint(n2.y)};
+  const uint32_t qfx[2] = {nx ? __float_as_uint(n2.x) : __float_as_uint(n3.z),
+                           nx ? __float_as_uint(n2.y) : __float_as_uint(n3.w)};
+  const uint32_t qny[2] = {ny ? __float_as_uint(n4.x) : __float_as_uint(n2.z),
+                           ny ? __float_as_uint(n4.y) : __float_as_uint(n2.w)};
+  const uint32_t qfy[2] = {ny ? __float_as_uint(n2.z) : __float_as_uint(n4.x),
+                           ny ? __float_as_uint(n2.w) : __float_as_uint(n4.y)};
+  const uint32_t qnz[2] = {nz ? __float_as_uint(n4.z) : __float_as_uint(n3.x),
+                           nz ? __float_as_uint(n4.w) : __float_as_uint(n3.y)};
+  const uint32_t qfz[2] = {nz ? __float_as_uint(n3.x) : __float_as_uint(n4.z),
+                           nz ? __float_as_uint(n3.y) : __float_as_uint(n4.w)};
+  const f2x grow2 = pk2(kSlabGrow, kSlabGrow);
+  const f2x sx2 = pk2(sx, sx), sy2 = pk2(sy, sy), sz2 = pk2(sz, sz);
+  const f2x ox2 = pk2(ox, ox), oy2 = pk2(oy, oy), oz2 = pk2(oz, oz);
+  uint32_t gap[8];  // bits of tmax * grow - tmin per slot: sign clear = hit
+#pragma unroll
+  for (int k = 0; k < 8; k += 2) {
+    const int w = k >> 2, b = k & 3;
+    float tnx[2], tfx[2], tny[2], tfy[2], tnz[2], tfz[2];
+    up2(fma2(boundPair(qnx[w], b), sx2, ox2), tnx[0], tnx[1]);
+    up2(fma2(boundPair(qfx[w], b), sx2, ox2), tfx[0], tfx[1]);
+    up2(fma2(boundPair(qny[w], b), sy2, oy2), tny[0], tny[1]);
+    up2(fma2(boundPair(qfy[w], b), sy2, oy2), tfy[0], tfy[1]);
+    up2(fma2(boundPair(qnz[w], b), sz2, oz2), tnz[0], tnz[1]);
+    up2(fma2(boundPair(qfz[w], b), sz2, oz2), tfz[0], tfz[1]);
+    float tmx[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      tminP[k + j] = fmaxf(fmaxf(tnx[j], tny[j]), fmaxf(tnz[j], tnear));
+      tmx[j] = fminf(fminf(tfx[j], tfy[j]), fminf(tfz[j], tmax));
+    }
+    float g0, g1;
+    up2(fma2(pk2(tmx[0], tmx[1]), grow2, pk2(-tminP[k], -tminP[k + 1])), g0, g1);
+    gap[k] = __float_as_uint(g0);
+    gap[k + 1] = __float_as_uint(g1);
+  }
+  // slot mask of the hit children: the sign bytes of the eight gaps gathered
+  // into two words, their sign bits moved to bits 28-31 by one multiply
+  // (partial products land on distinct bits below 28, so nothing carries).
+  const uint32_t sx4 = __byte_perm(__byte_perm(gap[0], gap[1], 0x0073u), __byte_perm(gap[2], gap[3], 0x0073u), 0x5410u);
+  const uint32_t sy4 = __byte_perm(__byte_perm(gap[4], gap[5], 0x0073u), __byte_perm(gap[6], gap[7], 0x0073u), 0x5410u);
+  const uint32_t neg = (((sx4 & 0x80808080u) * 0x00204081u) >> 28) | ((((sy4 & 0x80808080u) * 0x00204081u) >> 24) & 0xF0u);
+  return neg;
+}
+
+// Primitives of the hit leaves as a mask over the node's block: the slots
+// themselves, or each leaf's run (meta byte count << 5 | offset).
+UBR_D uint32_t leafPrims(const TravScene& s, int node, uint32_t leafHit) {
+  if (!s.wmeta) return leafHit;
+  uint32_t primMask = 0;
+  if (leafHit) {
+    const uint2 meta = __ldg(&s.wmeta[node]);
+    for (; leafHit; leafHit &= leafHit - 1u) {
+      const int k = __ffs(leafHit) - 1;
+      const uint32_t m = __byte_perm(k < 4 ? meta.x : meta.y, 0u, 0x4440u | uint32_t(k & 3));
+      primMask |= ((1u << (m >> 5)) - 1u) << (m & 31u);
+    }
+  }
+  return primMask;
 }
 
 // Traversal state of one ray, resumable one node at a time (the persistent
@@ -304,70 +371,12 @@ UBR_D bool travStep(const TravScene& s, const Ray& r, const f3& inv, const TriPr
     n3 = __ldg(nd + 3);
     n4 = __ldg(nd + 4);
   }
-  const uint32_t hdr = __float_as_uint(n0.w);
-  const float sx = __uint_as_float((hdr & 0xFFu) << 23) * inv.x;
-  const float sy = __uint_as_float(((hdr >> 8) & 0xFFu) << 23) * inv.y;
-  const float sz = __uint_as_float(((hdr >> 16) & 0xFFu) << 23) * inv.z;
-  const int nInt = int((hdr >> 24) & 0xFu);
-  const float ox = (n0.x - r.org.x) * inv.x, oy = (n0.y - r.org.y) * inv.y, oz = (n0.z - r.org.z) * inv.z;
-  const uint32_t childBase = __float_as_uint(n1.x);
-  const int primBase = __float_as_int(n1.y);
-  const uint32_t meta0 = __float_as_uint(n1.z), meta1 = __float_as_uint(n1.w);
-  // near/far planes per axis by the sign of the direction (swap lo/hi words)
-  const bool nx = inv.x < 0.0f, ny = inv.y < 0.0f, nz = inv.z < 0.0f;
-  const uint32_t qnx[2] = {nx ? __float_as_uint(n3.z) : __float_as_uint(n2.x),
-                           nx ? __float_as_uint(n3.w) : __float_as_uint(n2.y)};
-  const uint32_t qfx[2] = {nx ? __float_as_uint(n2.x) : __float_as_uint(n3.z),
-                           nx ? __float_as_uint(n2.y) : __float_as_uint(n3.w)};
-  const uint32_t qny[2] = {ny ? __float_as_uint(n4.x) : __float_as_uint(n2.z),
-                           ny ? __float_as_uint(n4.y) : __float_as_uint(n2.w)};
-  const uint32_t qfy[2] = {ny ? __float_as_uint(n2.z) : __float_as_uint(n4.x),
-                           ny ? __float_as_uint(n2.w) : __float_as_uint(n4.y)};
-  const uint32_t qnz[2] = {nz ? __float_as_uint(n4.z) : __float_as_uint(n3.x),
-                           nz ? __float_as_uint(n4.w) : __float_as_uint(n3.y)};
-  const uint32_t qfz[2] = {nz ? __float_as_uint(n3.x) : __float_as_uint(n4.z),
-                           nz ? __float_as_uint(n3.y) : __float_as_uint(n4.w)};
-  const f2x bias2 = pk2(-8388608.0f, -8388608.0f), grow2 = pk2(kSlabGrow, kSlabGrow);
-  const f2x sx2 = pk2(sx, sx), sy2 = pk2(sy, sy), sz2 = pk2(sz, sz);
-  const f2x ox2 = pk2(ox, ox), oy2 = pk2(oy, oy), oz2 = pk2(oz, oz);
   float tminP[8];
-  uint32_t gap[8];  // bits of tmax * grow - tmin per slot: sign clear = hit
-#pragma unroll
-  for (int k = 0; k < 8; k += 2) {
-    const int w = k >> 2, b = k & 3;
-    float tnx[2], tfx[2], tny[2], tfy[2], tnz[2], tfz[2];
-    up2(fma2(bytePairToFloat2(qnx[w], b, bias2), sx2, ox2), tnx[0], tnx[1]);
-    up2(fma2(bytePairToFloat2(qfx[w], b, bias2), sx2, ox2), tfx[0], tfx[1]);
-    up2(fma2(bytePairToFloat2(qny[w], b, bias2), sy2, oy2), tny[0], tny[1]);
-    up2(fma2(bytePairToFloat2(qfy[w], b, bias2), sy2, oy2), tfy[0], tfy[1]);
-    up2(fma2(bytePairToFloat2(qnz[w], b, bias2), sz2, oz2), tnz[0], tnz[1]);
-    up2(fma2(bytePairToFloat2(qfz[w], b, bias2), sz2, oz2), tfz[0], tfz[1]);
-    float tmx[2];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      tminP[k + j] = fmaxf(fmaxf(tnx[j], tny[j]), fmaxf(tnz[j], r.tnear));
-      tmx[j] = fminf(fminf(tfx[j], tfy[j]), fminf(tfz[j], st.tmax));
-    }
-    float g0, g1;
-    up2(fma2(pk2(tmx[0], tmx[1]), grow2, pk2(-tminP[k], -tminP[k + 1])), g0, g1);
-    gap[k] = __float_as_uint(g0);
-    gap[k + 1] = __float_as_uint(g1);
-  }
-  // slot mask of the hit children: the sign bytes of the eight gaps gathered
-  // into two words, their sign bits moved to bits 28-31 by one multiply
-  // (partial products land on distinct bits below 28, so nothing carries).
-  const uint32_t sx4 = __byte_perm(__byte_perm(gap[0], gap[1], 0x0073u), __byte_perm(gap[2], gap[3], 0x0073u), 0x5410u);
-  const uint32_t sy4 = __byte_perm(__byte_perm(gap[4], gap[5], 0x0073u), __byte_perm(gap[6], gap[7], 0x0073u), 0x5410u);
-  const uint32_t neg = (((sx4 & 0x80808080u) * 0x00204081u) >> 28) | ((((sy4 & 0x80808080u) * 0x00204081u) >> 24) & 0xF0u);
-  const uint32_t hitMask = ~neg & 0xFFu;
-  const uint32_t hitInt = hitMask & ((1u << nInt) - 1u);
-  // each hit leaf's meta byte (count << 5 | offset) adds its primitives
-  uint32_t primMask = 0;
-  for (uint32_t leafHit = hitMask & ~hitInt; leafHit; leafHit &= leafHit - 1u) {
-    const int k = __ffs(leafHit) - 1;
-    const uint32_t m = __byte_perm(k < 4 ? meta0 : meta1, 0u, 0x4440u | uint32_t(k & 3));
-    primMask |= ((1u << (m >> 5)) - 1u) << (m & 31u);
-  }
+  const uint32_t neg = nodeMisses(n0, n1, n2, n3, n4, r.org, inv, r.tnear, st.tmax, tminP);
+  const uint32_t link = __float_as_uint(n0.w);  // childBase << 8 | internal slots
+  const int primBase = __float_as_int(n1.w);
+  const uint32_t hitInt = ~neg & link & 0xFFu;
+  uint32_t primMask = leafPrims(s, st.node, ~neg & __float_as_uint(n1.z) & 0xFFu);
   const int nearK = nearestChild(tminP, hitInt);
   // primitives of the hit leaves.  Binary any-hit queries (no filter) of a
   // scene of two analytic kinds split them by kind: all lanes of a warp test
@@ -433,10 +442,10 @@ UBR_D bool travStep(const TravScene& s, const Ray& r, const f3& inv, const TriPr
   if (nearK >= 0) {
     const uint32_t rest = hitInt & ~(1u << nearK);
     if (rest) {
-      if (st.sp < kStackDepth) st.stack[st.sp++] = (childBase << 8) | rest;
+      if (st.sp < kStackDepth) st.stack[st.sp++] = (link & ~0xFFu) | rest;
       else ++overflow;
     }
-    st.node = int(childBase) + nearK;
+    st.node = int(link >> 8) + nearK;
     return false;
   }
   if (st.sp == 0) return true;
@@ -485,8 +494,6 @@ __device__ bool traverseAnyInterleaved(const TravScene& s, const Ray& r, uint32_
   int node = start, sp = 0, pendBase = 0;
   uint32_t pendMask = 0, steps = 0;
   uint32_t stack[kStackDepth];
-  const bool nx = inv.x < 0.0f, ny = inv.y < 0.0f, nz = inv.z < 0.0f;
-  const f2x bias2 = pk2(-8388608.0f, -8388608.0f), grow2 = pk2(kSlabGrow, kSlabGrow);
   for (;;) {
     if (pendMask) {
       const int q = __ffs(pendMask) - 1;
@@ -506,69 +513,22 @@ __device__ bool traverseAnyInterleaved(const TravScene& s, const Ray& r, uint32_
     if (COUNT) ++cnt->nodes;
     const float4* nd = s.wnodes + kWideF4 * node;
     const float4 n0 = __ldg(nd), n1 = __ldg(nd + 1), n2 = __ldg(nd + 2), n3 = __ldg(nd + 3), n4 = __ldg(nd + 4);
-    const uint32_t hdr = __float_as_uint(n0.w);
-    const float sx = __uint_as_float((hdr & 0xFFu) << 23) * inv.x;
-    const float sy = __uint_as_float(((hdr >> 8) & 0xFFu) << 23) * inv.y;
-    const float sz = __uint_as_float(((hdr >> 16) & 0xFFu) << 23) * inv.z;
-    const int nInt = int((hdr >> 24) & 0xFu), nCh = int(hdr >> 28);
-    const float ox = (n0.x - r.org.x) * inv.x, oy = (n0.y - r.org.y) * inv.y, oz = (n0.z - r.org.z) * inv.z;
-    const uint32_t childBase = __float_as_uint(n1.x);
-    const int primBase = __float_as_int(n1.y);
-    const uint32_t meta0 = __float_as_uint(n1.z), meta1 = __float_as_uint(n1.w);
-    const uint32_t qnx[2] = {nx ? __float_as_uint(n3.z) : __float_as_uint(n2.x),
-                             nx ? __float_as_uint(n3.w) : __float_as_uint(n2.y)};
-    const uint32_t qfx[2] = {nx ? __float_as_uint(n2.x) : __float_as_uint(n3.z),
-                             nx ? __float_as_uint(n2.y) : __float_as_uint(n3.w)};
-    const uint32_t qny[2] = {ny ? __float_as_uint(n4.x) : __float_as_uint(n2.z),
-                             ny ? __float_as_uint(n4.y) : __float_as_uint(n2.w)};
-    const uint32_t qfy[2] = {ny ? __float_as_uint(n2.z) : __float_as_uint(n4.x),
-                             ny ? __float_as_uint(n2.w) : __float_as_uint(n4.y)};
-    const uint32_t qnz[2] = {nz ? __float_as_uint(n4.z) : __float_as_uint(n3.x),
-                             nz ? __float_as_uint(n4.w) : __float_as_uint(n3.y)};
-    const uint32_t qfz[2] = {nz ? __float_as_uint(n3.x) : __float_as_uint(n4.z),
-                             nz ? __float_as_uint(n3.y) : __float_as_uint(n4.w)};
-    const f2x sx2 = pk2(sx, sx), sy2 = pk2(sy, sy), sz2 = pk2(sz, sz);
-    const f2x ox2 = pk2(ox, ox), oy2 = pk2(oy, oy), oz2 = pk2(oz, oz);
-    float tminP[8], tmaxP[8];
-#pragma unroll
-    for (int k = 0; k < 8; k += 2) {
-      const int w = k >> 2, b = k & 3;
-      float tnx[2], tfx[2], tny[2], tfy[2], tnz[2], tfz[2];
-      up2(fma2(bytePairToFloat2(qnx[w], b, bias2), sx2, ox2), tnx[0], tnx[1]);
-      up2(fma2(bytePairToFloat2(qfx[w], b, bias2), sx2, ox2), tfx[0], tfx[1]);
-      up2(fma2(bytePairToFloat2(qny[w], b, bias2), sy2, oy2), tny[0], tny[1]);
-      up2(fma2(bytePairToFloat2(qfy[w], b, bias2), sy2, oy2), tfy[0], tfy[1]);
-      up2(fma2(bytePairToFloat2(qnz[w], b, bias2), sz2, oz2), tnz[0], tnz[1]);
-      up2(fma2(bytePairToFloat2(qfz[w], b, bias2), sz2, oz2), tfz[0], tfz[1]);
-      float tmx[2];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        tminP[k + j] = fmaxf(fmaxf(tnx[j], tny[j]), fmaxf(tnz[j], r.tnear));
-        tmx[j] = fminf(fminf(tfx[j], tfy[j]), fminf(tfz[j], r.tfar));
-      }
-      up2(mul2(pk2(tmx[0], tmx[1]), grow2), tmaxP[k], tmaxP[k + 1]);
-    }
-    uint32_t hitMask = 0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) hitMask |= tminP[k] <= tmaxP[k] ? (1u << k) : 0u;
-    hitMask &= (1u << nCh) - 1u;
-    const uint32_t hitInt = hitMask & ((1u << nInt) - 1u);
-    uint32_t primMask = 0;
-    for (uint32_t leafHit = hitMask & ~hitInt; leafHit; leafHit &= leafHit - 1u) {
-      const int k = __ffs(leafHit) - 1;
-      const uint32_t m = __byte_perm(k < 4 ? meta0 : meta1, 0u, 0x4440u | uint32_t(k & 3));
-      primMask |= ((1u << (m >> 5)) - 1u) << (m & 31u);
-    }
+    float tminP[8];
+    const uint32_t neg = nodeMisses(n0, n1, n2, n3, n4, r.org, inv, r.tnear, r.tfar, tminP);
+    const uint32_t link = __float_as_uint(n0.w);
+    const uint32_t hitInt = ~neg & link & 0xFFu;
+    const int primBase = __float_as_int(n1.w);
+    const uint32_t primMask = leafPrims(s, node, ~neg & __float_as_uint(n1.z) & 0xFFu);
     pendBase = primBase;
     pendMask = primMask;
     const int nearK = nearestChild(tminP, hitInt);
     if (nearK >= 0) {
       const uint32_t rest = hitInt & ~(1u << nearK);
       if (rest) {
-        if (sp < kStackDepth) stack[sp++] = (childBase << 8) | rest;
+        if (sp < kStackDepth) stack[sp++] = (link & ~0xFFu) | rest;
         else ++overflow;
       }
-      node = int(childBase) + nearK;
+      node = int(link >> 8) + nearK;
     } else if (sp == 0) {
       node = -1;
     } else {
@@ -595,28 +555,26 @@ UBR_D int boxStartNode(const TravScene& s, f3 lo, f3 hi) {
   for (int depth = 0; depth < kStackDepth; ++depth) {
     const float4* nd = s.wnodes + kWideF4 * node;
     const float4 n0 = __ldg(nd), n1 = __ldg(nd + 1), n2 = __ldg(nd + 2), n3 = __ldg(nd + 3), n4 = __ldg(nd + 4);
-    const uint32_t hdr = __float_as_uint(n0.w);
-    const float sx = __uint_as_float((hdr & 0xFFu) << 23);
-    const float sy = __uint_as_float(((hdr >> 8) & 0xFFu) << 23);
-    const float sz = __uint_as_float(((hdr >> 16) & 0xFFu) << 23);
-    const int nInt = int((hdr >> 24) & 0xFu), nCh = int(hdr >> 28);
+    const float sx = n1.x, sy = n1.y, sz = n1.z;
+    const uint32_t link = __float_as_uint(n0.w);
+    const uint32_t imask = link & 0xFFu, slots = imask | (__float_as_uint(n1.z) & 0xFFu);  // the low slots, without gaps
     int count = 0, only = -1;
-    for (int k = 0; k < nCh; ++k) {
+    for (int k = 0; (slots >> k) & 1u; ++k) {
       const int w = k >> 2, b = k & 3;
-      const float lx = fmaf(byteToFloat(__float_as_uint(w ? n2.y : n2.x), b), sx, n0.x);
-      const float ly = fmaf(byteToFloat(__float_as_uint(w ? n2.w : n2.z), b), sy, n0.y);
-      const float lz = fmaf(byteToFloat(__float_as_uint(w ? n3.y : n3.x), b), sz, n0.z);
-      const float hx = fmaf(byteToFloat(__float_as_uint(w ? n3.w : n3.z), b), sx, n0.x);
-      const float hy = fmaf(byteToFloat(__float_as_uint(w ? n4.y : n4.x), b), sy, n0.y);
-      const float hz = fmaf(byteToFloat(__float_as_uint(w ? n4.w : n4.z), b), sz, n0.z);
+      const float lx = fmaf(boundValue(__float_as_uint(w ? n2.y : n2.x), b), sx, n0.x);
+      const float ly = fmaf(boundValue(__float_as_uint(w ? n2.w : n2.z), b), sy, n0.y);
+      const float lz = fmaf(boundValue(__float_as_uint(w ? n3.y : n3.x), b), sz, n0.z);
+      const float hx = fmaf(boundValue(__float_as_uint(w ? n3.w : n3.z), b), sx, n0.x);
+      const float hy = fmaf(boundValue(__float_as_uint(w ? n4.y : n4.x), b), sy, n0.y);
+      const float hz = fmaf(boundValue(__float_as_uint(w ? n4.w : n4.z), b), sz, n0.z);
       if (lx <= hi.x && hx >= lo.x && ly <= hi.y && hy >= lo.y && lz <= hi.z && hz >= lo.z) {
         ++count;
         only = k;
       }
     }
     if (count == 0) return -1;
-    if (count > 1 || only >= nInt) return node;
-    node = int(__float_as_uint(n1.x)) + only;
+    if (count > 1 || !((imask >> only) & 1u)) return node;
+    node = int(link >> 8) + only;
   }
   return node;
 }
