@@ -9,11 +9,10 @@
 // and glossy reflection, variance-adaptive spp, ReSTIR spatial rounds
 // (integrator/pt2/pt2_reservoir.hpp, pt2_spatial.hpp).
 //
-// Up to eight lanes share a gather point, each taking every eighth sample (a
-// ReSTIR gather, whose reservoir streams the samples in order, runs one
-// thread per point); every stream is a pure function of (grid index, sample
-// index, pt1Seed), as in the reference, so the oracle draws the same samples
-// and the frames agree up to traversal float order.
+// The gather is a wavefront of kernels over the samples of many points; every
+// stream is a pure function of (grid index, sample index, pt1Seed), as in the
+// reference, so the oracle draws the same samples and the frames agree up to
+// traversal float order.
 #include <algorithm>
 
 #include <cub/device/device_select.cuh>
@@ -100,19 +99,15 @@ UBR_D f3 giEnvironment(const GiP& g, f3 wi) {
             e * g.amb.z * (g.ground.z + (g.sky.z - g.ground.z) * w)};
 }
 
-// A gather-ray hit as a path vertex.
-struct Vertex {
-  f3 rad, emitted, alb, P, N;
+// A path vertex's surface at a gather-ray hit (pt1EvalVertex,
+// pt1_gather.hpp:117-227): position, shading normal faced toward the ray
+// origin, reflectance kd * C, emission * pigment, and the origin and epsilon
+// of its shadow rays.  False on an outline primitive, which ends the path.
+struct VertexSurf {
+  f3 P, N, alb, C, So;
+  float eps, kd, emission;
 };
-
-// pt1EvalVertex (pt1_gather.hpp:117-227): its reflected, shadow-tested direct
-// light, its reflectance kd * C, position and shading normal faced toward the
-// ray origin; with `emit` its emission * pigment; with a stream (pt2) an
-// area light (radius > 0) gets one cone-jittered shadow ray drawn from it,
-// otherwise the light's centre ray.  Outline primitives end the path.
-template <int KM>
-UBR_D bool evalVertex(const DScene& s, const LightD* lights, int nLights, const Hit& h, f3 O, f3 wi, bool emit,
-                      uint32_t* r0, uint32_t* r1, Vertex& v, uint32_t& nee, uint32_t& ovf) {
+UBR_D bool vertexSurface(const DScene& s, const Hit& h, f3 O, f3 wi, VertexSurf& v) {
   const int kind = refKind(h.ref);
   const uint32_t prim = refPrim(h.ref);
   f3 C, NgSh, Ny;
@@ -140,25 +135,53 @@ UBR_D bool evalVertex(const DScene& s, const LightD* lights, int nLights, const 
     NgSh = Ny;
   }
   const ubr_material& m = s.mats[mi];
-  const float kd = diffuseWeight(m);
+  v.kd = diffuseWeight(m);
+  v.emission = m.emission;
   if (dot(Ny, wi) > 0.0f) Ny = neg(Ny);
   const f3 Py{O.x + wi.x * h.t, O.y + wi.y * h.t, O.z + wi.z * h.t};
   const float eps = selfIntersectEps(Py, wi, h.t);
   f3 ng = dot(NgSh, Ny) < 0.0f ? neg(NgSh) : NgSh;
   ng = safeNormalize(ng, Ny);
-  const f3 So{Py.x + ng.x * eps, Py.y + ng.y * eps, Py.z + ng.z * eps};
+  v.So = f3{Py.x + ng.x * eps, Py.y + ng.y * eps, Py.z + ng.z * eps};
+  v.eps = eps;
+  v.C = C;
+  v.alb = f3{v.kd * C.x, v.kd * C.y, v.kd * C.z};
+  v.P = Py;
+  v.N = Ny;
+  return true;
+}
+// its emission, when `emit` asks for it
+UBR_D f3 vertexEmission(const VertexSurf& v, bool emit) {
+  if (!(emit && v.emission > 0.0f)) return f3{0.0f, 0.0f, 0.0f};
+  return f3{v.emission * v.C.x, v.emission * v.C.y, v.emission * v.C.z};
+}
+
+// A gather-ray hit as a path vertex.
+struct Vertex {
+  f3 rad, emitted, alb, P, N;
+};
+
+// pt1EvalVertex with its shadow rays traced in place (the reflection passes):
+// the reflected, shadow-tested direct light; with a stream (pt2) an area
+// light (radius > 0) gets one cone-jittered shadow ray drawn from it,
+// otherwise the light's centre ray.
+template <int KM>
+UBR_D bool evalVertex(const DScene& s, const LightD* lights, int nLights, const Hit& h, f3 O, f3 wi, bool emit,
+                      uint32_t* r0, uint32_t* r1, Vertex& v, uint32_t& nee, uint32_t& ovf) {
+  VertexSurf vs;
+  if (!vertexSurface(s, h, O, wi, vs)) return false;
   const TravScene ts = travOf(s);
   f3 E{0.0f, 0.0f, 0.0f};
   for (int l = 0; l < nLights; ++l) {
     const LightD L = lights[l];
-    const float ndl = dot(Ny, L.L);
+    const float ndl = dot(vs.N, L.L);
     if (ndl <= 0.0f) continue;
     f3 dir = L.L;
     if (r0 && L.radius > 0.0f) {
       tea2(*r0, *r1);
       dir = sampleLightDir(L, u32ToUnorm(*r0), u32ToUnorm(*r1));
     }
-    Ray r{So, dir, eps, kInfF};
+    Ray r{vs.So, dir, vs.eps, kInfF};
     Hit hh;
     Count cnt;
     const float sh = traverse<false, KM, true>(ts, r, hh, ovf, &cnt, true) ? 0.0f : 1.0f;
@@ -167,12 +190,11 @@ UBR_D bool evalVertex(const DScene& s, const LightD* lights, int nLights, const 
     E.y += ndl * L.color.y * sh;
     E.z += ndl * L.color.z * sh;
   }
-  v.rad = f3{kd * C.x * E.x, kd * C.y * E.y, kd * C.z * E.z};
-  v.emitted = f3{0.0f, 0.0f, 0.0f};
-  if (emit && m.emission > 0.0f) v.emitted = f3{m.emission * C.x, m.emission * C.y, m.emission * C.z};
-  v.alb = f3{kd * C.x, kd * C.y, kd * C.z};
-  v.P = Py;
-  v.N = Ny;
+  v.rad = f3{vs.alb.x * E.x, vs.alb.y * E.y, vs.alb.z * E.z};
+  v.emitted = vertexEmission(vs, emit);
+  v.alb = vs.alb;
+  v.P = vs.P;
+  v.N = vs.N;
   return true;
 }
 
@@ -355,197 +377,6 @@ UBR_D float emissiveHitWeight(const EmitD& el, int kind, uint32_t prim, f3 O, f3
   return 1.0f;
 }
 
-// pt1GatherPoint (pt1_gather.hpp:268-523) at one grid point (px, py) of a
-// grid: E_stored = (1/spp) sum over cosine-hemisphere paths of the NEE
-// radiance (and, pt2, the MIS-weighted emission) at every vertex and the sky
-// where the path escapes, plus (pt2 with emitters) one emissive NEE draw per
-// sample at the origin; Russian roulette from the second vertex on; a first
-// bounce below the geometric horizon adds nothing.  First bounce: pt2 the
-// scrambled Sobol point (blue-noise section or per-point sequence), pt1
-// Hammersley + Cranley-Patterson when ld, else the tea2 stream.  Returns
-// (sum of E, number of first bounces that hit or fall below the horizon)
-// over the samples sFirst, sFirst + sStep, ... < spp; `half` gets the sum of
-// those among the first spp/2.
-// ReSTIR (rsv non-null, sFirst 0, sStep 1): every sample is also one
-// candidate streamed, in sample order, into the point's reservoir
-// (pt1_gather.hpp:287-297, 451-470, 486-499).
-template <int KM>
-UBR_D float4 gatherPoint(const GiP& g, const DScene& s, const LightD* lights, int nLights, f3 P, f3 N, f3 Ng,
-                         float tEps, uint32_t seed, uint32_t px, uint32_t py, int spp, int sFirst, int sStep,
-                         f3& half, uint32_t& rays, uint32_t& nee, uint32_t& ovf, float4* rsv = nullptr) {
-  const Frame3 f = frameFromNormal(N);
-  const float eps = selfIntersectEps(P, N, tEps);
-  const f3 O{P.x + N.x * eps, P.y + N.y * eps, P.z + N.z * eps};
-  const int maxB = g.bounces < 1 ? 1 : g.bounces;
-  float cpx = 0.0f, cpy = 0.0f;
-  if (g.ld) {
-    uint32_t c0 = seed, c1 = 0x9E3779B9u;
-    tea2(c0, c1);
-    cpx = u32ToUnorm(c0);
-    cpy = u32ToUnorm(c1);
-  }
-  // pt2MakePixelSampler: a section of the global sequence (blue noise) or
-  // an independent sequence per point
-  uint32_t idxBase = 0, sSeed = seed;
-  if (g.pt2 && g.pattern == 1) {
-    const uint32_t morton = (expandBits16(px) << 1) | expandBits16(py);
-    idxBase = __brev(owenHashBase4(__brev(morton), g.seedMix)) * g.sppPow2;
-    sSeed = g.seedMix;
-  }
-  const bool emitNee = g.pt2 && g.em.n > 0;
-  const TravScene ts = travOf(s);
-  f3 Esum{0.0f, 0.0f, 0.0f};
-  half = f3{0.0f, 0.0f, 0.0f};
-  int nOcc = 0;
-  uint32_t rs0 = seed ^ 0x52455354u, rs1 = 0x47490001u;
-  double rWSum = 0.0;
-  f3 rPos{0.0f, 0.0f, 0.0f}, rNrm{0.0f, 0.0f, 0.0f}, rRad{0.0f, 0.0f, 0.0f};
-  float rPHat = 0.0f;
-  for (int sI = sFirst; sI < spp; sI += sStep) {
-    uint32_t s0 = seed, s1 = uint32_t(sI + g.sampleOffset);
-    tea2(s0, s1);
-    float u1, u2;
-    if (g.pt2) {
-      sobol2D(idxBase + uint32_t(sI + g.sampleOffset), sSeed, u1, u2);
-    } else if (g.ld) {
-      u1 = float(sI) / float(spp) + cpx;
-      u2 = radicalInverse2(uint32_t(sI)) + cpy;
-      if (u1 >= 1.0f) u1 -= 1.0f;
-      if (u2 >= 1.0f) u2 -= 1.0f;
-    } else {
-      u1 = u32ToUnorm(s0);
-      u2 = u32ToUnorm(s1);
-    }
-    f3 wi = cosineSampleHemisphere(u1, u2, f);
-    const bool horizonOk = dot(wi, Ng) > 0.0f;
-    if (!horizonOk) ++nOcc;
-    const float cand0Cos = dot(wi, N);
-    f3 org = O;
-    float tnear = eps;
-    f3 thr{1.0f, 1.0f, 1.0f}, L{0.0f, 0.0f, 0.0f};
-    f3 candPos{0.0f, 0.0f, 0.0f}, candN{0.0f, 0.0f, 0.0f};
-    bool candValid = false;
-    for (int bnc = 1; horizonOk && bnc <= maxB; ++bnc) {
-      Ray r{org, wi, tnear, g.maxDist};
-      Hit h;
-      Count cnt;
-      traverse<false, KM>(ts, r, h, ovf, &cnt, false);
-      ++rays;
-      if (h.ref == kInvalid) {
-        const f3 env = giEnvironment(g, wi);
-        L.x += thr.x * env.x;
-        L.y += thr.y * env.y;
-        L.z += thr.z * env.z;
-        if (rsv && bnc == 1) {  // escaped: the candidate sits 1e7 along the segment
-          candPos = f3{O.x + wi.x * 1.0e7f, O.y + wi.y * 1.0e7f, O.z + wi.z * 1.0e7f};
-          candN = neg(wi);
-          candValid = true;
-        }
-        break;
-      }
-      if (bnc == 1) ++nOcc;
-      Vertex v;
-      if (!evalVertex<KM>(s, lights, nLights, h, org, wi, g.pt2 && g.emissive, g.pt2 ? &s0 : nullptr,
-                          g.pt2 ? &s1 : nullptr, v, nee, ovf)) {
-        if (rsv && bnc == 1) {  // absorbed by an outline: a zero-radiance candidate at the hit
-          candPos = f3{org.x + wi.x * h.t, org.y + wi.y * h.t, org.z + wi.z * h.t};
-          candN = neg(wi);
-          candValid = true;
-        }
-        break;
-      }
-      if (rsv && bnc == 1) {
-        candPos = v.P;
-        candN = v.N;
-        candValid = true;
-      }
-      float emW = 1.0f;
-      if (emitNee && bnc == 1)
-        emW = emissiveHitWeight(g.em, refKind(h.ref), refPrim(h.ref), org, wi, h.t, cand0Cos, h.Ng);
-      L.x += thr.x * (v.rad.x + emW * v.emitted.x);
-      L.y += thr.y * (v.rad.y + emW * v.emitted.y);
-      L.z += thr.z * (v.rad.z + emW * v.emitted.z);
-      if (bnc == maxB) break;
-      thr.x *= v.alb.x;
-      thr.y *= v.alb.y;
-      thr.z *= v.alb.z;
-      if (bnc >= 2) {
-        tea2(s0, s1);
-        float pc = fmaxf(thr.x, fmaxf(thr.y, thr.z));
-        pc = fminf(0.95f, fmaxf(0.05f, pc));
-        if (u32ToUnorm(s0) >= pc) break;
-        const float inv = 1.0f / pc;
-        thr.x *= inv;
-        thr.y *= inv;
-        thr.z *= inv;
-      }
-      tea2(s0, s1);
-      const Frame3 fv = frameFromNormal(v.N);
-      wi = cosineSampleHemisphere(u32ToUnorm(s0), u32ToUnorm(s1), fv);
-      const float epsV = selfIntersectEps(v.P, wi, h.t);
-      org = f3{v.P.x + v.N.x * epsV, v.P.y + v.N.y * epsV, v.P.z + v.N.z * epsV};
-      tnear = epsV;
-    }
-    if (emitNee) {
-      const f3 e = emissiveNee<KM>(g.em, s, P, N, Ng, tEps, s0, s1, ovf);
-      ++nee;
-      L.x += e.x;
-      L.y += e.y;
-      L.z += e.z;
-    }
-    if (g.clampLum > 0.0f) {
-      const float lum = 0.2126f * L.x + 0.7152f * L.y + 0.0722f * L.z;
-      if (lum > g.clampLum) {
-        const float k = g.clampLum / lum;
-        L.x *= k;
-        L.y *= k;
-        L.z *= k;
-      }
-    }
-    if (rsv) {  // RIS weight pi * lum(L): p_hat = lum(L) cos over the cosine pdf
-      float w = 0.0f, pHat = 0.0f;
-      if (candValid && cand0Cos > 0.0f) {
-        pHat = lumOf(L.x, L.y, L.z) * cand0Cos;
-        w = lumOf(L.x, L.y, L.z) * kPiF;
-      }
-      tea2(rs0, rs1);
-      rWSum += double(w);
-      if (w > 0.0f && double(u32ToUnorm(rs0)) * rWSum <= double(w)) {
-        rPos = candPos;
-        rNrm = candN;
-        rRad = L;
-        rPHat = pHat;
-      }
-    }
-    Esum.x += L.x;
-    Esum.y += L.y;
-    Esum.z += L.z;
-    if (sI < spp / 2) {
-      half.x += L.x;
-      half.y += L.y;
-      half.z += L.z;
-    }
-  }
-  if (rsv) {  // W = wSum / (M p_hat(selected)), M = every candidate
-    const float M = float(spp > 0 ? spp : 1);
-    const float W = (rPHat > 0.0f && rWSum > 0.0) ? float(rWSum / (double(M) * double(rPHat))) : 0.0f;
-    rsv[0] = make_float4(rPos.x, rPos.y, rPos.z, M);
-    rsv[1] = make_float4(rNrm.x, rNrm.y, rNrm.z, W);
-    rsv[2] = make_float4(rRad.x, rRad.y, rRad.z, 0.0f);
-  }
-  return make_float4(Esum.x, Esum.y, Esum.z, float(nOcc));
-}
-
-// gatherPt1Grid (pt1_gather.hpp:525-614): E and the hit fraction of every
-// eligible point of a grid (or of the points a list names), seeded
-// hashU32(pix ^ hashU32(pt1Seed)); the primary hit distance scales the
-// origin epsilon.  Points not eligible get zero (grid form; a list names
-// eligible points).  `listCount` (device) bounds the list when non-null.
-// LANES neighbouring threads share one point, lane k taking its samples
-// k, k + LANES, ...: a warp traces 32 / LANES points' sample fans from a few
-// origins (coherent node fetches, as the AO rays of one hit), and a short
-// list (the edge patch) still fills the GPU.  The lanes' sums meet in a
-// shuffle tree, so E is the same mean summed in another order.
 // point i of a grid in 2 x 2 quads (a warp's four points form one quad), the
 // odd column and row in row order: a bijection on [0, W H)
 UBR_D uint32_t quadPixel(uint32_t i, uint32_t W, uint32_t H) {
@@ -579,68 +410,546 @@ UBR_D uint32_t tilePixel4(uint32_t i, uint32_t W, uint32_t H) {
   return fh * W + j;
 }
 
-template <int KM, int LANES>
-__global__ void __launch_bounds__(128, 8) k_gather(GiP g, DScene s, const LightD* lights, int nLights, GiGrid grid,
-                                                const uint32_t* list, const uint32_t* listCount, uint32_t n, int spp,
-                                                float4* E) {
-  uint32_t rays = 0, nee = 0, ovf = 0;
-  const uint32_t cnt = listCount ? min(n, *listCount) : n;
-  const uint64_t total = uint64_t(cnt) * LANES, stride = uint64_t(gridDim.x) * blockDim.x;
-  // grid-stride over (point, lane) pairs; a warp's lanes run the same
-  // iterations, as the shuffles below need
-  for (uint64_t t0 = uint64_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u); t0 < total; t0 += stride) {
-    const uint64_t t = t0 + (threadIdx.x & 31u);
-    const uint32_t i = uint32_t(t / LANES);
-    const int lane = int(t % LANES);
-    float4 e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    f3 half{0.0f, 0.0f, 0.0f};
-    uint32_t pix = 0;
-    if (i < cnt) {
-      // several lanes per point: a warp's points form a quad; one thread per
-      // point (the reservoir gather): its 32 points form an 8 x 4 block
-      // (-15 % against quads along a row)
-      pix = list                ? list[i]
-            : LANES == 1        ? tilePixel4(i, uint32_t(grid.W), uint32_t(grid.H))
-                                : quadPixel(i, uint32_t(grid.W), uint32_t(grid.H));
-      const float4 ne = grid.ne[pix];
-      if (ne.w != 0.0f) {
-        const float4 pd = grid.pd[pix];
-        const f3 N{ne.x, ne.y, ne.z};
-        f3 Ng = N;
-        if (grid.ng) {
-          const float4 q = grid.ng[pix];
-          Ng = f3{q.x, q.y, q.z};
-        }
-        const uint32_t seed = hashU32(pix ^ g.seedMix);
-        const float tEps = pd.w > 0.0f ? pd.w : 1.0f;
-        e = gatherPoint<KM>(g, s, lights, nLights, f3{pd.x, pd.y, pd.z}, N, Ng, tEps, seed, pix % uint32_t(grid.W),
-                            pix / uint32_t(grid.W), spp, lane, LANES, half, rays, nee, ovf,
-                            LANES == 1 && g.rsv ? g.rsv + size_t(kRsvF4) * pix : nullptr);
+// ---- the gather (gatherPt1Grid + pt1GatherPoint, pt1_gather.hpp:268-614) ----
+// E_stored of a point = (1/spp) sum over cosine-hemisphere paths of the NEE
+// radiance (and, pt2, the MIS-weighted emission) at every vertex and the sky
+// where the path escapes, plus (pt2 with emitters) one emissive NEE draw per
+// sample at the origin; Russian roulette from the second vertex on; a first
+// bounce below the geometric horizon adds nothing.  First bounce: pt2 the
+// scrambled Sobol point (blue-noise section or per-point sequence), pt1
+// Hammersley + Cranley-Patterson when ld, else the tea2 stream.
+//
+// The paths run as a wavefront over chunks of points, one kernel per kind of
+// work, with the hits and the shadow rays compacted in between:
+//   k_gather_first    one thread per sample: draw, closest hit
+//   k_gather_vertex   one thread per hit: surface, shadow rays queued
+//   k_gather_shadow   one thread per shadow ray: any hit
+//   k_gather_resolve  one thread per hit: radiance, the next bounce's ray
+//   k_gather_next     one thread per path of a later bounce: closest hit
+//   k_gather_emit     (emitters) one thread per sample: emissive NEE
+//   k_gather_sum      the samples of a point, summed
+// One kernel that walks a path from its draw to its last shadow ray was bound
+// by instruction fetch (closest-hit and any-hit traversal, four intersectors
+// and the shading in one loop: 5 stalls on a missing instruction per issue)
+// with 6.5 of 32 lanes active (a lane's shadow rays waited for the others'
+// closest hits) and spilled 780 B per thread at 64 registers.  At the pt2
+// defaults (20 k ball-and-stick, 1920x1080 ss2: 12.1 M gather rays, 5.1 M
+// shadow rays) the gather and the edge patch take 24.8 -> 12.1 ms, on the 2 k
+// sphere 640x480 frame (8 samples per pixel) 0.57 -> 0.40 ms, with the same
+// frames bit for bit.  What bounds it now: k_gather_first is three quarters,
+// 74 % of its issue slots with 8.7 of 32 lanes (rays of one hemisphere fan end
+// at different depths); at most 64 registers (6 or 7 blocks per SM are 1-2 %
+// slower, 10 2.5 %).
+
+// Workspace of a chunk.  A sample has a slot: LANES neighbouring slots hold
+// one point's consecutive samples, 32 slots (a warp) the same LANES samples
+// of 32 / LANES points, and `iters` such warps follow one another per group
+// of points: all of a point's samples, or (a workspace too small for them) a
+// window of them, its sums carried to the next.  A record is the hit, then
+// the vertex, of one path.
+struct GiWave {
+  uint32_t* ctr;      // [0] listed points, [1] records, [2] shadow rays, [3] paths of the next bounce
+  float4* L;          // per slot: radiance, 1 = the first bounce hit something or fell below the horizon
+  float4* r[4];       // records: (t,u,v,ref)|(Ng,slot)|(dir,s0)|(org,s1), then
+                      //          (shadow origin,eps; eps < 0: ended)|(N,slot)|(kd C,s0)|(emission,s1)
+  float4* thr;        // several bounces: (throughput, hit t) and
+  float4* pos;        //   (position, -) of a record
+  float4* path[4];    // several bounces: (org,tnear)|(dir,slot)|(throughput,s0)|(s1 bits,-,-,-)
+  float4* shadow;     // (direction, record * nLights + light)
+  uint8_t* vis;       // per record and light: 1 = occluded
+  uint2* rng;         // emitters: per slot, the stream where its path ended
+  float4* cand;       // ReSTIR: per slot (candidate position, -) (normal, cos at the origin, < 0: none)
+  float4* carry;      // windows: kCarryF4 per lane of a group, the sums so far
+  uint32_t p0, nPts;  // the chunk's points [p0, p0 + nPts) of the list
+  int spp, logLanes, iters;
+  int it0, itEnd;     // the window's first iteration, and the iterations of a point
+};
+constexpr int kCarryF4 = 6;
+
+// Point (list position) and sample of a slot; false past the list or the
+// sample count.
+UBR_D bool slotSample(const GiWave& w, uint32_t slot, uint32_t& point, int& sample) {
+  const uint32_t row = slot >> 5, lane = slot & 31u, it = row % uint32_t(w.iters);
+  point = w.p0 + (row / uint32_t(w.iters)) * (32u >> w.logLanes) + (lane >> w.logLanes);
+  sample = int(((uint32_t(w.it0) + it) << w.logLanes) + (lane & ((1u << w.logLanes) - 1u)));
+  return point < min(w.ctr[0], w.p0 + w.nPts) && sample < w.spp;
+}
+UBR_D uint32_t waveSlots(const GiWave& w) {
+  const uint32_t P = 32u >> w.logLanes;
+  return (w.nPts + P - 1) / P * uint32_t(w.iters) * 32u;
+}
+
+// What a sample's path starts from.
+struct GatherOrigin {
+  f3 P, N, Ng, O;
+  float eps, tEps;
+  uint32_t seed;
+};
+UBR_D GatherOrigin gatherOrigin(const GiP& g, const GiGrid& grid, uint32_t pix) {
+  GatherOrigin o;
+  const float4 ne = grid.ne[pix], pd = grid.pd[pix];
+  o.P = f3{pd.x, pd.y, pd.z};
+  o.N = f3{ne.x, ne.y, ne.z};
+  o.Ng = o.N;
+  if (grid.ng) {
+    const float4 q = grid.ng[pix];
+    o.Ng = f3{q.x, q.y, q.z};
+  }
+  o.tEps = pd.w > 0.0f ? pd.w : 1.0f;
+  o.eps = selfIntersectEps(o.P, o.N, o.tEps);
+  o.O = f3{o.P.x + o.N.x * o.eps, o.P.y + o.N.y * o.eps, o.P.z + o.N.z * o.eps};
+  o.seed = hashU32(pix ^ g.seedMix);
+  return o;
+}
+
+// Direction of sample sI's first bounce.
+UBR_D f3 gatherDirection(const GiP& g, const GiGrid& grid, const GatherOrigin& o, uint32_t pix, int spp, int sI) {
+  float u1, u2;
+  if (g.pt2) {
+    // pt2MakePixelSampler: a section of the global sequence (blue noise) or
+    // an independent sequence per point
+    uint32_t idxBase = 0, sSeed = o.seed;
+    if (g.pattern == 1) {
+      const uint32_t px = pix % uint32_t(grid.W), py = pix / uint32_t(grid.W);
+      const uint32_t morton = (expandBits16(px) << 1) | expandBits16(py);
+      idxBase = __brev(owenHashBase4(__brev(morton), g.seedMix)) * g.sppPow2;
+      sSeed = g.seedMix;
+    }
+    sobol2D(idxBase + uint32_t(sI + g.sampleOffset), sSeed, u1, u2);
+  } else if (g.ld) {
+    uint32_t c0 = o.seed, c1 = 0x9E3779B9u;
+    tea2(c0, c1);
+    u1 = float(sI) / float(spp) + u32ToUnorm(c0);
+    u2 = radicalInverse2(uint32_t(sI)) + u32ToUnorm(c1);
+    if (u1 >= 1.0f) u1 -= 1.0f;
+    if (u2 >= 1.0f) u2 -= 1.0f;
+  } else {
+    uint32_t s0 = o.seed, s1 = uint32_t(sI + g.sampleOffset);
+    tea2(s0, s1);
+    u1 = u32ToUnorm(s0);
+    u2 = u32ToUnorm(s1);
+  }
+  return cosineSampleHemisphere(u1, u2, frameFromNormal(o.N));
+}
+
+// The eligible points of a grid in the order the gather walks them.
+__global__ void k_gather_list(GiGrid grid, uint32_t n, int single, uint32_t* list, uint32_t* count) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t pix = 0;
+  bool take = false;
+  if (i < n) {
+    // several lanes per point: a warp's points form a quad; one thread per
+    // point (the reservoir gather): its 32 points form an 8 x 4 block
+    pix = single ? tilePixel4(i, uint32_t(grid.W), uint32_t(grid.H)) : quadPixel(i, uint32_t(grid.W), uint32_t(grid.H));
+    take = grid.ne[pix].w != 0.0f;
+  }
+  int off;
+  const int base = warpPushBase(take, count, off);
+  if (take) list[base + off] = pix;
+}
+
+template <int KM>
+__global__ void __launch_bounds__(128, 8) k_gather_first(GiP g, DScene s, GiGrid grid, const uint32_t* list, GiWave w,
+                                                         int multi) {
+  const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t rays = 0, ovf = 0, point;
+  int sI;
+  bool push = false;
+  Hit h;
+  f3 O{0.0f, 0.0f, 0.0f}, wi{0.0f, 0.0f, 0.0f};
+  uint32_t s0 = 0, s1 = 0;
+  if (slot < waveSlots(w) && slotSample(w, slot, point, sI)) {
+    const uint32_t pix = list[point];
+    bool horizonOk;
+    float cos0, eps;
+    {
+      const GatherOrigin o = gatherOrigin(g, grid, pix);
+      wi = gatherDirection(g, grid, o, pix, w.spp, sI);
+      horizonOk = dot(wi, o.Ng) > 0.0f;
+      cos0 = dot(wi, o.N);
+      O = o.O;
+      eps = o.eps;
+      s0 = o.seed;
+    }
+    s1 = uint32_t(sI + g.sampleOffset);
+    float4 out = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+    f3 candPos{0.0f, 0.0f, 0.0f};
+    bool escaped = false;
+    if (horizonOk) {
+      traverse<false, KM>(travOf(s), Ray{O, wi, eps, g.maxDist}, h, ovf, nullptr, false);
+      rays = 1;
+      push = h.ref != kInvalid;
+      if (!push) {
+        const f3 env = giEnvironment(g, wi);
+        out = make_float4(env.x, env.y, env.z, 0.0f);
+        // escaped: the candidate sits 1e7 along the segment
+        escaped = true;
+        candPos = f3{O.x + wi.x * 1.0e7f, O.y + wi.y * 1.0e7f, O.z + wi.z * 1.0e7f};
       }
     }
-#pragma unroll
-    for (int o = LANES / 2; o > 0; o >>= 1) {
-      e.x += __shfl_xor_sync(0xFFFFFFFFu, e.x, o);
-      e.y += __shfl_xor_sync(0xFFFFFFFFu, e.y, o);
-      e.z += __shfl_xor_sync(0xFFFFFFFFu, e.z, o);
-      e.w += __shfl_xor_sync(0xFFFFFFFFu, e.w, o);
-      half.x += __shfl_xor_sync(0xFFFFFFFFu, half.x, o);
-      half.y += __shfl_xor_sync(0xFFFFFFFFu, half.y, o);
-      half.z += __shfl_xor_sync(0xFFFFFFFFu, half.z, o);
-    }
-    if (i < cnt && lane == 0) {
-      const float invN = 1.0f / float(spp > 0 ? spp : 1);
-      E[pix] = make_float4(e.x * invN, e.y * invN, e.z * invN, e.w * invN);
-      if (g.halfE) {
-        g.halfE[3 * size_t(pix)] = half.x;
-        g.halfE[3 * size_t(pix) + 1] = half.y;
-        g.halfE[3 * size_t(pix) + 2] = half.z;
-      }
+    w.L[slot] = out;
+    tea2(s0, s1);
+    if (w.rng) w.rng[slot] = make_uint2(s0, s1);
+    if (w.cand) {  // a hit's candidate position and normal come with its vertex
+      w.cand[2 * size_t(slot)] = make_float4(candPos.x, candPos.y, candPos.z, 0.0f);
+      w.cand[2 * size_t(slot) + 1] = make_float4(-wi.x, -wi.y, -wi.z, (push || escaped) ? cos0 : -1.0f);
     }
   }
+  int off;
+  const int q = warpPushBase(push, w.ctr + 1, off) + off;
+  if (push) {
+    w.r[0][q] = make_float4(h.t, h.u, h.v, __uint_as_float(h.ref));
+    w.r[1][q] = make_float4(h.Ng.x, h.Ng.y, h.Ng.z, __uint_as_float(slot));
+    w.r[2][q] = make_float4(wi.x, wi.y, wi.z, __uint_as_float(s0));
+    w.r[3][q] = make_float4(O.x, O.y, O.z, __uint_as_float(s1));
+    if (multi) w.thr[q] = make_float4(1.0f, 1.0f, 1.0f, h.t);
+  }
   warpCount(&g.stats[0], rays);
+  warpCount(g.overflow, ovf);
+}
+
+// Closest hits of the paths of bounce 2 and later.
+template <int KM>
+__global__ void __launch_bounds__(128, 8) k_gather_next(GiP g, DScene s, GiWave w) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t rays = 0, ovf = 0;
+  bool push = false;
+  Hit h;
+  float4 a, b, c;
+  uint32_t s1 = 0;
+  if (i < w.ctr[3]) {
+    a = w.path[0][i];
+    b = w.path[1][i];
+    traverse<false, KM>(travOf(s), Ray{ld3(a), ld3(b), a.w, g.maxDist}, h, ovf, nullptr, false);
+    rays = 1;
+    c = w.path[2][i];
+    s1 = __float_as_uint(w.path[3][i].x);
+    push = h.ref != kInvalid;
+    if (!push) {
+      const uint32_t slot = __float_as_uint(b.w);
+      const f3 env = giEnvironment(g, ld3(b));
+      float4 L = w.L[slot];
+      L.x += c.x * env.x;
+      L.y += c.y * env.y;
+      L.z += c.z * env.z;
+      w.L[slot] = L;
+      if (w.rng) w.rng[slot] = make_uint2(__float_as_uint(c.w), s1);
+    }
+  }
+  int off;
+  const int q = warpPushBase(push, w.ctr + 1, off) + off;
+  if (push) {
+    w.r[0][q] = make_float4(h.t, h.u, h.v, __uint_as_float(h.ref));
+    w.r[1][q] = make_float4(h.Ng.x, h.Ng.y, h.Ng.z, b.w);
+    w.r[2][q] = make_float4(b.x, b.y, b.z, c.w);
+    w.r[3][q] = make_float4(a.x, a.y, a.z, __uint_as_float(s1));
+    w.thr[q] = make_float4(c.x, c.y, c.z, h.t);
+  }
+  warpCount(&g.stats[0], rays);
+  warpCount(g.overflow, ovf);
+}
+
+// The hits' surfaces; a shadow ray per light a vertex faces, pushed light by
+// light, so a warp of shadow rays holds runs of one light.
+__global__ void __launch_bounds__(128) k_gather_vertex(GiP g, DScene s, const LightD* lights, int nLights, GiGrid grid,
+                                                       const uint32_t* list, GiWave w, int bounce) {
+  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool on = q < w.ctr[1];
+  uint32_t nee = 0, s0 = 0, s1 = 0;
+  bool live = false;
+  VertexSurf v;
+  f3 emitted{0.0f, 0.0f, 0.0f};
+  if (on) {
+    const float4 ra = w.r[0][q], rb = w.r[1][q], rc = w.r[2][q], rd = w.r[3][q];
+    Hit h;
+    h.t = ra.x;
+    h.u = ra.y;
+    h.v = ra.z;
+    h.ref = __float_as_uint(ra.w);
+    h.Ng = ld3(rb);
+    const f3 dir = ld3(rc), org = ld3(rd);
+    s0 = __float_as_uint(rc.w);
+    s1 = __float_as_uint(rd.w);
+    const uint32_t slot = __float_as_uint(rb.w);
+    live = vertexSurface(s, h, org, dir, v);
+    if (bounce == 1 && w.cand) {
+      float4* c = w.cand + 2 * size_t(slot);
+      if (live) {
+        c[0] = make_float4(v.P.x, v.P.y, v.P.z, 0.0f);
+        c[1] = make_float4(v.N.x, v.N.y, v.N.z, c[1].w);
+      } else {  // absorbed by an outline: a zero-radiance candidate at the hit
+        c[0] = make_float4(org.x + dir.x * h.t, org.y + dir.y * h.t, org.z + dir.z * h.t, 0.0f);
+      }
+    }
+    if (!live) {
+      w.r[0][q] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+      if (w.rng) w.rng[slot] = make_uint2(s0, s1);
+    } else {
+      const f3 em = vertexEmission(v, g.pt2 && g.emissive);
+      float emW = 1.0f;
+      if (g.pt2 && g.em.n > 0 && bounce == 1) {
+        uint32_t point;
+        int sI;
+        slotSample(w, slot, point, sI);
+        emW = emissiveHitWeight(g.em, refKind(h.ref), refPrim(h.ref), org, dir, h.t,
+                                dot(dir, ld3(grid.ne[list[point]])), h.Ng);
+      }
+      w.r[0][q] = make_float4(v.So.x, v.So.y, v.So.z, v.eps);
+      w.r[1][q] = make_float4(v.N.x, v.N.y, v.N.z, rb.w);
+      emitted = f3{emW * em.x, emW * em.y, emW * em.z};
+      if (w.pos) w.pos[q] = make_float4(v.P.x, v.P.y, v.P.z, 0.0f);
+    }
+  }
+  for (int l = 0; l < nLights; ++l) {
+    const LightD L = lights[l];
+    const bool lit = live && dot(v.N, L.L) > 0.0f;
+    f3 dir = L.L;
+    if (lit && g.pt2 && L.radius > 0.0f) {
+      tea2(s0, s1);
+      dir = sampleLightDir(L, u32ToUnorm(s0), u32ToUnorm(s1));
+    }
+    int off;
+    const uint32_t e = uint32_t(warpPushBase(lit, w.ctr + 2, off) + off);
+    if (lit) {
+      w.shadow[e] = make_float4(dir.x, dir.y, dir.z, __uint_as_float(q * uint32_t(nLights) + uint32_t(l)));
+      ++nee;
+    }
+  }
+  if (live) {
+    w.r[2][q] = make_float4(v.alb.x, v.alb.y, v.alb.z, __uint_as_float(s0));
+    w.r[3][q] = make_float4(emitted.x, emitted.y, emitted.z, __uint_as_float(s1));
+  }
+  warpCount(&g.stats[1], nee);
+}
+
+// Visibility of the queued shadow rays.
+template <int KM>
+__global__ void __launch_bounds__(128, (KM & kMaskMesh) ? 8 : 9) k_gather_shadow(GiP g, DScene s, int nLights, GiWave w) {
+  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t ovf = 0;
+  if (e < w.ctr[2]) {
+    const float4 d = w.shadow[e];
+    const uint32_t code = __float_as_uint(d.w);
+    const float4 o = w.r[0][code / uint32_t(nLights)];
+    Hit h;
+    w.vis[code] = traverse<false, KM, true>(travOf(s), Ray{ld3(o), ld3(d), o.w, kInfF}, h, ovf, nullptr, true) ? 1 : 0;
+  }
+  warpCount(g.overflow, ovf);
+}
+
+// The vertices' radiance into their samples, and the next bounce's rays
+// (Russian roulette from the second vertex on).
+__global__ void __launch_bounds__(128) k_gather_resolve(GiP g, const LightD* lights, int nLights, GiWave w, int bounce,
+                                                        int maxB) {
+  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+  bool push = false;
+  f3 thr{1.0f, 1.0f, 1.0f}, wi{0.0f, 0.0f, 0.0f}, org{0.0f, 0.0f, 0.0f};
+  float tnear = 0.0f;
+  uint32_t slot = 0, s0 = 0, s1 = 0;
+  if (q < w.ctr[1] && !(w.r[0][q].w < 0.0f)) {
+    const float4 rb = w.r[1][q], rc = w.r[2][q], rd = w.r[3][q];
+    const f3 N = ld3(rb), alb = ld3(rc), em = ld3(rd);
+    slot = __float_as_uint(rb.w);
+    s0 = __float_as_uint(rc.w);
+    s1 = __float_as_uint(rd.w);
+    f3 E{0.0f, 0.0f, 0.0f};
+    for (int l = 0; l < nLights; ++l) {
+      const LightD L = lights[l];
+      const float ndl = dot(N, L.L);
+      if (ndl <= 0.0f) continue;
+      const float sh = w.vis[size_t(q) * uint32_t(nLights) + uint32_t(l)] ? 0.0f : 1.0f;
+      E.x += ndl * L.color.x * sh;
+      E.y += ndl * L.color.y * sh;
+      E.z += ndl * L.color.z * sh;
+    }
+    float hitT = 0.0f;
+    if (w.thr) {
+      const float4 t4 = w.thr[q];
+      thr = ld3(t4);
+      hitT = t4.w;
+    }
+    float4 L = w.L[slot];
+    L.x += thr.x * (alb.x * E.x + em.x);
+    L.y += thr.y * (alb.y * E.y + em.y);
+    L.z += thr.z * (alb.z * E.z + em.z);
+    w.L[slot] = L;
+    push = bounce < maxB;
+    if (push) {
+      thr.x *= alb.x;
+      thr.y *= alb.y;
+      thr.z *= alb.z;
+      if (bounce >= 2) {
+        tea2(s0, s1);
+        float pc = fmaxf(thr.x, fmaxf(thr.y, thr.z));
+        pc = fminf(0.95f, fmaxf(0.05f, pc));
+        if (u32ToUnorm(s0) >= pc) {
+          push = false;
+        } else {
+          const float inv = 1.0f / pc;
+          thr.x *= inv;
+          thr.y *= inv;
+          thr.z *= inv;
+        }
+      }
+    }
+    if (push) {
+      tea2(s0, s1);
+      wi = cosineSampleHemisphere(u32ToUnorm(s0), u32ToUnorm(s1), frameFromNormal(N));
+      const f3 P = ld3(w.pos[q]);
+      tnear = selfIntersectEps(P, wi, hitT);
+      org = f3{P.x + N.x * tnear, P.y + N.y * tnear, P.z + N.z * tnear};
+    } else if (w.rng) {
+      w.rng[slot] = make_uint2(s0, s1);
+    }
+  }
+  if (bounce >= maxB) return;
+  int off;
+  const int i = warpPushBase(push, w.ctr + 3, off) + off;
+  if (push) {
+    w.path[0][i] = make_float4(org.x, org.y, org.z, tnear);
+    w.path[1][i] = make_float4(wi.x, wi.y, wi.z, __uint_as_float(slot));
+    w.path[2][i] = make_float4(thr.x, thr.y, thr.z, __uint_as_float(s0));
+    w.path[3][i] = make_float4(__uint_as_float(s1), 0.0f, 0.0f, 0.0f);
+  }
+}
+
+// One emissive NEE draw per sample at its origin, continuing its stream.
+template <int KM>
+__global__ void __launch_bounds__(128) k_gather_emit(GiP g, DScene s, GiGrid grid, const uint32_t* list, GiWave w) {
+  const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t nee = 0, ovf = 0, point;
+  int sI;
+  if (slot < waveSlots(w) && slotSample(w, slot, point, sI)) {
+    const GatherOrigin o = gatherOrigin(g, grid, list[point]);
+    uint2 r = w.rng[slot];
+    const f3 e = emissiveNee<KM>(g.em, s, o.P, o.N, o.Ng, o.tEps, r.x, r.y, ovf);
+    nee = 1;
+    float4 L = w.L[slot];
+    L.x += e.x;
+    L.y += e.y;
+    L.z += e.z;
+    w.L[slot] = L;
+  }
   warpCount(&g.stats[1], nee);
   warpCount(g.overflow, ovf);
+}
+
+// The samples of a point summed (each lane its own in order, the lanes in a
+// shuffle tree) into E = (mean radiance, share of first bounces that hit or
+// fell below the horizon); halfE gets the sum of the first spp/2.  ReSTIR (one
+// lane per point): every sample is also one candidate streamed, in sample
+// order, into the point's reservoir (pt1_gather.hpp:287-297, 451-499).
+__global__ void __launch_bounds__(128) k_gather_sum(GiP g, GiGrid grid, const uint32_t* list, GiWave w, float4* E) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t group = t >> 5, lane = t & 31u, iters = uint32_t(w.iters);
+  const bool on = group * iters * 32u < waveSlots(w);
+  f3 e{0.0f, 0.0f, 0.0f}, half{0.0f, 0.0f, 0.0f};
+  float occ = 0.0f;
+  uint32_t point = 0, pix = 0;
+  bool own = false;
+  uint32_t rs0 = 0, rs1 = 0x47490001u;
+  double rWSum = 0.0;
+  f3 rPos{0.0f, 0.0f, 0.0f}, rNrm{0.0f, 0.0f, 0.0f}, rRad{0.0f, 0.0f, 0.0f};
+  float rPHat = 0.0f;
+  if (on && w.it0 > 0) {
+    const float4* c = w.carry + size_t(kCarryF4) * t;
+    e = ld3(c[0]);
+    occ = c[0].w;
+    half = ld3(c[1]);
+    rPos = ld3(c[2]);
+    rPHat = c[2].w;
+    rNrm = ld3(c[3]);
+    rRad = ld3(c[4]);
+    rWSum = __hiloint2double(__float_as_int(c[5].y), __float_as_int(c[5].x));
+    own = c[1].w != 0.0f;
+    pix = own ? __float_as_uint(c[3].w) : 0u;
+    rs0 = __float_as_uint(c[4].w);
+    rs1 = __float_as_uint(c[5].z);
+  }
+  for (uint32_t it = 0; on && it < iters; ++it) {
+    const uint32_t slot = (group * iters + it) * 32u + lane;
+    int sI;
+    if (!slotSample(w, slot, point, sI)) continue;
+    if (!own) {
+      own = true;
+      pix = list[point];
+      rs0 = hashU32(pix ^ g.seedMix) ^ 0x52455354u;
+    }
+    float4 L = w.L[slot];
+    if (g.clampLum > 0.0f) {
+      const float lum = 0.2126f * L.x + 0.7152f * L.y + 0.0722f * L.z;
+      if (lum > g.clampLum) {
+        const float k = g.clampLum / lum;
+        L.x *= k;
+        L.y *= k;
+        L.z *= k;
+      }
+    }
+    if (w.cand) {  // RIS weight pi * lum(L): p_hat = lum(L) cos over the cosine pdf
+      const float4 c0 = w.cand[2 * size_t(slot)], c1 = w.cand[2 * size_t(slot) + 1];
+      float wgt = 0.0f, pHat = 0.0f;
+      if (c1.w > 0.0f) {
+        pHat = lumOf(L.x, L.y, L.z) * c1.w;
+        wgt = lumOf(L.x, L.y, L.z) * kPiF;
+      }
+      tea2(rs0, rs1);
+      rWSum += double(wgt);
+      if (wgt > 0.0f && double(u32ToUnorm(rs0)) * rWSum <= double(wgt)) {
+        rPos = ld3(c0);
+        rNrm = ld3(c1);
+        rRad = ld3(L);
+        rPHat = pHat;
+      }
+    }
+    e.x += L.x;
+    e.y += L.y;
+    e.z += L.z;
+    occ += L.w;
+    if (sI < w.spp / 2) {
+      half.x += L.x;
+      half.y += L.y;
+      half.z += L.z;
+    }
+  }
+  if (w.it0 + w.iters < w.itEnd) {
+    if (!on) return;
+    float4* c = w.carry + size_t(kCarryF4) * t;
+    c[0] = make_float4(e.x, e.y, e.z, occ);
+    c[1] = make_float4(half.x, half.y, half.z, own ? 1.0f : 0.0f);
+    c[2] = make_float4(rPos.x, rPos.y, rPos.z, rPHat);
+    c[3] = make_float4(rNrm.x, rNrm.y, rNrm.z, __uint_as_float(pix));
+    c[4] = make_float4(rRad.x, rRad.y, rRad.z, __uint_as_float(rs0));
+    c[5] = make_float4(__int_as_float(__double2loint(rWSum)), __int_as_float(__double2hiint(rWSum)),
+                       __uint_as_float(rs1), 0.0f);
+    return;
+  }
+  const int lanes = 1 << w.logLanes;
+  for (int o = lanes / 2; o > 0; o >>= 1) {
+    e.x += __shfl_xor_sync(0xFFFFFFFFu, e.x, o);
+    e.y += __shfl_xor_sync(0xFFFFFFFFu, e.y, o);
+    e.z += __shfl_xor_sync(0xFFFFFFFFu, e.z, o);
+    occ += __shfl_xor_sync(0xFFFFFFFFu, occ, o);
+    half.x += __shfl_xor_sync(0xFFFFFFFFu, half.x, o);
+    half.y += __shfl_xor_sync(0xFFFFFFFFu, half.y, o);
+    half.z += __shfl_xor_sync(0xFFFFFFFFu, half.z, o);
+  }
+  // lane 0 of a point has its first sample: it always owns one
+  if (!own || (lane & uint32_t(lanes - 1)) != 0u) return;
+  const float invN = 1.0f / float(w.spp > 0 ? w.spp : 1);
+  E[pix] = make_float4(e.x * invN, e.y * invN, e.z * invN, occ * invN);
+  if (g.halfE) {
+    g.halfE[3 * size_t(pix)] = half.x;
+    g.halfE[3 * size_t(pix) + 1] = half.y;
+    g.halfE[3 * size_t(pix) + 2] = half.z;
+  }
+  if (w.cand) {  // W = wSum / (M p_hat(selected)), M = every candidate
+    float4* rsv = g.rsv + size_t(kRsvF4) * pix;
+    const float M = float(w.spp > 0 ? w.spp : 1);
+    const float W = (rPHat > 0.0f && rWSum > 0.0) ? float(rWSum / (double(M) * double(rPHat))) : 0.0f;
+    rsv[0] = make_float4(rPos.x, rPos.y, rPos.z, M);
+    rsv[1] = make_float4(rNrm.x, rNrm.y, rNrm.z, W);
+    rsv[2] = make_float4(rRad.x, rRad.y, rRad.z, 0.0f);
+  }
 }
 
 // tracePt1GBuffer (pt1_gbuffer.hpp:83-196): one primary ray per point of a
@@ -1500,28 +1809,145 @@ void giGBuffer(int km, cudaStream_t s, const Params& p, const DScene& sc, int w,
   });
 }
 
-// Lanes per gather point: the sample count rounded down to a power of two,
-// at most 8 (a warp then holds four points' fans).  The grid is at most 16
-// blocks per SM (a list's length is known only on the device).
-void giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, const LightD* lights, int nLights,
-              const GiGrid& grid, const uint32_t* list, const uint32_t* listCount, uint32_t n, int spp, float4* E) {
-  // a ReSTIR gather streams each point's samples in order: one thread per point
-  const int lanes = g.rsv ? 1 : spp >= 8 ? 8 : spp >= 4 ? 4 : spp >= 2 ? 2 : 1;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const uint32_t nb = std::max(1u, std::min(blocks(uint64_t(n) * uint64_t(lanes), 128), uint32_t(std::max(sms, 1)) * 16u));
-  byKind(km, [&](auto K) {
-    constexpr int k = decltype(K)::value;
-    if (lanes == 8)
-      k_gather<k, 8><<<nb, 128, 0, s>>>(g, sc, lights, nLights, grid, list, listCount, n, spp, E);
-    else if (lanes == 4)
-      k_gather<k, 4><<<nb, 128, 0, s>>>(g, sc, lights, nLights, grid, list, listCount, n, spp, E);
-    else if (lanes == 2)
-      k_gather<k, 2><<<nb, 128, 0, s>>>(g, sc, lights, nLights, grid, list, listCount, n, spp, E);
-    else
-      k_gather<k, 1><<<nb, 128, 0, s>>>(g, sc, lights, nLights, grid, list, listCount, n, spp, E);
-  });
+// Lanes per gather point: the sample count rounded down to a power of two, at
+// most 8 (a warp then holds four points' fans); one for a ReSTIR gather, which
+// streams each point's samples in order.
+static int gatherLogLanes(const GiP& g, int spp) { return g.rsv ? 0 : spp >= 8 ? 3 : spp >= 4 ? 2 : spp >= 2 ? 1 : 0; }
+
+// Bytes a slot takes in each array of the workspace, in GiWave's order.
+static size_t gatherSlotBytes(const GiP& g, int nLights) {
+  const size_t nl = size_t(std::max(nLights, 0));
+  return 16 + 64 + (g.bounces > 1 ? 32 + 64 : 0) + nl * 17 + (g.pt2 && g.em.n > 0 ? 8 : 0) + (g.rsv ? 32 : 0);
+}
+constexpr size_t kWaveHeader = 256, kWaveAlign = 256, kWaveArrays = 20;
+// A chunk: enough rays that its first and last wave of blocks weigh little, in
+// a workspace of the size of a frame's own buffers (0.5 GB with two lights):
+// 2^20 slots are 8 % slower on the pt2 default frame, 2^24 1.5 % faster.
+constexpr uint64_t kWaveSlots = 1u << 22;
+constexpr size_t kWaveBytes = size_t(1) << 30;
+
+size_t giGatherBytes(const GiP& g, int nLights, uint64_t n, int spp) {
+  const int lg = gatherLogLanes(g, spp);
+  const uint64_t P = 32u >> lg, iters = (uint64_t(std::max(spp, 1)) + (1u << lg) - 1) >> lg;
+  const uint64_t slots = (n + P - 1) / P * iters * 32u;
+  const size_t sb = gatherSlotBytes(g, nLights);
+  const uint64_t cap = std::min<uint64_t>(kWaveSlots, kWaveBytes / sb);
+  return std::max(kGatherMinBytes, kWaveHeader + kWaveArrays * kWaveAlign + size_t(std::min(slots, cap)) * sb);
+}
+
+cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, const LightD* lights, int nLights,
+                     const GiGrid& grid, const uint32_t* list, const uint32_t* listCount, uint32_t n, int spp,
+                     float4* E, uint32_t* listBuf, void* ws, size_t wsBytes, uint32_t* hostCount,
+                     uint32_t* launches) {
+  if (n == 0) return cudaSuccess;
+  GiWave w{};
+  w.ctr = static_cast<uint32_t*>(ws);
+  w.spp = std::max(spp, 0);
+  w.logLanes = gatherLogLanes(g, spp);
+  const uint32_t P = 32u >> w.logLanes;
+  w.itEnd = std::max(1, (w.spp + (1 << w.logLanes) - 1) >> w.logLanes);
+  const size_t sb = gatherSlotBytes(g, nLights);
+  const size_t carryBytes = size_t(kCarryF4) * 16 * 32;  // windows run one group at a time
+  const size_t room = std::min<size_t>(wsBytes - kWaveHeader - kWaveArrays * kWaveAlign, kWaveSlots * sb);
+  uint64_t groupsFit = room / (size_t(w.itEnd) * 32u * sb);
+  w.iters = w.itEnd;
+  if (groupsFit == 0) {
+    w.iters = int(std::max<size_t>(1, (room - carryBytes) / (32u * sb)));
+    groupsFit = 1;
+  }
+  cudaError_t e = cudaMemsetAsync(w.ctr, 0, 4 * sizeof(uint32_t), s);
+  if (e != cudaSuccess) return e;
+  const uint32_t* pts = list;
+  if (list) {
+    e = cudaMemcpyAsync(w.ctr, listCount, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
+  } else {
+    // points that are not eligible keep E = 0
+    e = cudaMemsetAsync(E, 0, size_t(n) * sizeof(float4), s);
+    if (e == cudaSuccess && g.halfE) e = cudaMemsetAsync(g.halfE, 0, size_t(n) * 3 * sizeof(float), s);
+    k_gather_list<<<blocks(n, 256), 256, 0, s>>>(grid, n, w.logLanes == 0 ? 1 : 0, listBuf, w.ctr);
+    ++*launches;
+    pts = listBuf;
+  }
+  if (e != cudaSuccess) return e;
+  // more than one chunk of the listed points at most: read how many there are
+  uint32_t count = n;
+  if ((uint64_t(n) + P - 1) / P > groupsFit || w.iters < w.itEnd) {
+    e = cudaMemcpyAsync(hostCount, w.ctr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return e;
+    count = std::min(n, *hostCount);
+    if (count == 0) return cudaGetLastError();
+  }
+  const uint64_t groups = (uint64_t(count) + P - 1) / P;
+  const uint64_t chunks = (groups + groupsFit - 1) / groupsFit;
+  const uint64_t perChunk = (groups + chunks - 1) / chunks;  // equal chunks: no short last one
+  const bool multi = g.bounces > 1, emit = g.pt2 && g.em.n > 0;
+  const int maxB = g.bounces < 1 ? 1 : g.bounces;
+  const uint64_t slotCap = perChunk * uint64_t(w.iters) * 32u;
+  // carve the workspace
+  char* at = static_cast<char*>(ws) + kWaveHeader;
+  auto take = [&](size_t bytes) {
+    char* p = at;
+    at += (bytes + kWaveAlign - 1) / kWaveAlign * kWaveAlign;
+    return p;
+  };
+  auto f4 = [&]() { return reinterpret_cast<float4*>(take(size_t(slotCap) * 16)); };
+  w.L = f4();
+  for (float4*& r : w.r) r = f4();
+  if (multi) {
+    w.thr = f4();
+    w.pos = f4();
+    for (float4*& p : w.path) p = f4();
+  }
+  const size_t nl = size_t(std::max(nLights, 0));
+  w.shadow = reinterpret_cast<float4*>(take(size_t(slotCap) * nl * 16));
+  w.vis = reinterpret_cast<uint8_t*>(take(size_t(slotCap) * nl));
+  if (emit) w.rng = reinterpret_cast<uint2*>(take(size_t(slotCap) * 8));
+  if (g.rsv) w.cand = reinterpret_cast<float4*>(take(size_t(slotCap) * 32));
+  if (w.iters < w.itEnd) w.carry = reinterpret_cast<float4*>(take(carryBytes));
+  const int itWindow = w.iters;
+  for (uint64_t g0 = 0; g0 < groups; g0 += perChunk) {
+    w.p0 = uint32_t(g0 * P);
+    w.nPts = uint32_t(std::min<uint64_t>(count, (g0 + perChunk) * P) - w.p0);
+    const uint64_t nGroups = (uint64_t(w.nPts) + P - 1) / P;
+    for (w.it0 = 0; w.it0 < w.itEnd; w.it0 += itWindow) {
+      w.iters = std::min(itWindow, w.itEnd - w.it0);
+      const uint64_t slots = nGroups * uint64_t(w.iters) * 32u;
+      for (int b = 1; b <= maxB; ++b) {
+        // [1] records and [2] shadow rays of this bounce; [3] its paths are
+        // consumed by the closest-hit launch before the next ones are pushed
+        e = cudaMemsetAsync(w.ctr + 1, 0, (b == 1 ? 3 : 2) * sizeof(uint32_t), s);
+        if (e != cudaSuccess) return e;
+        byKind(km, [&](auto K) {
+          constexpr int k = decltype(K)::value;
+          if (b == 1) k_gather_first<k><<<blocks(slots, 128), 128, 0, s>>>(g, sc, grid, pts, w, multi ? 1 : 0);
+          else k_gather_next<k><<<blocks(slots, 128), 128, 0, s>>>(g, sc, w);
+        });
+        k_gather_vertex<<<blocks(slots, 128), 128, 0, s>>>(g, sc, lights, nLights, grid, pts, w, b);
+        if (nl > 0)
+          byKind(km, [&](auto K) {
+            k_gather_shadow<decltype(K)::value><<<blocks(slots * nl, 128), 128, 0, s>>>(g, sc, nLights, w);
+          });
+        if (b > 1 && b < maxB) {
+          e = cudaMemsetAsync(w.ctr + 3, 0, sizeof(uint32_t), s);
+          if (e != cudaSuccess) return e;
+        }
+        k_gather_resolve<<<blocks(slots, 128), 128, 0, s>>>(g, lights, nLights, w, b, maxB);
+        *launches += 3u + (nl > 0 ? 1u : 0u);
+      }
+      if (emit) {
+        byKind(km, [&](auto K) {
+          k_gather_emit<decltype(K)::value><<<blocks(slots, 128), 128, 0, s>>>(g, sc, grid, pts, w);
+        });
+        ++*launches;
+      }
+      k_gather_sum<<<blocks(nGroups * 32u, 128), 128, 0, s>>>(g, grid, pts, w, E);
+      ++*launches;
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+    }
+  }
+  return cudaSuccess;
 }
 
 void giDenoiseInit(cudaStream_t s, uint32_t n, float4* E, const float4* ne, uint8_t* valid, float4* irr) {

@@ -479,7 +479,7 @@ __device__ __forceinline__ void occlusionBody(const Params& p1, const DScene& s1
 // One thread per AO / shadow ray, 9 blocks of 128 per SM (56 registers):
 // measured best for mesh and for sphere + cylinder scenes.
 template <bool COUNT, int KM, bool BATCH>
-__global__ void __launch_bounds__(128, 9)
+__global__ void __launch_bounds__(128, (KM & kMaskMesh) ? 8 : 9)
     k_trace_occlusion(Params p1, DScene s1, Batch bt, Bufs b, uint32_t n) {
   occlusionBody<COUNT, KM, BATCH, false>(p1, s1, bt, b);
 }
@@ -2722,6 +2722,32 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
       UBR_CUDA(c, cudaGetLastError());
       return UBR_OK;
     };
+    // the gather of `n` points of a grid or list.  Its workspace is context
+    // scratch of its own; under an arena cap, or where that allocation fails,
+    // the hit records of the finished layers (16 B per hi-res pixel) or, for a
+    // frame of few pixels, a small block outside the cap
+    auto gather = [&](const GiP& gg, const GiGrid& gr, const uint32_t* list, const uint32_t* cnt, uint32_t n, int nspp,
+                      float4* E) -> ubr_status {
+      const size_t want = giGatherBytes(gg, nL, n, nspp);
+      void* ws = nullptr;
+      size_t bytes = want;
+      if (c->arenaCap == 0 && scratchGet(c, 149, want, &ws) != UBR_OK) {
+        cudaGetLastError();
+        ws = nullptr;
+      }
+      if (!ws) {
+        ws = b.hitA;
+        bytes = size_t(nslot) * sizeof(float4);
+        if (bytes < kGatherMinBytes) {
+          if (!c->gatherMin) UBR_CUDA(c, cudaMalloc(&c->gatherMin, kGatherMinBytes));
+          ws = c->gatherMin;
+          bytes = kGatherMinBytes;
+        }
+      }
+      // the eligible points of a grid are listed in the first queue buffer
+      UBR_CUDA(c, giGather(km, s, gg, s1, lt, nL, gr, list, cnt, n, nspp, E, q0, ws, bytes, hostCount + 8, &kernels));
+      return UBR_OK;
+    };
     // the gather over a grid, with pt2's adaptive refinement (pt2_adaptive.hpp:
     // mask of noisy points, dilated twice, re-gathered continuing their
     // sequences, merged as a weighted mean)
@@ -2736,8 +2762,8 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
       float4* rsvB = restir ? scratchT<float4>(c, 145, size_t(n) * kRsvF4, as) : nullptr;
       if (as != UBR_OK) return as;
       g0.rsv = rsvA;
-      giGather(km, s, g0, s1, lt, nL, gr, nullptr, nullptr, n, spp, E);
-      ++kernels;
+      as = gather(g0, gr, nullptr, nullptr, n, spp, E);
+      if (as != UBR_OK) return as;
       if (restir) {
         // spatial rounds over the reservoirs, ping-pong; the last one writes E
         // (pt2_spatial.hpp:278-296)
@@ -2765,9 +2791,10 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
         giMaskList(s, n, m0, list, cnt);
         GiP g1 = gp;
         g1.sampleOffset = spp;
-        giGather(km, s, g1, s1, lt, nL, gr, list, cnt, n, extra, Er);
+        as = gather(g1, gr, list, cnt, n, extra, Er);
+        if (as != UBR_OK) return as;
         giMerge(s, list, cnt, n, spp, extra, Er, E);
-        kernels += 6;
+        kernels += 5;
       }
       UBR_CUDA(c, cudaGetLastError());
       return UBR_OK;
@@ -2813,11 +2840,12 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
         const int pspp = spp * std::max(1, d0.pt1_edge_patch_spp_mul);
         GiP gpat = gp;
         gpat.sppPow2 = pow2(uint32_t(pspp));
-        giGather(km, s, gpat, s1, lt, nL, full, patchList, patchCount, npix, pspp, Ef);
+        gs = gather(gpat, full, patchList, patchCount, npix, pspp, Ef);
+        if (gs != UBR_OK) return gs;
         UBR_CUDA(c, cudaMemcpyAsync(Esnap, Ef, size_t(npix) * sizeof(float4), cudaMemcpyDeviceToDevice, s));
         giSmooth(s, p1.W, p1.H, patchList, patchCount, npix, b.giA, b.giB, d0.pt1_upsample_normal_pow,
                  d0.pt1_upsample_depth_scale, 2, Esnap, Ef);
-        kernels += 2;
+        ++kernels;
         UBR_CUDA(c, cudaMemcpyAsync(static_cast<char*>(c->pinned) + 256, patchCount, sizeof(uint32_t),
                                     cudaMemcpyDeviceToHost, s));
       }

@@ -42,6 +42,7 @@ struct Context {
   std::vector<void*> sceneHandles;      // live ubr_scene handles built on this context
   cudaMemPool_t pool = nullptr;         // stream-ordered device allocations (scenes, scratch)
   void* noallocArray = nullptr;         // device address of the allocation-free query's fixed array
+  void* gatherMin = nullptr;            // GI gather workspace of last resort (kGatherMinBytes), on first use
   cudaEvent_t giEv[7] = {};             // GI pass stage boundaries, created on first use
 };
 
