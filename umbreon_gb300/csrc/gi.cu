@@ -451,7 +451,9 @@ struct GiWave {
   uint32_t* ctr;      // [0] listed points, [1] records, [2] shadow rays, [3] paths of the next bounce
   float4* L;          // per slot: radiance, 1 = the first bounce hit something or fell below the horizon
   float4* r[4];       // records: (t,u,v,ref)|(Ng,slot)|(dir,s0)|(org,s1), then
-                      //          (shadow origin,eps; eps < 0: ended)|(N,slot)|(kd C,s0)|(emission,s1)
+                      //          (shadow origin,eps; eps < 0: ended)|(N,slot)|(kd C,s0)|(emission,s1);
+                      //          r[3] only with several bounces or emitters: the first vertex's origin and
+                      //          stream follow from its slot, and its emission waits in L
   float4* thr;        // several bounces: (throughput, hit t) and
   float4* pos;        //   (position, -) of a record
   float4* path[4];    // several bounces: (org,tnear)|(dir,slot)|(throughput,s0)|(s1 bits,-,-,-)
@@ -549,8 +551,7 @@ __global__ void k_gather_list(GiGrid grid, uint32_t n, int single, uint32_t* lis
 }
 
 template <int KM>
-__global__ void __launch_bounds__(128, 8) k_gather_first(GiP g, DScene s, GiGrid grid, const uint32_t* list, GiWave w,
-                                                         int multi) {
+__global__ void __launch_bounds__(128, 8) k_gather_first(GiP g, DScene s, GiGrid grid, const uint32_t* list, GiWave w) {
   const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t rays = 0, ovf = 0, point;
   int sI;
@@ -601,8 +602,8 @@ __global__ void __launch_bounds__(128, 8) k_gather_first(GiP g, DScene s, GiGrid
     w.r[0][q] = make_float4(h.t, h.u, h.v, __uint_as_float(h.ref));
     w.r[1][q] = make_float4(h.Ng.x, h.Ng.y, h.Ng.z, __uint_as_float(slot));
     w.r[2][q] = make_float4(wi.x, wi.y, wi.z, __uint_as_float(s0));
-    w.r[3][q] = make_float4(O.x, O.y, O.z, __uint_as_float(s1));
-    if (multi) w.thr[q] = make_float4(1.0f, 1.0f, 1.0f, h.t);
+    if (w.r[3]) w.r[3][q] = make_float4(O.x, O.y, O.z, __uint_as_float(s1));
+    if (w.thr) w.thr[q] = make_float4(1.0f, 1.0f, 1.0f, h.t);
   }
   warpCount(&g.stats[0], rays);
   warpCount(g.overflow, ovf);
@@ -655,22 +656,36 @@ __global__ void __launch_bounds__(128) k_gather_vertex(GiP g, DScene s, const Li
                                                        const uint32_t* list, GiWave w, int bounce) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   const bool on = q < w.ctr[1];
-  uint32_t nee = 0, s0 = 0, s1 = 0;
+  uint32_t nee = 0, s0 = 0, s1 = 0, slot = 0;
   bool live = false;
   VertexSurf v;
   f3 emitted{0.0f, 0.0f, 0.0f};
   if (on) {
-    const float4 ra = w.r[0][q], rb = w.r[1][q], rc = w.r[2][q], rd = w.r[3][q];
+    const float4 ra = w.r[0][q], rb = w.r[1][q], rc = w.r[2][q];
     Hit h;
     h.t = ra.x;
     h.u = ra.y;
     h.v = ra.z;
     h.ref = __float_as_uint(ra.w);
     h.Ng = ld3(rb);
-    const f3 dir = ld3(rc), org = ld3(rd);
+    const f3 dir = ld3(rc);
+    f3 org;
     s0 = __float_as_uint(rc.w);
-    s1 = __float_as_uint(rd.w);
-    const uint32_t slot = __float_as_uint(rb.w);
+    slot = __float_as_uint(rb.w);
+    if (w.r[3]) {
+      const float4 rd = w.r[3][q];
+      org = ld3(rd);
+      s1 = __float_as_uint(rd.w);
+    } else {
+      uint32_t point;
+      int sI;
+      slotSample(w, slot, point, sI);
+      const GatherOrigin o = gatherOrigin(g, grid, list[point]);
+      org = o.O;
+      s0 = o.seed;
+      s1 = uint32_t(sI + g.sampleOffset);
+      tea2(s0, s1);
+    }
     live = vertexSurface(s, h, org, dir, v);
     if (bounce == 1 && w.cand) {
       float4* c = w.cand + 2 * size_t(slot);
@@ -717,7 +732,8 @@ __global__ void __launch_bounds__(128) k_gather_vertex(GiP g, DScene s, const Li
   }
   if (live) {
     w.r[2][q] = make_float4(v.alb.x, v.alb.y, v.alb.z, __uint_as_float(s0));
-    w.r[3][q] = make_float4(emitted.x, emitted.y, emitted.z, __uint_as_float(s1));
+    if (w.r[3]) w.r[3][q] = make_float4(emitted.x, emitted.y, emitted.z, __uint_as_float(s1));
+    else if (v.emission > 0.0f) w.L[slot] = make_float4(emitted.x, emitted.y, emitted.z, 1.0f);
   }
   warpCount(&g.stats[1], nee);
 }
@@ -747,20 +763,28 @@ __global__ void __launch_bounds__(128) k_gather_resolve(GiP g, const LightD* lig
   float tnear = 0.0f;
   uint32_t slot = 0, s0 = 0, s1 = 0;
   if (q < w.ctr[1] && !(w.r[0][q].w < 0.0f)) {
-    const float4 rb = w.r[1][q], rc = w.r[2][q], rd = w.r[3][q];
-    const f3 N = ld3(rb), alb = ld3(rc), em = ld3(rd);
+    const float4 rb = w.r[1][q], rc = w.r[2][q];
+    const f3 N = ld3(rb), alb = ld3(rc);
     slot = __float_as_uint(rb.w);
-    s0 = __float_as_uint(rc.w);
-    s1 = __float_as_uint(rd.w);
+    float4 L = w.L[slot];
+    f3 em{L.x, L.y, L.z};
+    if (w.r[3]) {
+      const float4 rd = w.r[3][q];
+      em = ld3(rd);
+      s0 = __float_as_uint(rc.w);
+      s1 = __float_as_uint(rd.w);
+    } else {
+      L.x = L.y = L.z = 0.0f;
+    }
     f3 E{0.0f, 0.0f, 0.0f};
     for (int l = 0; l < nLights; ++l) {
-      const LightD L = lights[l];
-      const float ndl = dot(N, L.L);
+      const LightD lt = lights[l];
+      const float ndl = dot(N, lt.L);
       if (ndl <= 0.0f) continue;
       const float sh = w.vis[size_t(q) * uint32_t(nLights) + uint32_t(l)] ? 0.0f : 1.0f;
-      E.x += ndl * L.color.x * sh;
-      E.y += ndl * L.color.y * sh;
-      E.z += ndl * L.color.z * sh;
+      E.x += ndl * lt.color.x * sh;
+      E.y += ndl * lt.color.y * sh;
+      E.z += ndl * lt.color.z * sh;
     }
     float hitT = 0.0f;
     if (w.thr) {
@@ -768,7 +792,6 @@ __global__ void __launch_bounds__(128) k_gather_resolve(GiP g, const LightD* lig
       thr = ld3(t4);
       hitT = t4.w;
     }
-    float4 L = w.L[slot];
     L.x += thr.x * (alb.x * E.x + em.x);
     L.y += thr.y * (alb.y * E.y + em.y);
     L.z += thr.z * (alb.z * E.z + em.z);
@@ -1817,7 +1840,8 @@ static int gatherLogLanes(const GiP& g, int spp) { return g.rsv ? 0 : spp >= 8 ?
 // Bytes a slot takes in each array of the workspace, in GiWave's order.
 static size_t gatherSlotBytes(const GiP& g, int nLights) {
   const size_t nl = size_t(std::max(nLights, 0));
-  return 16 + 64 + (g.bounces > 1 ? 32 + 64 : 0) + nl * 17 + (g.pt2 && g.em.n > 0 ? 8 : 0) + (g.rsv ? 32 : 0);
+  const bool lean = g.bounces <= 1 && !(g.pt2 && g.em.n > 0);
+  return 16 + (lean ? 48 : 64) + (g.bounces > 1 ? 32 + 64 : 0) + nl * 17 + (g.pt2 && g.em.n > 0 ? 8 : 0) + (g.rsv ? 32 : 0);
 }
 constexpr size_t kWaveHeader = 256, kWaveAlign = 256, kWaveArrays = 20;
 // A chunk: enough rays that its first and last wave of blocks weigh little, in
@@ -1893,7 +1917,8 @@ cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, con
   };
   auto f4 = [&]() { return reinterpret_cast<float4*>(take(size_t(slotCap) * 16)); };
   w.L = f4();
-  for (float4*& r : w.r) r = f4();
+  for (int k = 0; k < 3; ++k) w.r[k] = f4();
+  if (multi || emit) w.r[3] = f4();
   if (multi) {
     w.thr = f4();
     w.pos = f4();
@@ -1920,7 +1945,7 @@ cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, con
         if (e != cudaSuccess) return e;
         byKind(km, [&](auto K) {
           constexpr int k = decltype(K)::value;
-          if (b == 1) k_gather_first<k><<<blocks(slots, 128), 128, 0, s>>>(g, sc, grid, pts, w, multi ? 1 : 0);
+          if (b == 1) k_gather_first<k><<<blocks(slots, 128), 128, 0, s>>>(g, sc, grid, pts, w);
           else k_gather_next<k><<<blocks(slots, 128), 128, 0, s>>>(g, sc, w);
         });
         k_gather_vertex<<<blocks(slots, 128), 128, 0, s>>>(g, sc, lights, nLights, grid, pts, w, b);

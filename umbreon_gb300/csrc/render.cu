@@ -424,8 +424,9 @@ UBR_D void occRayOf(uint64_t rid, uint32_t nq, uint64_t R, uint64_t A, uint32_t&
   }
 }
 
-// The occlusion kernel's body: one thread per AO / shadow ray.
-template <bool COUNT, int KM, bool BATCH, bool IL>
+// The occlusion kernel's body: one thread per AO / shadow ray.  NEAREST: a
+// frame of the launch wants its AO rays' nearest hits (enhanced AO, AOVs).
+template <bool COUNT, int KM, bool BATCH, bool IL, bool NEAREST>
 __device__ __forceinline__ void occlusionBody(const Params& p1, const DScene& s1, const Batch& bt, const Bufs& b) {
   Count cnt;
   const uint64_t tid = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -457,7 +458,7 @@ __device__ __forceinline__ void occlusionBody(const Params& p1, const DScene& s1
       h.t = kInfF;
       if (o.trace) {
         const TravScene ts = travOf(s);
-        if (p.aoEnhanced || p.aoWriteAov)
+        if (NEAREST && (p.aoEnhanced || p.aoWriteAov))
           hit = traverse<COUNT, KM, false>(ts, o.r, h, ovf, &cnt, o.anyHit, o.start);
         else if (IL)
           hit = traverseAnyInterleaved<COUNT, KM>(ts, o.r, ovf, &cnt, o.start);
@@ -476,12 +477,24 @@ __device__ __forceinline__ void occlusionBody(const Params& p1, const DScene& s1
   }
 }
 
-// One thread per AO / shadow ray, 9 blocks of 128 per SM (56 registers):
-// measured best for mesh and for sphere + cylinder scenes.
+// One thread per AO / shadow ray, 9 blocks of 128 per SM (56 registers) for
+// spheres and cylinders, 8 (64 registers) with triangles: one block more or
+// less per SM is 1-2 % slower (ball-and-stick 1920x1080 ss2, transparent
+// surface 1023x769).
 template <bool COUNT, int KM, bool BATCH>
 __global__ void __launch_bounds__(128, (KM & kMaskMesh) ? 8 : 9)
     k_trace_occlusion(Params p1, DScene s1, Batch bt, Bufs b, uint32_t n) {
-  occlusionBody<COUNT, KM, BATCH, false>(p1, s1, bt, b);
+  occlusionBody<COUNT, KM, BATCH, false, false>(p1, s1, bt, b);
+}
+
+// The same for launches that want nearest hits.  Apart from the binary kernel
+// because two traversals in one kernel cost it registers and instruction
+// cache: split, the ball-and-stick frame is 1 % and a batch of 24 sphere
+// frames 2.6 % faster (7.42 -> 7.35 ms, 9.41 -> 9.16 ms).
+template <bool COUNT, int KM, bool BATCH>
+__global__ void __launch_bounds__(128, (KM & kMaskMesh) ? 8 : 9)
+    k_trace_occlusion_nearest(Params p1, DScene s1, Batch bt, Bufs b, uint32_t n) {
+  occlusionBody<COUNT, KM, BATCH, false, true>(p1, s1, bt, b);
 }
 
 // The same with node visits and primitive tests interleaved one per step
@@ -489,7 +502,7 @@ __global__ void __launch_bounds__(128, (KM & kMaskMesh) ? 8 : 9)
 template <bool COUNT, int KM, bool BATCH>
 __global__ void __launch_bounds__(128, (KM & kMaskMesh) ? 9 : 8)
     k_trace_occlusion_il(Params p1, DScene s1, Batch bt, Bufs b, uint32_t n) {
-  occlusionBody<COUNT, KM, BATCH, true>(p1, s1, bt, b);
+  occlusionBody<COUNT, KM, BATCH, true, true>(p1, s1, bt, b);
 }
 
 // Resident-grid variant: each CTA stages the top wide nodes (root and the two
@@ -592,7 +605,7 @@ __global__ void __launch_bounds__(128, 8) k_trace_occlusion_persistent(Params p1
           } else if (o.trace && s.primCount > 0 && o.start >= 0) {
             ts = travOf(s);
             inv = safeInv(o.r.dir);
-            if (KM & kMaskMesh) pre = triPre(o.r.dir);
+            if (KM & kMaskMesh) pre = triPre(o.r.dir, o.r.org);
             travInit(o.r, st, best, o.start);
             active = true;
             ++traced;
@@ -2053,8 +2066,9 @@ void launchClosest(int km, bool count, bool batch, uint32_t grid, int tb, cudaSt
 }
 
 void launchOcclusion(int km, bool count, bool batch, uint32_t grid, int tb, cudaStream_t st, const Params& p,
-                     const DScene& s, const Batch& bt, const Bufs& b, uint32_t n, bool il = false) {
+                     const DScene& s, const Batch& bt, const Bufs& b, uint32_t n, bool il, bool nearest) {
   if (il) UBR_KM_DISPATCH(k_trace_occlusion_il, km, count, batch, grid, tb, st, p, s, bt, b, n);
+  else if (nearest) UBR_KM_DISPATCH(k_trace_occlusion_nearest, km, count, batch, grid, tb, st, p, s, bt, b, n);
   else UBR_KM_DISPATCH(k_trace_occlusion, km, count, batch, grid, tb, st, p, s, bt, b, n);
 }
 
@@ -2118,7 +2132,7 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
   uint64_t npix64 = 0, nout64 = 0;
   uint32_t R = 0, aoStride = 0, aoMin = 0xFFFFFFFFu;
   int km = 0, maxIters = 1;
-  bool secondary = false, enhanced = false, singleLayer = true, aov = false;
+  bool secondary = false, enhanced = false, nearest = false, singleLayer = true, aov = false;
   for (size_t f = 0; f < nf; ++f) {
     std::vector<LightD> fl;
     Params& p = fds[f].p;
@@ -2135,6 +2149,7 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
     nout64 += uint64_t(p.outW) * uint64_t(p.outH);
     R = std::max(R, uint32_t(p.raysPerHit));
     aoMin = std::min(aoMin, uint32_t(p.aoSamples));
+    nearest = nearest || p.aoEnhanced || p.aoWriteAov;
     if ((p.aoEnhanced || p.aoWriteAov) && p.aoSamples > 0) {
       enhanced = true;
       aoStride = std::max(aoStride, uint32_t(p.aoSamples));
@@ -2431,7 +2446,7 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
       mark(2, true);
       if (c->traceMode == 1 || c->traceMode == 4) {
         launchOcclusion(km, count, batch, uint32_t((nr + TB - 1) / TB), TB, s, pr, s1, bt, br, n,
-                        c->traceMode == 4);
+                        c->traceMode == 4, nearest);
       } else if (c->traceMode == 3) {
         launchOcclusionGridStride(km, count, batch, gridStrideGrid(c->device), TB, s, pr, s1, bt, br);
       } else {
@@ -2462,7 +2477,7 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
     mark(2, true);
     if (c->traceMode == 1 || c->traceMode == 4) {
       launchOcclusion(km, count, false, uint32_t((nr + TB - 1) / TB), TB, s, pCoarse, s1, bt, b, nCell,
-                      c->traceMode == 4);
+                      c->traceMode == 4, nearest);
     } else if (c->traceMode == 3) {
       launchOcclusionGridStride(km, count, false, gridStrideGrid(c->device), TB, s, pCoarse, s1, bt, b);
     } else {

@@ -770,10 +770,8 @@ __global__ void k_refit(BuildIn in, int n, int idxBits, const unsigned long long
   leafRef[sIdx] = packRef(kind, prim);
   float4* lg = leafGeo + kLeafF4 * sIdx;
   if (kind == kMesh) {
-    for (int k = 0; k < 3; ++k) {
-      const uint32_t v = in.idx[3 * prim + k];
-      lg[k] = make_float4(in.pos[3 * v], in.pos[3 * v + 1], in.pos[3 * v + 2], 0.0f);
-    }
+    const uint32_t a = 3 * in.idx[3 * prim], b = 3 * in.idx[3 * prim + 1], c = 3 * in.idx[3 * prim + 2];
+    for (int k = 0; k < 3; ++k) lg[k] = make_float4(in.pos[a + k], in.pos[b + k], in.pos[c + k], 0.0f);
   } else if (kind == kSphere) {
     lg[0] = in.sph[prim];
   } else {

@@ -84,8 +84,13 @@ UBR_D bool testKnown(const TravScene& s, int slot, const Ray& r, const TriPre& p
     return isectSphere<ATTR>(r, f3{q.x, q.y, q.z}, q.w, tnear, tmax, h);
   }
   if (KIND == kMesh) {
-    const float4 a = __ldg(g), b = __ldg(g + 1), c = __ldg(g + 2);
-    return isectTriangle(r, pre, ld3(a), ld3(b), ld3(c), tnear, tmax, h);
+    if (!isectTriangle(pre, __ldg(g + pre.kx), __ldg(g + pre.ky), __ldg(g + pre.kz), tnear, tmax, h)) return false;
+    if (ATTR) {
+      const float4 x = __ldg(g), y = __ldg(g + 1), z = __ldg(g + 2);
+      const f3 v0{x.x, y.x, z.x};
+      h.Ng = cross(f3{x.y, y.y, z.y} - v0, f3{x.z, y.z, z.z} - v0);
+    }
+    return true;
   }
   const float4 a = __ldg(g), b = __ldg(g + 1);
   if (KIND == kCone) {
@@ -125,6 +130,17 @@ UBR_D uint32_t leafBytes(int kind) {
 struct Count {
   uint32_t nodes = 0, primBytes = 0;
 };
+
+// Slots of `primMask` that hold primitives of the scene's higher kind.
+template <int KM>
+UBR_D uint32_t highKindSlots(const TravScene& s, int primBase, uint32_t primMask) {
+  uint32_t mask = 0;
+  for (uint32_t m = primMask; m; m &= m - 1u) {
+    const int q = __ffs(m) - 1;
+    if (refKind(__ldg(&s.leafRef[primBase + q])) == highKind(KM)) mask |= 1u << q;
+  }
+  return mask;
+}
 
 // One kind's any-hit tests over the primitive slots of `mask` (a phase of
 // the kind-split leaf loop): true at the first hit.
@@ -301,6 +317,41 @@ UBR_D void travInit(const Ray& r, TravState& st, Hit& best, int start = 0) {
   best.ref = kInvalid;
 }
 
+// A candidate hit of a primitive: the answer of an any-hit query (true), else
+// kept when it is nearer (ties to the lowest ids).
+UBR_D bool takeHit(const TravScene& s, const Hit& h, uint32_t ref, int kind, bool any, TravState& st, Hit& best) {
+  if (any) {
+    best = h;
+    best.ref = ref;
+    return true;
+  }
+  const uint32_t gid = s.geomID[kind], prim = refPrim(ref);
+  const bool better = best.ref == kInvalid || h.t < best.t ||
+                      (h.t == best.t && (gid < st.bestGeom || (gid == st.bestGeom && prim < st.bestPrim)));
+  if (better) {
+    best = h;
+    best.ref = ref;
+    st.bestGeom = gid;
+    st.bestPrim = prim;
+    st.tmax = h.t;
+  }
+  return false;
+}
+
+// One kind's tests of a query that reports its hit (the kind-split leaf loop).
+template <bool COUNT, int KIND>
+UBR_D bool closestPhase(const TravScene& s, const Ray& r, const TriPre& pre, int primBase, uint32_t mask, TravState& st,
+                        Hit& best, Count* cnt, bool any) {
+  for (; mask; mask &= mask - 1u) {
+    const int q = __ffs(mask) - 1;
+    if (COUNT) cnt->primBytes += leafBytes(KIND);
+    Hit h;
+    if (!testKnown<KIND, true>(s, primBase + q, r, pre, r.tnear, st.tmax, h, kInvalid)) continue;
+    if (takeHit(s, h, __ldg(&s.leafRef[primBase + q]), KIND, any, st, best)) return true;
+  }
+  return false;
+}
+
 // Visit st.node: test its 8 children, its hit leaves' primitives, choose the
 // next node.  Returns true when the ray is finished (any-hit found, stack
 // empty, or the step bound reached).
@@ -378,25 +429,27 @@ UBR_D bool travStep(const TravScene& s, const Ray& r, const f3& inv, const TriPr
   const uint32_t hitInt = ~neg & link & 0xFFu;
   uint32_t primMask = leafPrims(s, st.node, ~neg & __float_as_uint(n1.z) & 0xFFu);
   const int nearK = nearestChild(tminP, hitInt);
-  // primitives of the hit leaves.  Binary any-hit queries (no filter) of a
-  // scene of two analytic kinds split them by kind: all lanes of a warp test
-  // one kind, then the other (a mixed loop runs both intersectors in every
-  // step where the lanes' kinds differ; spheres and capped cylinders of a
-  // ball-and-stick model mix in most leaves: -1.3 % in the occlusion kernel).
-  // Not with triangles: a surface with a few atoms rarely mixes, and the pass
-  // over the references costs more than it saves (+3.9 %).  A one-kind scene
-  // reads no primitive references.
-  constexpr bool kSplit = ALWAYS_ANY && !FILTER && kindCount(KM) == 2 && !(KM & kMaskMesh);
+  // primitives of the hit leaves.  A scene of two analytic kinds tests them in
+  // two phases (no filter): all lanes of a warp test one kind, then the other
+  // (a mixed loop runs both intersectors in every step where the lanes' kinds
+  // differ; spheres and capped cylinders of a ball-and-stick model mix in most
+  // leaves: -1.3 % in the occlusion kernel, and for closest hits -1.5 % on the
+  // 1920x1080 ss2 frame and -3.3 % on its pt2 GI).  Not with triangles: a
+  // surface with a few atoms rarely mixes, and the pass over the references
+  // costs more than it saves (+3.9 %).  A one-kind scene reads no primitive
+  // references in any-hit queries.
+  constexpr bool kSplit = !FILTER && kindCount(KM) == 2 && !(KM & kMaskMesh);
   constexpr bool kKnown = ALWAYS_ANY && !FILTER && kindCount(KM) == 1;
   if (kSplit) {
-    uint32_t maskHigh = 0;
-    for (uint32_t m = primMask; m; m &= m - 1u) {
-      const int q = __ffs(m) - 1;
-      if (refKind(__ldg(&s.leafRef[primBase + q])) == highKind(KM)) maskHigh |= 1u << q;
-    }
-    if (anyHitPhase<COUNT, lowKind(KM)>(s, r, pre, primBase, primMask & ~maskHigh, st.tmax, best, cnt) ||
-        anyHitPhase<COUNT, highKind(KM)>(s, r, pre, primBase, maskHigh, st.tmax, best, cnt))
+    const uint32_t high = highKindSlots<KM>(s, primBase, primMask), low = primMask & ~high;
+    if (ALWAYS_ANY) {
+      if (anyHitPhase<COUNT, lowKind(KM)>(s, r, pre, primBase, low, st.tmax, best, cnt) ||
+          anyHitPhase<COUNT, highKind(KM)>(s, r, pre, primBase, high, st.tmax, best, cnt))
+        return true;
+    } else if (closestPhase<COUNT, lowKind(KM)>(s, r, pre, primBase, low, st, best, cnt, any) ||
+               closestPhase<COUNT, highKind(KM)>(s, r, pre, primBase, high, st, best, cnt, any)) {
       return true;
+    }
     primMask = 0;
   } else if (kKnown) {
     if (anyHitPhase<COUNT, lowKind(KM)>(s, r, pre, primBase, primMask, st.tmax, best, cnt)) return true;
@@ -422,22 +475,7 @@ UBR_D bool travStep(const TravScene& s, const Ray& r, const f3& inv, const TriPr
       }
       if (!second) continue;
     }
-    if (any) {
-      best = h;
-      best.ref = ref;
-      return true;
-    }
-    const int kind = refKind(ref);
-    const uint32_t gid = s.geomID[kind], prim = refPrim(ref);
-    const bool better = best.ref == kInvalid || h.t < best.t ||
-                        (h.t == best.t && (gid < st.bestGeom || (gid == st.bestGeom && prim < st.bestPrim)));
-    if (better) {
-      best = h;
-      best.ref = ref;
-      st.bestGeom = gid;
-      st.bestPrim = prim;
-      st.tmax = h.t;
-    }
+    if (takeHit(s, h, ref, refKind(ref), any, st, best)) return true;
   }
   if (nearK >= 0) {
     const uint32_t rest = hitInt & ~(1u << nearK);
@@ -468,7 +506,7 @@ __device__ bool traverse(const TravScene& s, const Ray& r, Hit& best, uint32_t& 
   if (s.primCount == 0 || start < 0) return false;
   const f3 inv = safeInv(r.dir);
   TriPre pre;
-  if (KM & kMaskMesh) pre = triPre(r.dir);
+  if (KM & kMaskMesh) pre = triPre(r.dir, r.org);
   TravState st;
   travInit(r, st, best, start);
   while (!travStep<COUNT, KM, ALWAYS_ANY, FILTER>(s, r, inv, pre, st, best, overflow, cnt, any, top, nTop, flt)) {
@@ -490,7 +528,7 @@ __device__ bool traverseAnyInterleaved(const TravScene& s, const Ray& r, uint32_
   if (s.primCount == 0 || start < 0) return false;
   const f3 inv = safeInv(r.dir);
   TriPre pre;
-  if (KM & kMaskMesh) pre = triPre(r.dir);
+  if (KM & kMaskMesh) pre = triPre(r.dir, r.org);
   int node = start, sp = 0, pendBase = 0;
   uint32_t pendMask = 0, steps = 0;
   uint32_t stack[kStackDepth];
