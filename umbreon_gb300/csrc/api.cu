@@ -1,8 +1,8 @@
 // api.cu -- the extern "C" entry points of libubr (declared in include/ubr.h).
 // The C-ABI never throws: every failure is a ubr_status plus a message kept
 // on the context (ubr_context_last_error).
-#include <cstdio>
 #include <algorithm>
+#include <cstdio>
 #include <cstring>
 #include <new>
 #include <string>
@@ -42,14 +42,15 @@ ubr_status cudaFail(Context* c, cudaError_t e, const char* what) {
   return setError(c, e == cudaErrorMemoryAllocation ? UBR_OUT_OF_MEMORY : UBR_CUDA_ERROR, m);
 }
 
-ubr_status devAlloc(Context* c, DevBuf& b, size_t bytes) {
+ubr_status devAlloc(Context* c, DevBuf& b, size_t bytes, bool direct) {
   if (bytes == 0) bytes = 16;
   if (c->arenaCap && c->arenaUsed + bytes > c->arenaCap)
     return setError(c, UBR_OUT_OF_MEMORY, "device arena cap exceeded");
   void* p = nullptr;
   // stream-ordered from the context's pool: after the first frames a scene
   // build or a scratch growth reuses pooled memory instead of cudaMalloc
-  cudaError_t e = c->pool ? cudaMallocFromPoolAsync(&p, bytes, c->pool, c->stream) : cudaMalloc(&p, bytes);
+  b.direct = direct || !c->pool;
+  cudaError_t e = b.direct ? cudaMalloc(&p, bytes) : cudaMallocFromPoolAsync(&p, bytes, c->pool, c->stream);
   if (e != cudaSuccess) return cudaFail(c, e, "device allocation");
   b.ptr = p;
   b.bytes = bytes;
@@ -59,15 +60,21 @@ ubr_status devAlloc(Context* c, DevBuf& b, size_t bytes) {
 
 void devFree(Context* c, DevBuf& b) {
   if (b.ptr) {
-    if (c->pool) cudaFreeAsync(b.ptr, c->stream);
-    else cudaFree(b.ptr);
+    if (b.direct) cudaFree(b.ptr);
+    else cudaFreeAsync(b.ptr, c->stream);
     c->arenaUsed -= b.bytes;
   }
   b.ptr = nullptr;
   b.bytes = 0;
 }
 
-ubr_status scratchGet(Context* c, int i, size_t bytes, void** out) {
+// Scratch blocks from this size on come from cudaMalloc: a new pool grows by
+// about 65 us plus 0.8 us per MB (128 MB 155 us, 512 MB 460 us), cudaMalloc
+// takes 60-110 us at any size, and a block of the scratch lives as long as its
+// context.  Scenes stay in the pool, which hands freed blocks on in 2 us.
+constexpr size_t kDirectBytes = size_t(96) << 20;
+
+ubr_status scratchGet(Context* c, int i, size_t bytes, void** out, bool slack) {
   if (size_t(i) >= c->scratch.size()) c->scratch.resize(size_t(i) + 1);
   DevBuf& b = c->scratch[size_t(i)];
   if (b.bytes < bytes) {
@@ -75,11 +82,42 @@ ubr_status scratchGet(Context* c, int i, size_t bytes, void** out) {
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cudaFail(c, e, "cudaStreamSynchronize");
     devFree(c, b);
-    ubr_status st = devAlloc(c, b, bytes + bytes / 4);
+    const size_t grown = slack ? bytes + bytes / 4 : bytes;
+    ubr_status st = devAlloc(c, b, grown, grown >= kDirectBytes);
     if (st != UBR_OK) return st;
   }
   *out = b.ptr;
   return UBR_OK;
+}
+
+ubr_status workspaceMin(Context* c, void** out, size_t* bytes) {
+  if (!c->workMin) UBR_CUDA(c, cudaMalloc(&c->workMin, kWorkspaceMin));
+  *out = c->workMin;
+  *bytes = kWorkspaceMin;
+  return UBR_OK;
+}
+
+ubr_status workspaceGet(Context* c, int slot, size_t least, void** out, size_t* bytes) {
+  if (c->arenaCap == 0) {
+    if (scratchGet(c, slot, *bytes, out) == UBR_OK) return UBR_OK;
+    cudaGetLastError();
+  }
+  const DevBuf* lend = nullptr;
+  for (int k = 16; k <= 31 && size_t(k) < c->scratch.size(); ++k)
+    if (c->scratch[size_t(k)].ptr && (!lend || c->scratch[size_t(k)].bytes > lend->bytes)) lend = &c->scratch[size_t(k)];
+  if (lend && lend->bytes >= std::max(least, kWorkspaceMin)) {
+    *out = lend->ptr;
+    *bytes = std::min(*bytes, lend->bytes);
+    return UBR_OK;
+  }
+  if (least <= kWorkspaceMin) {
+    const size_t want = *bytes;
+    const ubr_status st = workspaceMin(c, out, bytes);
+    *bytes = std::min(*bytes, std::max(want, least));
+    return st;
+  }
+  *bytes = least;
+  return scratchGet(c, slot, least, out);
 }
 
 }  // namespace ubr
@@ -227,7 +265,7 @@ ubr_status ubr_context_destroy(ubr_context* c) {
   for (cudaEvent_t& e : x.giEv)
     if (e) cudaEventDestroy(e);
   if (x.graphExec) cudaGraphExecDestroy(x.graphExec);
-  if (x.gatherMin) cudaFree(x.gatherMin);
+  if (x.workMin) cudaFree(x.workMin);
   if (x.pinned) cudaFreeHost(x.pinned);
   if (x.ownStream && x.stream) cudaStreamDestroy(x.stream);
   delete c;

@@ -457,7 +457,8 @@ struct GiWave {
   float4* thr;        // several bounces: (throughput, hit t) and
   float4* pos;        //   (position, -) of a record
   float4* path[4];    // several bounces: (org,tnear)|(dir,slot)|(throughput,s0)|(s1 bits,-,-,-)
-  float4* shadow;     // (direction, record * nLights + light)
+  uint32_t* shadow;   // record * nLights + light
+  float4* shadowDir;  // area lights: the jittered direction (else the light's)
   uint8_t* vis;       // per record and light: 1 = occluded
   uint2* rng;         // emitters: per slot, the stream where its path ended
   float4* cand;       // ReSTIR: per slot (candidate position, -) (normal, cos at the origin, < 0: none)
@@ -577,7 +578,7 @@ __global__ void __launch_bounds__(128, 8) k_gather_first(GiP g, DScene s, GiGrid
     f3 candPos{0.0f, 0.0f, 0.0f};
     bool escaped = false;
     if (horizonOk) {
-      traverse<false, KM>(travOf(s), Ray{O, wi, eps, g.maxDist}, h, ovf, nullptr, false);
+      traverse<false, KM, false, false, true>(travOf(s), Ray{O, wi, eps, g.maxDist}, h, ovf, nullptr, false);
       rays = 1;
       push = h.ref != kInvalid;
       if (!push) {
@@ -621,7 +622,7 @@ __global__ void __launch_bounds__(128, 8) k_gather_next(GiP g, DScene s, GiWave 
   if (i < w.ctr[3]) {
     a = w.path[0][i];
     b = w.path[1][i];
-    traverse<false, KM>(travOf(s), Ray{ld3(a), ld3(b), a.w, g.maxDist}, h, ovf, nullptr, false);
+    traverse<false, KM, false, false, true>(travOf(s), Ray{ld3(a), ld3(b), a.w, g.maxDist}, h, ovf, nullptr, false);
     rays = 1;
     c = w.path[2][i];
     s1 = __float_as_uint(w.path[3][i].x);
@@ -726,7 +727,8 @@ __global__ void __launch_bounds__(128) k_gather_vertex(GiP g, DScene s, const Li
     int off;
     const uint32_t e = uint32_t(warpPushBase(lit, w.ctr + 2, off) + off);
     if (lit) {
-      w.shadow[e] = make_float4(dir.x, dir.y, dir.z, __uint_as_float(q * uint32_t(nLights) + uint32_t(l)));
+      w.shadow[e] = q * uint32_t(nLights) + uint32_t(l);
+      if (w.shadowDir) w.shadowDir[e] = make_float4(dir.x, dir.y, dir.z, 0.0f);
       ++nee;
     }
   }
@@ -740,15 +742,16 @@ __global__ void __launch_bounds__(128) k_gather_vertex(GiP g, DScene s, const Li
 
 // Visibility of the queued shadow rays.
 template <int KM>
-__global__ void __launch_bounds__(128, (KM & kMaskMesh) ? 8 : 9) k_gather_shadow(GiP g, DScene s, int nLights, GiWave w) {
+__global__ void __launch_bounds__(128, (KM & kMaskMesh) ? 8 : 9) k_gather_shadow(GiP g, DScene s, const LightD* lights,
+                                                                                  int nLights, GiWave w) {
   const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t ovf = 0;
   if (e < w.ctr[2]) {
-    const float4 d = w.shadow[e];
-    const uint32_t code = __float_as_uint(d.w);
-    const float4 o = w.r[0][code / uint32_t(nLights)];
+    const uint32_t code = w.shadow[e], q = code / uint32_t(nLights);
+    const float4 o = w.r[0][q];
+    const f3 d = w.shadowDir ? ld3(w.shadowDir[e]) : lights[code - q * uint32_t(nLights)].L;
     Hit h;
-    w.vis[code] = traverse<false, KM, true>(travOf(s), Ray{ld3(o), ld3(d), o.w, kInfF}, h, ovf, nullptr, true) ? 1 : 0;
+    w.vis[code] = traverse<false, KM, true>(travOf(s), Ray{ld3(o), d, o.w, kInfF}, h, ovf, nullptr, true) ? 1 : 0;
   }
   warpCount(g.overflow, ovf);
 }
@@ -1002,7 +1005,7 @@ __global__ void __launch_bounds__(128) k_gbuffer(Params p, DScene s, int w, int 
     Ray r{org, rd, 0.0f, kInfF};
     Hit hh;
     Count cnt;
-    traverse<false, KM>(travOf(s), r, hh, ovf, &cnt, false);
+    traverse<false, KM, false, false, true>(travOf(s), r, hh, ovf, &cnt, false);
     traced = 1;
     float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a, c = a;
     if (hh.ref != kInvalid) {
@@ -1594,7 +1597,7 @@ UBR_D f3 reflectedRadiance(const GiP& g, const DScene& s, const LightD* lights, 
   Ray r{O, d, tn, kInfF};
   Hit h;
   Count cnt;
-  traverse<false, KM>(travOf(s), r, h, ovf, &cnt, false);
+  traverse<false, KM, false, false, true>(travOf(s), r, h, ovf, &cnt, false);
   ++rays;
   if (h.ref == kInvalid) return giEnvironment(g, d);
   tea2(r0, r1);
@@ -1838,29 +1841,29 @@ void giGBuffer(int km, cudaStream_t s, const Params& p, const DScene& sc, int w,
 static int gatherLogLanes(const GiP& g, int spp) { return g.rsv ? 0 : spp >= 8 ? 3 : spp >= 4 ? 2 : spp >= 2 ? 1 : 0; }
 
 // Bytes a slot takes in each array of the workspace, in GiWave's order.
-static size_t gatherSlotBytes(const GiP& g, int nLights) {
+static size_t gatherSlotBytes(const GiP& g, int nLights, bool area) {
   const size_t nl = size_t(std::max(nLights, 0));
   const bool lean = g.bounces <= 1 && !(g.pt2 && g.em.n > 0);
-  return 16 + (lean ? 48 : 64) + (g.bounces > 1 ? 32 + 64 : 0) + nl * 17 + (g.pt2 && g.em.n > 0 ? 8 : 0) + (g.rsv ? 32 : 0);
+  return 16 + (lean ? 48 : 64) + (g.bounces > 1 ? 32 + 64 : 0) + nl * (area ? 21 : 5) + (g.pt2 && g.em.n > 0 ? 8 : 0) + (g.rsv ? 32 : 0);
 }
 constexpr size_t kWaveHeader = 256, kWaveAlign = 256, kWaveArrays = 20;
 // A chunk: enough rays that its first and last wave of blocks weigh little, in
-// a workspace of the size of a frame's own buffers (0.5 GB with two lights):
+// a workspace of the size of a frame's own buffers (0.3 GB with two lights):
 // 2^20 slots are 8 % slower on the pt2 default frame, 2^24 1.5 % faster.
 constexpr uint64_t kWaveSlots = 1u << 22;
 constexpr size_t kWaveBytes = size_t(1) << 30;
 
-size_t giGatherBytes(const GiP& g, int nLights, uint64_t n, int spp) {
+size_t giGatherBytes(const GiP& g, int nLights, bool area, uint64_t n, int spp) {
   const int lg = gatherLogLanes(g, spp);
   const uint64_t P = 32u >> lg, iters = (uint64_t(std::max(spp, 1)) + (1u << lg) - 1) >> lg;
   const uint64_t slots = (n + P - 1) / P * iters * 32u;
-  const size_t sb = gatherSlotBytes(g, nLights);
+  const size_t sb = gatherSlotBytes(g, nLights, area);
   const uint64_t cap = std::min<uint64_t>(kWaveSlots, kWaveBytes / sb);
-  return std::max(kGatherMinBytes, kWaveHeader + kWaveArrays * kWaveAlign + size_t(std::min(slots, cap)) * sb);
+  return std::max(kGatherMin, kWaveHeader + kWaveArrays * kWaveAlign + size_t(std::min(slots, cap)) * sb);
 }
 
 cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, const LightD* lights, int nLights,
-                     const GiGrid& grid, const uint32_t* list, const uint32_t* listCount, uint32_t n, int spp,
+                     bool area, const GiGrid& grid, const uint32_t* list, const uint32_t* listCount, uint32_t n, int spp,
                      float4* E, uint32_t* listBuf, void* ws, size_t wsBytes, uint32_t* hostCount,
                      uint32_t* launches) {
   if (n == 0) return cudaSuccess;
@@ -1870,7 +1873,7 @@ cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, con
   w.logLanes = gatherLogLanes(g, spp);
   const uint32_t P = 32u >> w.logLanes;
   w.itEnd = std::max(1, (w.spp + (1 << w.logLanes) - 1) >> w.logLanes);
-  const size_t sb = gatherSlotBytes(g, nLights);
+  const size_t sb = gatherSlotBytes(g, nLights, area);
   const size_t carryBytes = size_t(kCarryF4) * 16 * 32;  // windows run one group at a time
   const size_t room = std::min<size_t>(wsBytes - kWaveHeader - kWaveArrays * kWaveAlign, kWaveSlots * sb);
   uint64_t groupsFit = room / (size_t(w.itEnd) * 32u * sb);
@@ -1925,7 +1928,8 @@ cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, con
     for (float4*& p : w.path) p = f4();
   }
   const size_t nl = size_t(std::max(nLights, 0));
-  w.shadow = reinterpret_cast<float4*>(take(size_t(slotCap) * nl * 16));
+  w.shadow = reinterpret_cast<uint32_t*>(take(size_t(slotCap) * nl * 4));
+  if (area) w.shadowDir = reinterpret_cast<float4*>(take(size_t(slotCap) * nl * 16));
   w.vis = reinterpret_cast<uint8_t*>(take(size_t(slotCap) * nl));
   if (emit) w.rng = reinterpret_cast<uint2*>(take(size_t(slotCap) * 8));
   if (g.rsv) w.cand = reinterpret_cast<float4*>(take(size_t(slotCap) * 32));
@@ -1951,7 +1955,7 @@ cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, con
         k_gather_vertex<<<blocks(slots, 128), 128, 0, s>>>(g, sc, lights, nLights, grid, pts, w, b);
         if (nl > 0)
           byKind(km, [&](auto K) {
-            k_gather_shadow<decltype(K)::value><<<blocks(slots * nl, 128), 128, 0, s>>>(g, sc, nLights, w);
+            k_gather_shadow<decltype(K)::value><<<blocks(slots * nl, 128), 128, 0, s>>>(g, sc, lights, nLights, w);
           });
         if (b > 1 && b < maxB) {
           e = cudaMemsetAsync(w.ctr + 3, 0, sizeof(uint32_t), s);

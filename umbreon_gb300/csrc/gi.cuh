@@ -100,12 +100,13 @@ void giGBuffer(int km, cudaStream_t s, const Params& p, const DScene& sc, int w,
 // The gather over a grid (list null: its eligible points, listed in listBuf of
 // n; the others get E = 0) or over the points of a list (listCount of them, on
 // the device).  Runs in chunks that fit the workspace ws of wsBytes, at least
-// kGatherMinBytes; giGatherBytes is what n points use well.  Reads the number
+// kGatherMin; giGatherBytes is what n points use well.  Reads the number
 // of points back (hostCount, pinned) when they may need more than one chunk.
-constexpr size_t kGatherMinBytes = size_t(1) << 16;
-size_t giGatherBytes(const GiP& g, int nLights, uint64_t n, int spp);
+// area: some light's shadow rays are jittered (pt2, radius > 0).
+constexpr size_t kGatherMin = size_t(1) << 16;
+size_t giGatherBytes(const GiP& g, int nLights, bool area, uint64_t n, int spp);
 cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, const LightD* lights, int nLights,
-                     const GiGrid& grid, const uint32_t* list, const uint32_t* listCount, uint32_t n, int spp,
+                     bool area, const GiGrid& grid, const uint32_t* list, const uint32_t* listCount, uint32_t n, int spp,
                      float4* E, uint32_t* listBuf, void* ws, size_t wsBytes, uint32_t* hostCount, uint32_t* launches);
 void giDenoiseInit(cudaStream_t s, uint32_t n, float4* E, const float4* ne, uint8_t* valid, float4* irr);
 void giDenoiseAux(cudaStream_t s, int W, int H, const uint8_t* valid, const float4* irr, const float4* pd,

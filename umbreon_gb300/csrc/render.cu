@@ -90,24 +90,6 @@ struct Bufs {
 // coordinate table of a fine-lattice pass.
 UBR_D uint32_t latticeOf(const Bufs& b, uint32_t gpix) { return b.coord ? __ldg(&b.coord[gpix]) : gpix; }
 
-// Pixel of slot i in a grid frame's first round (all W x H hi-res pixels, no
-// queue): 8 x 4 pixel tiles in slot order, so a warp's primary rays are a
-// compact bundle and the hits queued after them stay neighbours (a warp of
-// one light's shadow rays covers a tile); the columns and rows that do not
-// fill a tile follow in row order.  A bijection on [0, W H).
-UBR_D uint32_t tiledPixel(uint32_t i, uint32_t W, uint32_t H) {
-  const uint32_t fw = W & ~7u, fh = H & ~3u, nt = fw * fh;
-  if (i < nt) {
-    const uint32_t t = i >> 5, k = i & 31u, tilesX = fw >> 3;
-    return ((t / tilesX) * 4u + (k >> 3)) * W + (t % tilesX) * 8u + (k & 7u);
-  }
-  uint32_t j = i - nt;
-  const uint32_t rw = W - fw;  // right strip of rows [0, fh)
-  if (j < rw * fh) return (j / rw) * W + fw + j % rw;
-  j -= rw * fh;
-  return fh * W + j;  // bottom rows
-}
-
 // AO of a coarse grid cell or of an interpolated lookup: openness and the
 // quality-estimator channels (neutral when not gathered).
 struct AoQ {
@@ -242,7 +224,7 @@ __global__ void __launch_bounds__(128, 8) k_trace_closest(Params p1, DScene s1, 
     Ray r{org, rd, layer == 0 ? ctn : b.tnear[gpix], ctf};
     Hit h;
     const TravScene ts = travOf(s);
-    traverse<COUNT, KM>(ts, r, h, ovf, &cnt, false);
+    traverse<COUNT, KM, false, false, true>(ts, r, h, ovf, &cnt, false);
     traced = 1;
     b.hitA[i] = make_float4(h.t, h.u, h.v, __uint_as_float(h.ref));
     b.hitB[i] = make_float4(h.Ng.x, h.Ng.y, h.Ng.z, 0.0f);
@@ -1550,7 +1532,7 @@ __global__ void __launch_bounds__(128) k_cao_trace(Params pc, DScene s, Bufs b, 
     Hit h;
     uint32_t ovf = 0;
     Count cnt;
-    traverse<false, KM>(travOf(s), r, h, ovf, &cnt, false);
+    traverse<false, KM, false, false, true>(travOf(s), r, h, ovf, &cnt, false);
     uint8_t eligible = 0;
     f3 N{0.0f, 0.0f, 0.0f}, Ng{0.0f, 0.0f, 0.0f};
     if (h.ref != kInvalid) {
@@ -1672,14 +1654,14 @@ __global__ void __launch_bounds__(128) k_gb_clip(Params p, DScene s, Bufs b, uin
       const float t0 = fmaxf(1.0e-4f, 1.0e-6f * ctn), t1 = ctn * (1.0f - 1.0e-6f);
       if (t0 < t1) {
         Hit h;
-        if (traverse<false, KM>(ts, Ray{org, rd, t0, t1}, h, ovf, &cnt, false)) b.gbNear[i] = h.t * camCos;
+        if (traverse<false, KM, false, false, true>(ts, Ray{org, rd, t0, t1}, h, ovf, &cnt, false)) b.gbNear[i] = h.t * camCos;
       }
     }
     if (ctf < kInfF) {
       const float t0 = ctf * (1.0f + 1.0e-6f);
       if (t0 < kInfF) {
         Hit h;
-        if (traverse<false, KM>(ts, Ray{org, rd, t0, kInfF}, h, ovf, &cnt, false)) b.gbFar[i] = h.t * camCos;
+        if (traverse<false, KM, false, false, true>(ts, Ray{org, rd, t0, kInfF}, h, ovf, &cnt, false)) b.gbFar[i] = h.t * camCos;
       }
     }
   }
@@ -2694,6 +2676,8 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
     gp.pattern = d0.pt2_pattern;
     gp.emissive = (pt2 && d0.pt2_emissive) ? 1 : 0;
     gp.em = (pt2 && d0.pt2_emissive && d0.pt2_emissive_nee) ? jobs[0].scene->emit : EmitD{};
+    bool area = false;
+    for (int l = 0; l < nL; ++l) area = area || (pt2 && lights[size_t(p1.lightOff + l)].radius > 0.0f);
     gp.sampleOffset = 0;
     gp.halfE = nullptr;
     gp.rsv = nullptr;
@@ -2743,24 +2727,25 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
     // frame of few pixels, a small block outside the cap
     auto gather = [&](const GiP& gg, const GiGrid& gr, const uint32_t* list, const uint32_t* cnt, uint32_t n, int nspp,
                       float4* E) -> ubr_status {
-      const size_t want = giGatherBytes(gg, nL, n, nspp);
+      // (a list names the points on the device: room for a sixteenth of the
+      // grid, about what edges and noise take, and more chunks past that)
+      const size_t want = giGatherBytes(gg, nL, area, list ? n / 16 + 32 : n, nspp);
       void* ws = nullptr;
       size_t bytes = want;
-      if (c->arenaCap == 0 && scratchGet(c, 149, want, &ws) != UBR_OK) {
+      if (c->arenaCap == 0 && scratchGet(c, 149, want, &ws, false) != UBR_OK) {
         cudaGetLastError();
         ws = nullptr;
       }
       if (!ws) {
         ws = b.hitA;
         bytes = size_t(nslot) * sizeof(float4);
-        if (bytes < kGatherMinBytes) {
-          if (!c->gatherMin) UBR_CUDA(c, cudaMalloc(&c->gatherMin, kGatherMinBytes));
-          ws = c->gatherMin;
-          bytes = kGatherMinBytes;
+        if (bytes < kWorkspaceMin) {
+          const ubr_status ms = workspaceMin(c, &ws, &bytes);
+          if (ms != UBR_OK) return ms;
         }
       }
       // the eligible points of a grid are listed in the first queue buffer
-      UBR_CUDA(c, giGather(km, s, gg, s1, lt, nL, gr, list, cnt, n, nspp, E, q0, ws, bytes, hostCount + 8, &kernels));
+      UBR_CUDA(c, giGather(km, s, gg, s1, lt, nL, area, gr, list, cnt, n, nspp, E, q0, ws, bytes, hostCount + 8, &kernels));
       return UBR_OK;
     };
     // the gather over a grid, with pt2's adaptive refinement (pt2_adaptive.hpp:

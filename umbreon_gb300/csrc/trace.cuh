@@ -34,6 +34,24 @@ UBR_D void primaryRay(const Params& p, int px, int py, f3& org, f3& rd) {
   }
 }
 
+// Pixel of slot i in a grid frame's first round (all W x H hi-res pixels, no
+// queue): 8 x 4 pixel tiles in slot order, so a warp's primary rays are a
+// compact bundle and the hits queued after them stay neighbours (a warp of
+// one light's shadow rays covers a tile); the columns and rows that do not
+// fill a tile follow in row order.  A bijection on [0, W H).
+UBR_D uint32_t tiledPixel(uint32_t i, uint32_t W, uint32_t H) {
+  const uint32_t fw = W & ~7u, fh = H & ~3u, nt = fw * fh;
+  if (i < nt) {
+    const uint32_t t = i >> 5, k = i & 31u, tilesX = fw >> 3;
+    return ((t / tilesX) * 4u + (k >> 3)) * W + (t % tilesX) * 8u + (k & 7u);
+  }
+  uint32_t j = i - nt;
+  const uint32_t rw = W - fw;  // right strip of rows [0, fh)
+  if (j < rw * fh) return (j / rw) * W + fw + j % rw;
+  j -= rw * fh;
+  return fh * W + j;  // bottom rows
+}
+
 // clipRangeT (transparency.hpp:118-129)
 UBR_D void clipRange(const Params& p, f3 rd, float& tn, float& tf) {
   tn = 0.0f;
@@ -208,20 +226,24 @@ UBR_D f2x mul2(f2x a, f2x b) {
 // Bounds b and b+1 of q as a float pair.
 UBR_D f2x boundPair(uint32_t q, int b) { return pk2(boundValue(q, b), boundValue(q, b + 1)); }
 
-// Slot of the nearest hit internal child (-1: none): the smallest key among
-// the hit slots, a key being the entry distance's bits with the slot in the
-// low three bits (one integer min per child instead of a compare and two
-// selects).  Non-negative floats order as unsigned integers; distances within
-// 8 ulps go to the lower slot.  The visiting order never changes an answer:
-// an any-hit query reports whether some primitive is hit, a closest-hit query
-// the nearest hit with ties to the lowest ids.
-UBR_D int nearestChild(const float (&tmin)[8], uint32_t hitInt) {
+// Nearest of the given hit slots, and the slot of the nearest hit internal
+// child (-1: none): the smallest key, a key being the entry distance's bits
+// with the slot in the low three bits (one integer min per child instead of a
+// compare and two selects).  Non-negative floats order as unsigned integers;
+// distances within 8 ulps go to the lower slot.  The visiting order never
+// changes an answer: an any-hit query reports whether some primitive is hit, a
+// closest-hit query the nearest hit with ties to the lowest ids.
+UBR_D uint32_t nearestKey(const float (&tmin)[8], uint32_t slots) {
   uint32_t best = 0xFFFFFFFFu;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const uint32_t key = (__float_as_uint(tmin[k]) & ~7u) | uint32_t(k);
-    best = ((hitInt >> k) & 1u) ? min(best, key) : best;
+    best = ((slots >> k) & 1u) ? min(best, key) : best;
   }
+  return best;
+}
+UBR_D int nearestChild(const float (&tmin)[8], uint32_t hitInt) {
+  const uint32_t best = nearestKey(tmin, hitInt);
   return hitInt ? int(best & 7u) : -1;
 }
 
@@ -305,6 +327,7 @@ struct TravState {
   float tmax;
   uint32_t bestGeom, bestPrim;
   uint32_t stack[kStackDepth];   // group entries: (childBase << 8) | slot mask
+  uint32_t next[kStackDepth];    // CULL: key of the group's nearest child
 };
 
 UBR_D void travInit(const Ray& r, TravState& st, Hit& best, int start = 0) {
@@ -396,7 +419,15 @@ UBR_D bool filterAccept(const HitFilter& f, const Ray& r, const Hit& h, uint32_t
 // memory and pass them as `top` (nTop of them).
 constexpr int kTopNodes = 73;
 
-template <bool COUNT, int KM, bool ALWAYS_ANY = false, bool FILTER = false>
+//
+// CULL (closest hits of rays without a short range): a pushed group keeps the
+// key of its nearest child, which is visited next, and is dropped when the
+// hits found since lie before it; the rest of a group keeps that key as a
+// lower bound.  A third of the node visits of gather rays met nothing, partly
+// in such groups: 2 k sphere pt1 frame 0.544 -> 0.523 ms, pt2 frame 14.55 ->
+// 14.34, batch of 24 9.18 -> 9.03.  Not for AO rays, whose range ends the
+// search anyway: enhanced AO +3.7 %, adjoint +5.2 %.
+template <bool COUNT, int KM, bool ALWAYS_ANY = false, bool FILTER = false, bool CULL = false>
 UBR_D bool travStep(const TravScene& s, const Ray& r, const f3& inv, const TriPre& pre, TravState& st, Hit& best,
                     uint32_t& overflow, Count* cnt, bool any, const float4* top = nullptr, int nTop = 0,
                     const HitFilter* flt = nullptr) {
@@ -480,25 +511,42 @@ UBR_D bool travStep(const TravScene& s, const Ray& r, const f3& inv, const TriPr
   if (nearK >= 0) {
     const uint32_t rest = hitInt & ~(1u << nearK);
     if (rest) {
-      if (st.sp < kStackDepth) st.stack[st.sp++] = (link & ~0xFFu) | rest;
-      else ++overflow;
+      if (st.sp < kStackDepth) {
+        if (CULL) st.next[st.sp] = nearestKey(tminP, rest);
+        st.stack[st.sp++] = (link & ~0xFFu) | rest;
+      } else {
+        ++overflow;
+      }
     }
     st.node = int(link >> 8) + nearK;
     return false;
   }
-  if (st.sp == 0) return true;
-  const uint32_t g = st.stack[st.sp - 1];
-  const uint32_t mask = g & 0xFFu;
-  const int k = __ffs(mask) - 1;
-  const uint32_t left = mask & (mask - 1u);
-  if (left) st.stack[st.sp - 1] = (g & ~0xFFu) | left;
-  else --st.sp;
-  st.node = int(g >> 8) + k;
-  return false;
+  for (;;) {
+    if (st.sp == 0) return true;
+    const uint32_t g = st.stack[st.sp - 1];
+    uint32_t key = 0;
+    if (CULL) {
+      key = st.next[st.sp - 1];
+      if (__uint_as_float(key & ~7u) > st.tmax * kSlabGrow) {
+        --st.sp;
+        continue;
+      }
+    }
+    const int k = CULL ? int(key & 7u) : __ffs(g & 0xFFu) - 1;
+    const uint32_t left = g & ~(1u << k);
+    if (left & 0xFFu) {
+      st.stack[st.sp - 1] = left;
+      if (CULL) st.next[st.sp - 1] = (key & ~7u) | uint32_t(__ffs(left & 0xFFu) - 1);
+    } else {
+      --st.sp;
+    }
+    st.node = int(g >> 8) + k;
+    return false;
+  }
 }
 
 // Whole traversal of one ray (one thread per ray).
-template <bool COUNT = false, int KM = kMaskAll, bool ALWAYS_ANY = false, bool FILTER = false>
+template <bool COUNT = false, int KM = kMaskAll, bool ALWAYS_ANY = false, bool FILTER = false, bool CULL = false>
 __device__ bool traverse(const TravScene& s, const Ray& r, Hit& best, uint32_t& overflow, Count* cnt,
                          const bool any, int start = 0, const float4* top = nullptr, int nTop = 0,
                          const HitFilter* flt = nullptr) {
@@ -509,7 +557,7 @@ __device__ bool traverse(const TravScene& s, const Ray& r, Hit& best, uint32_t& 
   if (KM & kMaskMesh) pre = triPre(r.dir, r.org);
   TravState st;
   travInit(r, st, best, start);
-  while (!travStep<COUNT, KM, ALWAYS_ANY, FILTER>(s, r, inv, pre, st, best, overflow, cnt, any, top, nTop, flt)) {
+  while (!travStep<COUNT, KM, ALWAYS_ANY, FILTER, CULL>(s, r, inv, pre, st, best, overflow, cnt, any, top, nTop, flt)) {
   }
   return best.ref != kInvalid;
 }

@@ -17,6 +17,7 @@ namespace ubr {
 struct DevBuf {
   void* ptr = nullptr;
   size_t bytes = 0;
+  bool direct = false;  // from cudaMalloc, not from the context's pool
 };
 
 struct Context {
@@ -42,7 +43,7 @@ struct Context {
   std::vector<void*> sceneHandles;      // live ubr_scene handles built on this context
   cudaMemPool_t pool = nullptr;         // stream-ordered device allocations (scenes, scratch)
   void* noallocArray = nullptr;         // device address of the allocation-free query's fixed array
-  void* gatherMin = nullptr;            // GI gather workspace of last resort (kGatherMinBytes), on first use
+  void* workMin = nullptr;              // workspace of last resort (kWorkspaceMin bytes), on first use
   cudaEvent_t giEv[7] = {};             // GI pass stage boundaries, created on first use
 };
 
@@ -72,10 +73,21 @@ struct Scene {
 ubr_status setError(Context* c, ubr_status s, const std::string& msg);
 ubr_status cudaFail(Context* c, cudaError_t e, const char* what);
 // allocate `bytes` on the context's device, honouring the arena cap
-ubr_status devAlloc(Context* c, DevBuf& b, size_t bytes);
+// (direct: by cudaMalloc instead of from the context's pool)
+ubr_status devAlloc(Context* c, DevBuf& b, size_t bytes, bool direct = false);
 void devFree(Context* c, DevBuf& b);
-// scratch slot `i` of at least `bytes`
-ubr_status scratchGet(Context* c, int i, size_t bytes, void** out);
+// scratch slot `i` of at least `bytes` (a quarter more when it grows, unless
+// `slack` is false)
+ubr_status scratchGet(Context* c, int i, size_t bytes, void** out, bool slack = true);
+
+// A workspace of a pass that runs in chunks.  *bytes: what it uses well on
+// entry, what it got on exit (at least `least`).  Scratch slot `slot`, or,
+// under an arena cap and where that allocation fails, memory the context holds
+// already: the largest frame buffer that is idle outside a render (slots
+// 16..31), or a small block outside the cap (workspaceMin).
+ubr_status workspaceMin(Context* c, void** out, size_t* bytes);
+ubr_status workspaceGet(Context* c, int slot, size_t least, void** out, size_t* bytes);
+constexpr size_t kWorkspaceMin = size_t(1) << 16;
 
 // typed view of scratch slot `slot` (count elements); a no-op once st != OK
 template <class T>
