@@ -406,6 +406,19 @@ UBR_D void occRayOf(uint64_t rid, uint32_t nq, uint64_t R, uint64_t A, uint32_t&
   }
 }
 
+// An AO ray (origin, direction, range) the centre pass of adaptive AA traced
+// already: its binary result copied.
+UBR_D bool reuseRay(const Params& p, const Bufs& b, uint64_t R, uint32_t slot, uint2 sc, int j) {
+  if (!(b.reuseOcc && j < p.reuseAo && (sc.y & 2u))) return false;
+  const uint32_t pix = latticeOf(b, sc.x);
+  const uint32_t px = pix % uint32_t(p.W), py = pix / uint32_t(p.W);
+  const uint64_t o = uint64_t(py / uint32_t(p.ss)) * uint32_t(p.outW) + px / uint32_t(p.ss);
+  b.occ[uint64_t(slot) * R + j] = b.reuseOcc[o * b.reuseR + j];
+  if (p.aoEnhanced || p.aoWriteAov)
+    b.aoT[uint64_t(slot) * uint64_t(p.aoSamples) + j] = b.reuseAoT[o * uint64_t(p.reuseAo) + j];
+  return true;
+}
+
 // The occlusion kernel's body: one thread per AO / shadow ray.  NEAREST: a
 // frame of the launch wants its AO rays' nearest hits (enhanced AO, AOVs).
 template <bool COUNT, int KM, bool BATCH, bool IL, bool NEAREST>
@@ -425,14 +438,8 @@ __device__ __forceinline__ void occlusionBody(const Params& p1, const DScene& s1
     const int f = BATCH ? int(sc.y >> 8) : 0;
     const Params& p = BATCH ? bt.frames[f].p : p1;
     const DScene& s = BATCH ? bt.frames[f].s : s1;
-    if (!BATCH && b.reuseOcc && j < p.reuseAo && (sc.y & 2u)) {
-      // the same AO ray (origin, direction, range) was traced by the centre
-      // pass: copy its result
-      const uint32_t pix = latticeOf(b, sc.x);
-      const uint32_t px = pix % uint32_t(p.W), py = pix / uint32_t(p.W);
-      const uint64_t o = uint64_t(py / uint32_t(p.ss)) * uint32_t(p.outW) + px / uint32_t(p.ss);
-      b.occ[uint64_t(slot) * R + j] = b.reuseOcc[o * b.reuseR + j];
-      if (p.aoEnhanced || p.aoWriteAov) b.aoT[uint64_t(slot) * aoStride + j] = b.reuseAoT[o * uint64_t(p.reuseAo) + j];
+    if (!BATCH && reuseRay(p, b, R, slot, sc, j)) {
+      // copied from an earlier pass
     } else if (j < p.raysPerHit) {
       const OccRay o = occlusionRay(p, b, slot, BATCH ? sc.x - bt.frames[f].pixOff : latticeOf(b, sc.x), sc.y, j);
       bool hit = false;
@@ -542,10 +549,20 @@ __global__ void __launch_bounds__(128, 8) k_trace_occlusion_gs(Params p1, DScene
 // list with one atomic per warp (dynamic fetch after Aila and Laine,
 // "Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009), so
 // lanes whose rays end early do not wait for the warp's longest ray.
-constexpr int kRefill = 28;  // measured: 8 -> +14 %, 16 -> +6 %, 24 -> 0 %, 32 -> +4 % against 28
+// GENERAL: the traversal that also reports nearest hits, for both kinds of
+// launches (a context's trace mode 2).  With the binary traversal (8 or 9
+// blocks of 128 per SM) it is the faster kernel for many rays through spheres and
+// cylinders (chooseFetch): 20 k ball-and-stick 1920x1080 ss2 frame 7.36 ->
+// 6.69 ms, batch of 24 sphere frames 8.98 -> 8.18.  Refill at 20 / 24 / 28 /
+// 30 idle lanes: figure 6.97 / 6.80 / 6.80 / 6.88 (8 blocks), batch 8.20 /
+// 8.18 / 8.31 / 8.52; blocks per SM 8 / 9 / 10: figure 6.80 / 6.68 / 7.2,
+// batch 8.18 / 8.36 / 8.7 (a batch keeps its frame's scene in registers).
+constexpr int kRefill = 24;
+constexpr int kFetchBlocks = 9, kFetchBlocksBatch = 8, kFetchBlocksGeneral = 8;
 
-template <bool COUNT, int KM, bool BATCH>
-__global__ void __launch_bounds__(128, 8) k_trace_occlusion_persistent(Params p1, DScene s1, Batch bt, Bufs b) {
+template <bool COUNT, int KM, bool BATCH, bool GENERAL>
+__global__ void __launch_bounds__(128, GENERAL ? kFetchBlocksGeneral : BATCH ? kFetchBlocksBatch : kFetchBlocks)
+    k_trace_occlusion_persistent(Params p1, DScene s1, Batch bt, Bufs b) {
   Count cnt;
   uint32_t traced = 0, ovf = 0;
   const uint64_t R = BATCH ? uint64_t(bt.R) : uint64_t(p1.raysPerHit);
@@ -584,6 +601,8 @@ __global__ void __launch_bounds__(128, 8) k_trace_occlusion_persistent(Params p1
           else o.trace = o.grazing = o.ao = false;
           if (j >= p.raysPerHit) {
             // stride padding of a frame with fewer rays per hit: nothing to do
+          } else if (!BATCH && !GENERAL && reuseRay(p, b, R, slot, sc, j)) {
+            // copied from an earlier pass
           } else if (o.trace && s.primCount > 0 && o.start >= 0) {
             ts = travOf(s);
             inv = safeInv(o.r.dir);
@@ -604,9 +623,14 @@ __global__ void __launch_bounds__(128, 8) k_trace_occlusion_persistent(Params p1
       continue;
     }
     if (active) {
-      const Params& p = BATCH ? bt.frames[f].p : p1;
-      if (travStep<COUNT, KM>(ts, o.r, inv, pre, st, best, ovf, &cnt, o.anyHit)) {
-        occlusionWrite(p, b, R, aoStride, slot, j, o, best.ref != kInvalid, best.t);
+      if (GENERAL) {
+        const Params& p = BATCH ? bt.frames[f].p : p1;
+        if (travStep<COUNT, KM>(ts, o.r, inv, pre, st, best, ovf, &cnt, o.anyHit)) {
+          occlusionWrite(p, b, R, aoStride, slot, j, o, best.ref != kInvalid, best.t);
+          active = false;
+        }
+      } else if (travStep<COUNT, KM, true>(ts, o.r, inv, pre, st, best, ovf, &cnt, true)) {
+        b.occ[uint64_t(slot) * R + j] = best.ref != kInvalid ? 1 : 0;
         active = false;
       }
     }
@@ -2054,17 +2078,23 @@ void launchOcclusion(int km, bool count, bool batch, uint32_t grid, int tb, cuda
   else UBR_KM_DISPATCH(k_trace_occlusion, km, count, batch, grid, tb, st, p, s, bt, b, n);
 }
 
-// Resident grid of the persistent occlusion kernel: SMs x resident blocks.
-uint32_t persistentGrid(int device) {
-  static int cached[64] = {};
-  if (device >= 0 && device < 64 && cached[device]) return uint32_t(cached[device]);
-  int sms = 0, perSm = 0;
+uint32_t smCount(int device) {
+  int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_trace_occlusion_persistent<false, kMaskAll, false>, 128,
-                                                0);
-  const int g = std::max(1, sms) * std::max(1, perSm);
-  if (device >= 0 && device < 64) cached[device] = g;
-  return uint32_t(g);
+  return uint32_t(std::max(1, sms));
+}
+
+// Whether a launch of n hits' rays (R each, n counting the misses too, as the
+// host knows it) runs the persistent kernel: binary answers, spheres and
+// cylinders only (with triangles the larger ray state costs 5-10 %), and
+// enough rays.  Ball-and-stick of 5 k atoms, one thread per ray against the
+// persistent kernel: 640x480 with 18 rays (5.5 M) 0.353 / 0.378 ms, 800x600
+// (8.6 M) 0.501 / 0.510, 1024x768 (14 M) 0.723 / 0.700, 1280x720 ss2 (66 M)
+// 2.61 / 2.26.
+constexpr uint64_t kFetchRays = 12000000;
+bool chooseFetch(int mode, int km, bool nearest, uint64_t n, uint64_t R) {
+  if (mode != 0) return mode == 2;
+  return !nearest && !(km & kMaskMesh) && n * R >= kFetchRays;
 }
 
 uint32_t gridStrideGrid(int device) {
@@ -2083,9 +2113,42 @@ void launchOcclusionGridStride(int km, bool count, bool batch, uint32_t grid, in
   UBR_KM_DISPATCH(k_trace_occlusion_gs, km, count, batch, grid, tb, st, p, s, bt, b);
 }
 
-void launchOcclusionPersistent(int km, bool count, bool batch, uint32_t grid, int tb, cudaStream_t st,
-                               const Params& p, const DScene& s, const Batch& bt, const Bufs& b) {
-  UBR_KM_DISPATCH(k_trace_occlusion_persistent, km, count, batch, grid, tb, st, p, s, bt, b);
+template <bool COUNT, int KM, bool BATCH>
+void launchPersistent(bool general, uint32_t sms, cudaStream_t st, const Params& p, const DScene& s, const Batch& bt,
+                      const Bufs& b) {
+  if constexpr ((KM & kMaskMesh) == 0) {
+    if (!general) {
+      const uint32_t blocks = BATCH ? kFetchBlocksBatch : kFetchBlocks;
+      k_trace_occlusion_persistent<COUNT, KM, BATCH, false><<<sms * blocks, 128, 0, st>>>(p, s, bt, b);
+      return;
+    }
+  }
+  k_trace_occlusion_persistent<COUNT, KM, BATCH, true><<<sms * kFetchBlocksGeneral, 128, 0, st>>>(p, s, bt, b);
+}
+
+cudaError_t launchOcclusionPersistent(int km, bool count, bool batch, bool general, int device, cudaStream_t st,
+                                      const Params& p, const DScene& s, const Batch& bt, const Bufs& b) {
+  const cudaError_t e = cudaMemsetAsync(b.cursor, 0, sizeof(unsigned long long), st);
+  if (e != cudaSuccess) return e;
+  const uint32_t sms = smCount(device);
+  auto go = [&](auto K) {
+    constexpr int k = decltype(K)::value;
+    if (count) {
+      if (batch) launchPersistent<true, k, true>(general, sms, st, p, s, bt, b);
+      else launchPersistent<true, k, false>(general, sms, st, p, s, bt, b);
+    } else {
+      if (batch) launchPersistent<false, k, true>(general, sms, st, p, s, bt, b);
+      else launchPersistent<false, k, false>(general, sms, st, p, s, bt, b);
+    }
+  };
+  switch (km) {
+    case kMaskMesh: go(std::integral_constant<int, kMaskMesh>{}); break;
+    case kMaskSphere: go(std::integral_constant<int, kMaskSphere>{}); break;
+    case kMaskMesh | kMaskSphere: go(std::integral_constant<int, kMaskMesh | kMaskSphere>{}); break;
+    case kMaskSphere | kMaskCone: go(std::integral_constant<int, kMaskSphere | kMaskCone>{}); break;
+    default: go(std::integral_constant<int, kMaskAll>{});
+  }
+  return cudaSuccess;
 }
 
 }  // namespace
@@ -2336,7 +2399,7 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
       // low-discrepancy set does): copy them instead of tracing, for single
       // layer frames and the per-ray occlusion kernel
       if (p1.aoSamples > 0 && !p1.aoLowDiscrepancy && !coarseOn && singleLayer &&
-          (c->traceMode == 1 || c->traceMode == 4)) {
+          (c->traceMode != 2 && c->traceMode != 3)) {
         pBoost.reuseAo = p1.aoSamples;
         reuseOccBuf = scratchT<uint8_t>(c, 105, size_t(nCentre) * R, st);
         if (p1.aoEnhanced || p1.aoWriteAov) reuseAoTBuf = scratchT<float>(c, 106, size_t(nCentre) * p1.aoSamples, st);
@@ -2426,15 +2489,13 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
       mark(1, false);
       const uint64_t nr = uint64_t(n) * uint64_t(Rr);
       mark(2, true);
-      if (c->traceMode == 1 || c->traceMode == 4) {
+      if (chooseFetch(c->traceMode, km, nearest, n, Rr))
+        UBR_CUDA(c, launchOcclusionPersistent(km, count, batch, c->traceMode == 2, c->device, s, pr, s1, bt, br));
+      else if (c->traceMode == 3)
+        launchOcclusionGridStride(km, count, batch, gridStrideGrid(c->device), TB, s, pr, s1, bt, br);
+      else
         launchOcclusion(km, count, batch, uint32_t((nr + TB - 1) / TB), TB, s, pr, s1, bt, br, n,
                         c->traceMode == 4, nearest);
-      } else if (c->traceMode == 3) {
-        launchOcclusionGridStride(km, count, batch, gridStrideGrid(c->device), TB, s, pr, s1, bt, br);
-      } else {
-        UBR_CUDA(c, cudaMemsetAsync(br.cursor, 0, sizeof(unsigned long long), s));
-        launchOcclusionPersistent(km, count, batch, persistentGrid(c->device), TB, s, pr, s1, bt, br);
-      }
       mark(2, false);
       kernels += 2;
     }
@@ -2457,15 +2518,13 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
     mark(1, false);
     const uint64_t nr = uint64_t(nCell) * uint64_t(pCoarse.raysPerHit);
     mark(2, true);
-    if (c->traceMode == 1 || c->traceMode == 4) {
+    if (chooseFetch(c->traceMode, km, nearest, nCell, uint64_t(pCoarse.raysPerHit)))
+      UBR_CUDA(c, launchOcclusionPersistent(km, count, false, c->traceMode == 2, c->device, s, pCoarse, s1, bt, b));
+    else if (c->traceMode == 3)
+      launchOcclusionGridStride(km, count, false, gridStrideGrid(c->device), TB, s, pCoarse, s1, bt, b);
+    else
       launchOcclusion(km, count, false, uint32_t((nr + TB - 1) / TB), TB, s, pCoarse, s1, bt, b, nCell,
                       c->traceMode == 4, nearest);
-    } else if (c->traceMode == 3) {
-      launchOcclusionGridStride(km, count, false, gridStrideGrid(c->device), TB, s, pCoarse, s1, bt, b);
-    } else {
-      UBR_CUDA(c, cudaMemsetAsync(b.cursor, 0, sizeof(unsigned long long), s));
-      launchOcclusionPersistent(km, count, false, persistentGrid(c->device), TB, s, pCoarse, s1, bt, b);
-    }
     mark(2, false);
     mark(3, true);
     k_cao_finish<<<(nCell + 255) / 256, 256, 0, s>>>(pCoarse, b, cgHit, cgQ, cgB);

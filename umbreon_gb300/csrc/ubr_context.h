@@ -29,7 +29,7 @@ struct Context {
   int builder = 1;           // binary tree before the 8-wide collapse: 1 Karras radix tree, 2 PLOC
   int collapse = 1;          // 8-wide collapse: 1 greedy (fixed leaf size), 2 SAH-optimal (leaves 1..3)
   float sahPrimScale = 1.0f; // SAH collapse: weight of primitive tests against node visits
-  int traceMode = 1;         // occlusion kernel: 1 one thread per ray (measured faster), 2 persistent
+  int traceMode = 0;         // occlusion kernel: 0 chosen per launch, else the context desc's trace_mode
   uint64_t arenaUsed = 0;
   std::string lastError;
   // frame scratch, reused across frames
