@@ -958,14 +958,10 @@ ubr_status adjoint(Context* c, const Scene* sc, const ubr_render_desc& d, const 
     if (gCen) UBR_CUDA(c, cudaMemcpyAsync(g.sphere_center, gCen, 3 * nSph * sizeof(float), back, s));
     if (gRad) UBR_CUDA(c, cudaMemcpyAsync(g.sphere_radius, gRad, nSph * sizeof(float), back, s));
   }
-  struct {
-    double g[kGlobals];
-    unsigned long long s[4];
-  } read;
-  UBR_CUDA(c, cudaMemcpyAsync(&read, gg, sizeof(read), back, s));
+  double* hg = reinterpret_cast<double*>(static_cast<char*>(c->pinned) + 2048);
+  const unsigned long long* hs = reinterpret_cast<const unsigned long long*>(hg + kGlobals);
+  UBR_CUDA(c, cudaMemcpyAsync(hg, gg, kGlobals * sizeof(double) + 4 * sizeof(unsigned long long), back, s));
   UBR_CUDA(c, cudaStreamSynchronize(s));
-  const double* hg = read.g;
-  const unsigned long long* hs = read.s;
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, c->ev[2], c->ev[3]);
   // fill the host struct; light vectors: L = normalize(-direction),

@@ -18,6 +18,14 @@ struct DevBuf {
   void* ptr = nullptr;
   size_t bytes = 0;
   bool direct = false;  // from cudaMalloc, not from the context's pool
+  int slab = 0;         // > 0: part of the context's slab of that number
+};
+
+// One cudaMalloc that several scratch blocks are cut from (scratchReserve).
+struct Slab {
+  void* ptr = nullptr;
+  size_t bytes = 0, used = 0;
+  int live = 0;  // blocks cut from it and not yet freed
 };
 
 struct Context {
@@ -34,6 +42,7 @@ struct Context {
   std::string lastError;
   // frame scratch, reused across frames
   std::vector<DevBuf> scratch;
+  std::vector<Slab> slabs;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   std::vector<cudaEvent_t> pev;  // profiling events, created on first use
   void* pinned = nullptr;    // small pinned host block for counters
@@ -79,6 +88,12 @@ void devFree(Context* c, DevBuf& b);
 // scratch slot `i` of at least `bytes` (a quarter more when it grows, unless
 // `slack` is false)
 ubr_status scratchGet(Context* c, int i, size_t bytes, void** out, bool slack = true);
+
+// Memory for the scratch blocks that the next scratchGet calls grow, `bytes` in
+// all: one allocation instead of one each.  Nothing under an arena cap, for
+// little, above kSlabBytes, or when it fails.
+void scratchReserve(Context* c, size_t bytes);
+constexpr size_t kSlabBytes = size_t(512) << 20;
 
 // A workspace of a pass that runs in chunks.  *bytes: what it uses well on
 // entry, what it got on exit (at least `least`).  Scratch slot `slot`, or,
