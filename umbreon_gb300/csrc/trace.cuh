@@ -8,7 +8,6 @@
 namespace ubr {
 namespace {
 
-constexpr int kStackDepth = 32;  // group entries: one per tree level
 constexpr float kInfF = __builtin_huge_valf();
 
 UBR_D f3 ld3(const float4 v) { return f3{v.x, v.y, v.z}; }

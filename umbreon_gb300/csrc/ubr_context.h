@@ -35,7 +35,7 @@ struct Context {
   uint64_t arenaCap = 0;     // 0 = unlimited
   int leafMax = 1;           // wide-BVH leaf size (1..kWideLeafMax); 1 measured fastest
   int builder = 1;           // binary tree before the 8-wide collapse: 1 Karras radix tree, 2 PLOC
-  int collapse = 1;          // 8-wide collapse: 1 greedy (fixed leaf size), 2 SAH-optimal (leaves 1..3)
+  int collapse = 0;          // 8-wide collapse: 0 library default, 1 greedy (fixed leaf size), 2 SAH-optimal (leaves 1..3)
   float sahPrimScale = 1.0f; // SAH collapse: weight of primitive tests against node visits
   int traceMode = 0;         // occlusion kernel: 0 chosen per launch, else the context desc's trace_mode
   uint64_t arenaUsed = 0;

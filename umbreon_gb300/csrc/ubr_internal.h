@@ -144,6 +144,7 @@ constexpr int kLeafF4 = 3;
 // (count << 5) | offset = count (1..3) primitives at primBase + offset.
 constexpr int kWideF4 = 5;
 constexpr int kWideLeafMax = 3;
+constexpr int kStackDepth = 32;   // traversal stack: group entries, one per level of the 8-wide tree
 
 struct DScene {
   const float4* wnodes = nullptr;  // 8-wide nodes (root = 0)
