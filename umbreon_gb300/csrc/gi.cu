@@ -560,25 +560,29 @@ __global__ void __launch_bounds__(128, 8) k_gather_first(GiP g, DScene s, GiGrid
   Hit h;
   f3 O{0.0f, 0.0f, 0.0f}, wi{0.0f, 0.0f, 0.0f};
   uint32_t s0 = 0, s1 = 0;
-  if (slot < waveSlots(w) && slotSample(w, slot, point, sI)) {
+  bool horizonOk = false;
+  float cos0 = 0.0f, eps = 0.0f;
+  const bool mine = slot < waveSlots(w) && slotSample(w, slot, point, sI);
+  if (mine) {
     const uint32_t pix = list[point];
-    bool horizonOk;
-    float cos0, eps;
-    {
-      const GatherOrigin o = gatherOrigin(g, grid, pix);
-      wi = gatherDirection(g, grid, o, pix, w.spp, sI);
-      horizonOk = dot(wi, o.Ng) > 0.0f;
-      cos0 = dot(wi, o.N);
-      O = o.O;
-      eps = o.eps;
-      s0 = o.seed;
-    }
+    const GatherOrigin o = gatherOrigin(g, grid, pix);
+    wi = gatherDirection(g, grid, o, pix, w.spp, sI);
+    horizonOk = dot(wi, o.Ng) > 0.0f;
+    cos0 = dot(wi, o.N);
+    O = o.O;
+    eps = o.eps;
+    s0 = o.seed;
     s1 = uint32_t(sI + g.sampleOffset);
+  }
+  // whole warps: the traversal below votes
+  if constexpr (postponesTests(KM)) traversePostponed<KM>(travOf(s), Ray{O, wi, eps, g.maxDist}, h, ovf, horizonOk);
+  if (mine) {
     float4 out = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
     f3 candPos{0.0f, 0.0f, 0.0f};
     bool escaped = false;
     if (horizonOk) {
-      traverse<false, KM, false, false, true>(travOf(s), Ray{O, wi, eps, g.maxDist}, h, ovf, nullptr, false);
+      if constexpr (!postponesTests(KM))
+        traverse<false, KM, false, false, true>(travOf(s), Ray{O, wi, eps, g.maxDist}, h, ovf, nullptr, false);
       rays = 1;
       push = h.ref != kInvalid;
       if (!push) {

@@ -339,6 +339,50 @@ UBR_D void travInit(const Ray& r, TravState& st, Hit& best, int start = 0) {
   best.ref = kInvalid;
 }
 
+// Goes on to the nearest hit child; the other hit children of the node are
+// pushed as one group.
+template <bool CULL>
+UBR_D void enterChild(const float (&tmin)[8], uint32_t link, uint32_t hitInt, int nearK, TravState& st,
+                      uint32_t& overflow) {
+  const uint32_t rest = hitInt & ~(1u << nearK);
+  if (rest) {
+    if (st.sp < kStackDepth) {
+      if (CULL) st.next[st.sp] = nearestKey(tmin, rest);
+      st.stack[st.sp++] = (link & ~0xFFu) | rest;
+    } else {
+      ++overflow;
+    }
+  }
+  st.node = int(link >> 8) + nearK;
+}
+
+// Goes on to the next pushed child; false when there is none.
+template <bool CULL>
+UBR_D bool nextNode(TravState& st) {
+  for (;;) {
+    if (st.sp == 0) return false;
+    const uint32_t g = st.stack[st.sp - 1];
+    uint32_t key = 0;
+    if (CULL) {
+      key = st.next[st.sp - 1];
+      if (__uint_as_float(key & ~7u) > st.tmax * kSlabGrow) {
+        --st.sp;
+        continue;
+      }
+    }
+    const int k = CULL ? int(key & 7u) : __ffs(g & 0xFFu) - 1;
+    const uint32_t left = g & ~(1u << k);
+    if (left & 0xFFu) {
+      st.stack[st.sp - 1] = left;
+      if (CULL) st.next[st.sp - 1] = (key & ~7u) | uint32_t(__ffs(left & 0xFFu) - 1);
+    } else {
+      --st.sp;
+    }
+    st.node = int(g >> 8) + k;
+    return true;
+  }
+}
+
 // A candidate hit of a primitive: the answer of an any-hit query (true), else
 // kept when it is nearer (ties to the lowest ids).
 UBR_D bool takeHit(const TravScene& s, const Hit& h, uint32_t ref, int kind, bool any, TravState& st, Hit& best) {
@@ -508,40 +552,10 @@ UBR_D bool travStep(const TravScene& s, const Ray& r, const f3& inv, const TriPr
     if (takeHit(s, h, ref, refKind(ref), any, st, best)) return true;
   }
   if (nearK >= 0) {
-    const uint32_t rest = hitInt & ~(1u << nearK);
-    if (rest) {
-      if (st.sp < kStackDepth) {
-        if (CULL) st.next[st.sp] = nearestKey(tminP, rest);
-        st.stack[st.sp++] = (link & ~0xFFu) | rest;
-      } else {
-        ++overflow;
-      }
-    }
-    st.node = int(link >> 8) + nearK;
+    enterChild<CULL>(tminP, link, hitInt, nearK, st, overflow);
     return false;
   }
-  for (;;) {
-    if (st.sp == 0) return true;
-    const uint32_t g = st.stack[st.sp - 1];
-    uint32_t key = 0;
-    if (CULL) {
-      key = st.next[st.sp - 1];
-      if (__uint_as_float(key & ~7u) > st.tmax * kSlabGrow) {
-        --st.sp;
-        continue;
-      }
-    }
-    const int k = CULL ? int(key & 7u) : __ffs(g & 0xFFu) - 1;
-    const uint32_t left = g & ~(1u << k);
-    if (left & 0xFFu) {
-      st.stack[st.sp - 1] = left;
-      if (CULL) st.next[st.sp - 1] = (key & ~7u) | uint32_t(__ffs(left & 0xFFu) - 1);
-    } else {
-      --st.sp;
-    }
-    st.node = int(g >> 8) + k;
-    return false;
-  }
+  return !nextNode<CULL>(st);
 }
 
 // Whole traversal of one ray (one thread per ray).
@@ -557,6 +571,77 @@ __device__ bool traverse(const TravScene& s, const Ray& r, Hit& best, uint32_t& 
   TravState st;
   travInit(r, st, best, start);
   while (!travStep<COUNT, KM, ALWAYS_ANY, FILTER, CULL>(s, r, inv, pre, st, best, overflow, cnt, any, top, nTop, flt)) {
+  }
+  return best.ref != kInvalid;
+}
+
+// Closest hits of a whole warp's rays (lanes without one pass active = false)
+// with the primitive tests put off: a lane goes on through nodes with up to two
+// groups of primitives pending, and the warp tests one primitive per lane once
+// kPendingLanes lanes have some, or at most kWalkLanes can still visit a node.
+// For scattered rays through spheres and cylinders: there a node step is made
+// by 15 lanes, but the tests after it by 3, and the exact cylinder test costs
+// as much as a node.  The visits that a later hit would have saved cost less.
+// 1920x1080 ss2 ball-and-stick pt2 frame 13.89 -> 13.24 ms (kPendingLanes 4 / 8 /
+// 12 / 16 in a first form: 13.76 / 13.60 / 13.52 / 13.47; 20 and 24 no better).  Not for
+// spheres alone, whose test is cheap (2 k sphere pt1 frame 0.472 -> 0.489), nor
+// for any-hit queries, which end at the first hit (batch of 24 +8 %, the
+// ball-and-stick frame's AO rays +-0.3 %).
+constexpr int kPendingLanes = 16, kWalkLanes = 6;
+__host__ __device__ constexpr bool postponesTests(int km) { return km == (kMaskSphere | kMaskCone); }
+
+template <int KM>
+__device__ bool traversePostponed(const TravScene& s, const Ray& r, Hit& best, uint32_t& overflow, bool active) {
+  static_assert((KM & kMaskMesh) == 0, "no triangle setup here");
+  bool walk = active && s.primCount > 0;
+  TravState st;
+  travInit(r, st, best);
+  f3 inv{0.0f, 0.0f, 0.0f};
+  if (walk) inv = safeInv(r.dir);
+  const TriPre pre{};
+  int base0 = 0, base1 = 0;  // pending groups: primitive base and slots
+  uint32_t mask0 = 0, mask1 = 0;
+  for (;;) {
+    if (walk && mask1 == 0) {
+      if (++st.steps > s.primCount + 16u) {  // each node at most once per ray in a valid tree
+        ++overflow;
+        walk = false;
+      } else {
+        const float4* nd = s.wnodes + kWideF4 * st.node;
+        const float4 n0 = __ldg(nd), n1 = __ldg(nd + 1), n2 = __ldg(nd + 2), n3 = __ldg(nd + 3), n4 = __ldg(nd + 4);
+        float tminP[8];
+        const uint32_t neg = nodeMisses(n0, n1, n2, n3, n4, r.org, inv, r.tnear, st.tmax, tminP);
+        const uint32_t link = __float_as_uint(n0.w);
+        const uint32_t hitInt = ~neg & link & 0xFFu;
+        const uint32_t prims = leafPrims(s, st.node, ~neg & __float_as_uint(n1.z) & 0xFFu);
+        const int nearK = nearestChild(tminP, hitInt);
+        if (prims && mask0) {
+          base1 = __float_as_int(n1.w);
+          mask1 = prims;
+        } else if (prims) {
+          base0 = __float_as_int(n1.w);
+          mask0 = prims;
+        }
+        if (nearK >= 0) enterChild<true>(tminP, link, hitInt, nearK, st, overflow);
+        else walk = nextNode<true>(st);
+      }
+    }
+    const unsigned pending = __ballot_sync(0xFFFFFFFFu, mask0 != 0);
+    const unsigned can = __ballot_sync(0xFFFFFFFFu, walk && mask1 == 0);
+    if (__popc(pending) < kPendingLanes && __popc(can) > kWalkLanes) continue;
+    if (!(pending | can)) break;
+    if (mask0) {
+      const int slot = base0 + __ffs(mask0) - 1;
+      mask0 &= mask0 - 1u;
+      if (mask0 == 0) {
+        base0 = base1;
+        mask0 = mask1;
+        mask1 = 0;
+      }
+      Hit h;
+      uint32_t ref;
+      if (testLeaf<KM>(s, slot, r, pre, r.tnear, st.tmax, h, ref)) takeHit(s, h, ref, refKind(ref), false, st, best);
+    }
   }
   return best.ref != kInvalid;
 }
