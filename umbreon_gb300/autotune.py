@@ -7,10 +7,12 @@ fastest:
 
 * BVH builder: Morton radix tree or PLOC clustering over the same order;
 * 8-wide collapse: greedy with a fixed leaf size (1..3 primitives), or the
-  SAH-optimal dynamic programme at a few weights of primitive tests against
-  node visits (its leaves hold 1..3 primitives as the costs decide);
-* occlusion kernel: one thread per ray, persistent warps refilling idle
-  lanes, or a resident grid with the top BVH levels in shared memory.
+  SAH-optimal dynamic programme with one-primitive leaves (the library's
+  default) or at a few weights of primitive tests against node visits (its
+  leaves hold 1..3 primitives as the costs decide);
+* occlusion kernel: the library's choice per launch (one thread per ray, or
+  persistent warps that fetch rays), persistent warps with the general
+  traversal, or a resident grid with the top BVH levels in shared memory.
 
 Results depend on the scene's primitive mix and ray lengths, so a caller
 tunes once per scene class and creates its context with the result
@@ -27,6 +29,7 @@ from .api import Context
 
 # (label, context fields) of the tree candidates
 TREES = (
+    [("sah_leaf1", dict(bvh_collapse=0))] +
     [(f"greedy_leaf{leaf}", dict(bvh_collapse=1, bvh_leaf_max=leaf)) for leaf in (1, 2, 3)] +
     [(f"sah_x{scale:g}", dict(bvh_collapse=2, sah_prim_scale=scale)) for scale in (1.0, 2.0, 4.0)]
 )
@@ -57,7 +60,7 @@ def _time(fields, scene, opt, device, repeats, key="total_ms", with_build=False)
 
 
 def autotune(scene, opt, device: int = 0, pixels: int = 256 * 256, repeats: int = 3,
-             builders=(1, 2), trees=TREES, trace_modes=(1, 2, 3), finalists: int = 3,
+             builders=(1, 2), trees=TREES, trace_modes=(0, 2, 3), finalists: int = 3,
              objective: str = "render"):
     """objective "render": the frame alone (a scene built once, rendered many
     times); "frame": scene build + frame (one render call per scene)."""

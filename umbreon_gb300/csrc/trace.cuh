@@ -69,17 +69,6 @@ UBR_D bool clipOn(const Params& p, f3 rd) {
   return !(dot(rd, p.camDir) <= 1.0e-6f);
 }
 
-UBR_D bool slabHit(float lox, float hix, float loy, float hiy, float loz, float hiz, const f3& o,
-                   const f3& inv, float tnear, float tmax, float& tEntry) {
-  const float t0x = (lox - o.x) * inv.x, t1x = (hix - o.x) * inv.x;
-  const float t0y = (loy - o.y) * inv.y, t1y = (hiy - o.y) * inv.y;
-  const float t0z = (loz - o.z) * inv.z, t1z = (hiz - o.z) * inv.z;
-  const float tmin = fmaxf(fmaxf(fminf(t0x, t1x), fminf(t0y, t1y)), fmaxf(fminf(t0z, t1z), tnear));
-  const float tmx = fminf(fminf(fmaxf(t0x, t1x), fmaxf(t0y, t1y)), fminf(fmaxf(t0z, t1z), tmax));
-  tEntry = tmin;
-  return tmin <= tmx;
-}
-
 // Kind masks: bit k set when primitives of kind k exist.  Kernels are
 // instantiated per mask so a scene only carries the intersectors it needs.
 constexpr int kMaskMesh = 1 << kMesh, kMaskSphere = 1 << kSphere, kMaskRound = 1 << kRound,
@@ -135,9 +124,6 @@ UBR_D bool testLeaf(const TravScene& s, int slot, const Ray& r, const TriPre& pr
   return false;
 }
 
-// Stack traversal of the binary LBVH, near child first.  ANY: return at the
-// first hit in [tnear, tfar].  Closest: smallest t, ties to lowest
-// (geomID, primID).
 // Bytes of the leaf record fetched for one primitive test, by kind
 // (leafRef 4 B + geometry float4s; round segments add their 32 B clip planes).
 UBR_D uint32_t leafBytes(int kind) {
@@ -197,7 +183,7 @@ UBR_D float boundValue(uint32_t q, int b) {
 }
 
 // Packed pairs of floats for the slab test of two children at once:
-// sm_100-family add/mul/fma on .f32x2 round each lane like the scalar
+// sm_100-family fma on .f32x2 rounds each lane like the scalar
 // instruction (round to nearest even), so the pair form gives the same bits
 // as two scalar operations with half the instructions issued.
 typedef unsigned long long f2x;
@@ -210,16 +196,6 @@ UBR_D void up2(f2x v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a
 UBR_D f2x fma2(f2x a, f2x b, f2x c) {
   f2x d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-UBR_D f2x add2(f2x a, f2x b) {
-  f2x d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-UBR_D f2x mul2(f2x a, f2x b) {
-  f2x d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
 // Bounds b and b+1 of q as a float pair.
@@ -586,7 +562,8 @@ __device__ bool traverse(const TravScene& s, const Ray& r, Hit& best, uint32_t& 
 // 12 / 16 in a first form: 13.76 / 13.60 / 13.52 / 13.47; 20 and 24 no better).  Not for
 // spheres alone, whose test is cheap (2 k sphere pt1 frame 0.472 -> 0.489), nor
 // for any-hit queries, which end at the first hit (batch of 24 +8 %, the
-// ball-and-stick frame's AO rays +-0.3 %).
+// ball-and-stick frame's AO rays +-0.3 %, a surface's +9 to +12 %), nor for a
+// surface's AO distances (+12 %).
 constexpr int kPendingLanes = 16, kWalkLanes = 6;
 __host__ __device__ constexpr bool postponesTests(int km) { return km == (kMaskSphere | kMaskCone); }
 
