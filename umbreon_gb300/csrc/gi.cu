@@ -621,12 +621,17 @@ __global__ void __launch_bounds__(128, 8) k_gather_next(GiP g, DScene s, GiWave 
   uint32_t rays = 0, ovf = 0;
   bool push = false;
   Hit h;
-  float4 a, b, c;
+  float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a, c;
   uint32_t s1 = 0;
-  if (i < w.ctr[3]) {
+  const bool mine = i < w.ctr[3];
+  if (mine) {
     a = w.path[0][i];
     b = w.path[1][i];
-    traverse<false, KM, false, false, true>(travOf(s), Ray{ld3(a), ld3(b), a.w, g.maxDist}, h, ovf, nullptr, false);
+  }
+  if constexpr (postponesTests(KM)) traversePostponed<KM>(travOf(s), Ray{ld3(a), ld3(b), a.w, g.maxDist}, h, ovf, mine);
+  if (mine) {
+    if constexpr (!postponesTests(KM))
+      traverse<false, KM, false, false, true>(travOf(s), Ray{ld3(a), ld3(b), a.w, g.maxDist}, h, ovf, nullptr, false);
     rays = 1;
     c = w.path[2][i];
     s1 = __float_as_uint(w.path[3][i].x);
