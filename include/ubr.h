@@ -396,7 +396,8 @@ typedef struct ubr_context_desc {
   /* BVH tuning (0 = library default): the most primitives a wide-BVH leaf
    * holds (1..3); smaller leaves mean more nodes and fewer primitive tests */
   uint32_t bvh_leaf_max;
-  /* occlusion-ray kernel (0 = library default): 1 = one thread per ray,
+  /* occlusion-ray kernel (0 = library default: chosen per launch by its kinds
+   * of primitives and number of rays): 1 = one thread per ray,
    * 2 = persistent warps that refill idle lanes with new rays, 3 = resident
    * grid striding over the rays with the top BVH levels in shared memory,
    * 4 = one thread per ray with node visits and primitive tests interleaved
@@ -409,7 +410,8 @@ typedef struct ubr_context_desc {
    * codes, 2 = locally-ordered clustering (PLOC) over the same Morton order;
    * leaf sizes above 1 always use the radix tree */
   uint32_t bvh_builder;
-  /* binary -> 8-wide collapse (0 = library default): 1 = greedy (open the
+  /* binary -> 8-wide collapse (0 = library default: SAH-optimal with leaves of
+   * one primitive, greedy where bvh_leaf_max asks for more): 1 = greedy (open the
    * largest child, leaves of bvh_leaf_max primitives), 2 = SAH-optimal
    * dynamic programme choosing every node's children and leaves of 1..3
    * primitives */
