@@ -21,6 +21,8 @@ def spheres(kind, n):
     else:
         cr[:, :3] = r.random((n, 3))
         cr[:, 3] = 0.3 / n ** 0.4
+        if kind == "outlier":  # areas above it overflow
+            cr[n // 2] = (1e25, -1e25, 3e24, 1.0)
     color = np.ones((n, 4)) if kind == "same" else 0.5 + 0.5 * r.random((n, 4))
     return Scene(sphere_center_radius=cr.astype(np.float32), sphere_color=color.astype(np.float32),
                  sphere_material=np.full(n, abi.material(), abi.MATERIAL_DTYPE), lights=[DistantLight()],
@@ -28,7 +30,8 @@ def spheres(kind, n):
 
 
 @pytest.mark.parametrize("kind,n", [("cloud", n) for n in (1, 2, 3, 8, 9, 16, 17, 57, 129, 1025, 20000)]
-                         + [("chain", 40), ("same", 300)])
+                         + [("chain", 40), ("same", 300)]
+                         + [("outlier", n) for n in (12, 100, 3000)])
 def test_trees_show_the_same_picture(kind, n):
     sc = spheres(kind, n)
     opt = RenderOptions(width=128, height=96, aoSamples=4, aoDistance=0.5)

@@ -825,7 +825,8 @@ __device__ __forceinline__ void sahRow(float* out, uint8_t* d, const float (&r0)
   const float cInt = A * kSahNode + dist[8];
   float cj = fminf(cLeaf, cInt);
   out[0] = cj;
-  d[0] = cLeaf <= cInt ? 1 : 0;  // j = 1: 1 leaf, 0 wide node
+  // j = 1: 1 leaf, 0 wide node (the count decides where areas overflow)
+  d[0] = cnt <= leafCap && cLeaf <= cInt ? 1 : 0;
   for (int j = 2; j <= 7; ++j) {
     if (dist[j] < cj) {
       cj = dist[j];
@@ -1249,6 +1250,7 @@ __global__ void __launch_bounds__(128) k_collapse(CollapseIO io, int level, int 
     for (bool more = true; __any_sync(kAll, more);) {
       // the largest child worth opening, ties to the lowest lane
       float a = t < en && c >= 0 && cnt > leafMax ? halfArea(lo, hi) : -1.0f;
+      if (!(a > -1.0f)) a = -1.0f;  // not a number: never opened, and the lanes agree
       int at = t;
       for (int o = 4; o > 0; o >>= 1) {
         const float oa = __shfl_xor_sync(kAll, a, o);
@@ -1258,7 +1260,7 @@ __global__ void __launch_bounds__(128) k_collapse(CollapseIO io, int level, int 
           at = ot;
         }
       }
-      more = a >= 0.0f && en < 8;
+      more = a > -1.0f && en < 8;
       const int pc = __shfl_sync(kAll, c, g0 + at);
       if (more) {
         if (t == at || t == en) {
