@@ -3115,21 +3115,30 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
   };
   const bool useGraph = singleLayer && !prof && !count && c->useGraphs && !adaptive && !giOn;
   if (useGraph) {
-    // key: everything the captured launches depend on
-    std::vector<unsigned char> key(sizeof(Params) + sizeof(DScene) + sizeof(Batch) + sizeof(Bufs) + 64);
-    size_t o = 0;
+    // key: everything the captured launches depend on -- the parameter blocks
+    // they are given, the choices made here, and the buffers and scalars that
+    // reach a launch outside the blocks (the denoiser's, the next layer's queue,
+    // the frame table)
+    std::vector<unsigned char> key;
     auto put = [&](const void* src, size_t n) {
-      std::memcpy(key.data() + o, src, n);
-      o += n;
+      const unsigned char* q = static_cast<const unsigned char*>(src);
+      key.insert(key.end(), q, q + n);
     };
+    key.reserve(sizeof(Params) + sizeof(DScene) + sizeof(Batch) + sizeof(Bufs) + 256);
     put(&p1, sizeof(Params));
     put(&s1, sizeof(DScene));
     put(&bt, sizeof(Batch));
     put(&b, sizeof(Bufs));
-    const uint64_t misc[7] = {npix, nout, uint64_t(km), uint64_t(c->traceMode), uint64_t(outColor), R,
-                              uint64_t(plain) | uint64_t(nearest) << 1};
+    const uint64_t misc[] = {npix, nout, uint64_t(km), uint64_t(c->traceMode), R,
+                             uint64_t(plain) | uint64_t(nearest) << 1, uint64_t(q0), uint64_t(frameTable)};
     put(misc, sizeof(misc));
-    key.resize(o);
+    if (denoise) {
+      const float sigmas[2] = {d0.denoise_sigma_n, d0.denoise_sigma_l};
+      const uint64_t dn[] = {uint64_t(d0.denoise_iters), uint64_t(d0.denoise_demodulate_albedo != 0), uint64_t(dnValid),
+                             uint64_t(dnIrr[0]), uint64_t(dnIrr[1]), uint64_t(dnLum), uint64_t(dnVar)};
+      put(sigmas, sizeof(sigmas));
+      put(dn, sizeof(dn));
+    }
     if (!c->graphExec || key != c->graphKey) {
       UBR_CUDA(c, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
       cudaMemsetAsync(b.stats, 0, 8 * sizeof(unsigned long long), s);
