@@ -304,6 +304,10 @@ typedef enum ubr_memory {
  *   view_z  : Wss*Hss  hi-res plane eye-z of the first hit
  *   hit_geom, hit_prim : Wss*Hss first-hit (geomID, primID); UBR_INVALID_ID
  *             on a miss (parity evidence, not a FrameResult field)
+ * Device planes are written while the frame is rendered and read back by its
+ * later passes; planes that share memory are rendered elsewhere and copied at
+ * the end, in the order of the frames and of the members.  A call that fails
+ * may leave them half written.
  * Statistics are written back into the struct. */
 #define UBR_FRAME_PROFILE 1u  /* time each kernel phase with CUDA events */
 #define UBR_FRAME_COUNT 2u    /* count BVH node / primitive bytes fetched */

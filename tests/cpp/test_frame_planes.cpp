@@ -1,0 +1,43 @@
+// The choice of the planes a call writes in place (csrc/frame_planes.h) against
+// a check of every pair.
+#include <cstdio>
+#include <random>
+
+#include "frame_planes.h"
+
+using ubr::PlaneUse;
+
+static int failures = 0;
+static void check(bool ok, const char* what) {
+  if (!ok && ++failures < 20) std::printf("FAILED: %s\n", what);
+}
+static const void* at(uintptr_t a) { return reinterpret_cast<const void*>(a); }
+
+int main() {
+  std::mt19937 rng(7);
+  for (int round = 0; round < 20000; ++round) {
+    const int n = int(rng() % 14);
+    const uintptr_t span = 16u << (rng() % 12);  // dense to sparse
+    std::vector<PlaneUse> in;
+    for (int k = 0; k < n; ++k) {
+      const bool none = rng() % 6 == 0;
+      in.push_back(PlaneUse{none ? nullptr : at(4096 + 4 * (rng() % span)), 4 * size_t(rng() % 40), rng() % 5 != 0});
+    }
+    std::vector<PlaneUse> out = in;
+    choosePlanes(out);
+    for (int i = 0; i < n; ++i) {
+      const uintptr_t a = reinterpret_cast<uintptr_t>(in[i].ptr);
+      bool want = in[i].inPlace && in[i].ptr && in[i].bytes;
+      for (int j = 0; j < n; ++j) {
+        const uintptr_t c = reinterpret_cast<uintptr_t>(in[j].ptr);
+        if (i != j && in[i].ptr && in[j].ptr && in[i].bytes && in[j].bytes && a < c + in[j].bytes &&
+            c < a + in[i].bytes)
+          want = false;
+      }
+      check(out[i].inPlace == want, "planes that meet no other plane, and only they, stay in place");
+      check(out[i].ptr == in[i].ptr && out[i].bytes == in[i].bytes, "order and extents are kept");
+    }
+  }
+  if (failures) std::printf("%d failures\n", failures);
+  return failures ? 1 : 0;
+}

@@ -1,0 +1,42 @@
+// frame_planes.h -- which of the caller's device planes a call writes as it
+// renders (host code only).
+//
+// A plane written in place is also read back: later transparency layers ask
+// the depth plane whether a pixel had its first hit, the fog reads view z, the
+// denoiser reads the colour and the AOVs.  That is only right for memory that
+// belongs to one plane of one frame.  The other planes are shaded into the
+// context's buffers and copied at the end of the call, in the order of the
+// frames, so planes that share memory end up as the last copy leaves them.
+#pragma once
+
+#include <algorithm>
+#include <cstddef>
+#include <cstdint>
+#include <vector>
+
+namespace ubr {
+
+struct PlaneUse {
+  const void* ptr;  // null: not asked for
+  size_t bytes;
+  bool inPlace;     // in: the call could write it as it renders; out: it may
+};
+
+// Takes inPlace from planes whose memory meets another plane's.
+inline void choosePlanes(std::vector<PlaneUse>& planes) {
+  std::vector<PlaneUse*> by;
+  by.reserve(planes.size());
+  for (PlaneUse& u : planes) {
+    if (u.ptr && u.bytes) by.push_back(&u);
+    else u.inPlace = false;
+  }
+  auto at = [](const PlaneUse* u) { return reinterpret_cast<uintptr_t>(u->ptr); };
+  std::sort(by.begin(), by.end(), [&](const PlaneUse* a, const PlaneUse* b) { return at(a) < at(b); });
+  uintptr_t end = 0;  // of the planes so far
+  for (size_t k = 0; k < by.size(); ++k) {
+    if (at(by[k]) < end) by[k]->inPlace = by[k - 1]->inPlace = false;
+    end = std::max(end, at(by[k]) + by[k]->bytes);
+  }
+}
+
+}  // namespace ubr

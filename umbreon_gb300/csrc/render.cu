@@ -24,6 +24,7 @@
 #include <cstring>
 #include <vector>
 
+#include "frame_planes.h"
 #include "gi.cuh"
 #include "trace.cuh"
 
@@ -2712,8 +2713,29 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
   const bool direct = !adaptive && !edgeGb;
   std::vector<unsigned char> table(outBytes + lights.size() * sizeof(LightD));
   std::vector<FrameOut> outs(nf);
+  // per frame: colour, depth, view z, ids, six AOVs, and the patch mask, which
+  // is always copied
+  constexpr size_t kPlanes = 12;
+  std::vector<PlaneUse> planes(nf * kPlanes, PlaneUse{nullptr, 0, false});
   for (size_t f = 0; f < nf; ++f) {
     const ubr_frame& fr = *jobs[f].frame;
+    if (!direct || fr.memory != UBR_MEMORY_DEVICE) continue;
+    const Params& p = fds[f].p;
+    const size_t fpix = size_t(p.W) * p.H, fout = size_t(p.outW) * p.outH;
+    PlaneUse* u = &planes[f * kPlanes];
+    u[0] = PlaneUse{fr.color, fout * 16, reinterpret_cast<uintptr_t>(fr.color) % 16 == 0};
+    const void* const perPixel[4] = {fr.depth, fr.view_z, fr.hit_geom, fr.hit_prim};
+    for (int k = 0; k < 4; ++k) u[1 + k] = PlaneUse{perPixel[k], fpix * 4, true};
+    if (outAov && p.aoWriteAov) {
+      const void* const aovs[6] = {fr.albedo, fr.normal, fr.bent_normal, fr.contact_ao, fr.shape_ao, fr.avg_hit_dist};
+      for (int k = 0; k < 6; ++k) u[5 + k] = PlaneUse{aovs[k], size_t(kAovWidth[k]) * fout * 4, true};
+    }
+    if (b.aoPatch) u[11] = PlaneUse{fr.ao_patch_mask, fpix * 4, false};
+  }
+  choosePlanes(planes);
+  for (size_t f = 0; f < nf; ++f) {
+    const ubr_frame& fr = *jobs[f].frame;
+    const PlaneUse* u = &planes[f * kPlanes];
     const size_t po = fds[f].pixOff, oo = fds[f].outOff;
     FrameOut& o = outs[f];
     o = FrameOut{outColor + oo, b.depth + po, b.viewZ + po, b.hitGeom + po, b.hitPrim + po, {}};
@@ -2722,17 +2744,14 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
       o.aov[k] = outAov + at + size_t(kAovWidth[k]) * oo;
       at += size_t(kAovWidth[k]) * nout;
     }
-    if (!direct || fr.memory != UBR_MEMORY_DEVICE) continue;
-    if (fr.color && reinterpret_cast<uintptr_t>(fr.color) % 16 == 0) o.color = reinterpret_cast<float4*>(fr.color);
-    if (fr.depth) o.depth = fr.depth;
-    if (fr.view_z) o.viewZ = fr.view_z;
-    if (fr.hit_geom) o.hitGeom = fr.hit_geom;
-    if (fr.hit_prim) o.hitPrim = fr.hit_prim;
-    if (outAov && fds[f].p.aoWriteAov) {
-      float* const dst[6] = {fr.albedo, fr.normal, fr.bent_normal, fr.contact_ao, fr.shape_ao, fr.avg_hit_dist};
-      for (int k = 0; k < 6; ++k)
-        if (dst[k]) o.aov[k] = dst[k];
-    }
+    if (u[0].inPlace) o.color = reinterpret_cast<float4*>(fr.color);
+    if (u[1].inPlace) o.depth = fr.depth;
+    if (u[2].inPlace) o.viewZ = fr.view_z;
+    if (u[3].inPlace) o.hitGeom = fr.hit_geom;
+    if (u[4].inPlace) o.hitPrim = fr.hit_prim;
+    float* const aovs[6] = {fr.albedo, fr.normal, fr.bent_normal, fr.contact_ao, fr.shape_ao, fr.avg_hit_dist};
+    for (int k = 0; k < 6; ++k)
+      if (u[5 + k].inPlace) o.aov[k] = aovs[k];
   }
   std::memcpy(table.data(), outs.data(), nf * sizeof(FrameOut));
   if (!lights.empty()) std::memcpy(table.data() + outBytes, lights.data(), lights.size() * sizeof(LightD));
