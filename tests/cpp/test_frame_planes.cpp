@@ -21,20 +21,23 @@ int main() {
     std::vector<PlaneUse> in;
     for (int k = 0; k < n; ++k) {
       const bool none = rng() % 6 == 0;
-      in.push_back(PlaneUse{none ? nullptr : at(4096 + 4 * (rng() % span)), 4 * size_t(rng() % 40), rng() % 5 != 0});
+      const size_t align = rng() % 5 == 0 ? 0 : rng() % 4 == 0 ? 16 : 4;
+      const uintptr_t odd = rng() % 8 == 0 ? 1 + rng() % 15 : 0;
+      in.push_back(PlaneUse{none ? nullptr : at(4096 + 4 * (rng() % span) + odd), 4 * size_t(rng() % 40), align,
+                            rng() % 2 == 0});
     }
     std::vector<PlaneUse> out = in;
     choosePlanes(out);
     for (int i = 0; i < n; ++i) {
       const uintptr_t a = reinterpret_cast<uintptr_t>(in[i].ptr);
-      bool want = in[i].inPlace && in[i].ptr && in[i].bytes;
+      bool want = in[i].align && in[i].ptr && in[i].bytes && a % in[i].align == 0;
       for (int j = 0; j < n; ++j) {
         const uintptr_t c = reinterpret_cast<uintptr_t>(in[j].ptr);
         if (i != j && in[i].ptr && in[j].ptr && in[i].bytes && in[j].bytes && a < c + in[j].bytes &&
             c < a + in[i].bytes)
           want = false;
       }
-      check(out[i].inPlace == want, "planes that meet no other plane, and only they, stay in place");
+      check(out[i].inPlace == want, "aligned planes that meet no other plane, and only they, are written in place");
       check(out[i].ptr == in[i].ptr && out[i].bytes == in[i].bytes, "order and extents are kept");
     }
   }

@@ -19,18 +19,22 @@ namespace ubr {
 struct PlaneUse {
   const void* ptr;  // null: not asked for
   size_t bytes;
-  bool inPlace;     // in: the call could write it as it renders; out: it may
+  size_t align;     // of the kernels' stores; 0: the call only copies this plane
+  bool inPlace;     // out: the call may write it as it renders
 };
 
-// Takes inPlace from planes whose memory meets another plane's.
+// A plane is written in place unless its memory meets another plane's, or it
+// starts between two of the kernels' elements (a copy takes any address, a
+// kernel's store there is a fault).
 inline void choosePlanes(std::vector<PlaneUse>& planes) {
   std::vector<PlaneUse*> by;
   by.reserve(planes.size());
-  for (PlaneUse& u : planes) {
-    if (u.ptr && u.bytes) by.push_back(&u);
-    else u.inPlace = false;
-  }
   auto at = [](const PlaneUse* u) { return reinterpret_cast<uintptr_t>(u->ptr); };
+  for (PlaneUse& u : planes) {
+    const bool some = u.ptr && u.bytes;
+    u.inPlace = some && u.align && at(&u) % u.align == 0;
+    if (some) by.push_back(&u);
+  }
   std::sort(by.begin(), by.end(), [&](const PlaneUse* a, const PlaneUse* b) { return at(a) < at(b); });
   uintptr_t end = 0;  // of the planes so far
   for (size_t k = 0; k < by.size(); ++k) {

@@ -2716,21 +2716,21 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
   // per frame: colour, depth, view z, ids, six AOVs, and the patch mask, which
   // is always copied
   constexpr size_t kPlanes = 12;
-  std::vector<PlaneUse> planes(nf * kPlanes, PlaneUse{nullptr, 0, false});
+  std::vector<PlaneUse> planes(nf * kPlanes, PlaneUse{});
   for (size_t f = 0; f < nf; ++f) {
     const ubr_frame& fr = *jobs[f].frame;
     if (!direct || fr.memory != UBR_MEMORY_DEVICE) continue;
     const Params& p = fds[f].p;
     const size_t fpix = size_t(p.W) * p.H, fout = size_t(p.outW) * p.outH;
     PlaneUse* u = &planes[f * kPlanes];
-    u[0] = PlaneUse{fr.color, fout * 16, reinterpret_cast<uintptr_t>(fr.color) % 16 == 0};
+    u[0] = PlaneUse{fr.color, fout * 16, alignof(float4), false};
     const void* const perPixel[4] = {fr.depth, fr.view_z, fr.hit_geom, fr.hit_prim};
-    for (int k = 0; k < 4; ++k) u[1 + k] = PlaneUse{perPixel[k], fpix * 4, true};
+    for (int k = 0; k < 4; ++k) u[1 + k] = PlaneUse{perPixel[k], fpix * 4, 4, false};
     if (outAov && p.aoWriteAov) {
       const void* const aovs[6] = {fr.albedo, fr.normal, fr.bent_normal, fr.contact_ao, fr.shape_ao, fr.avg_hit_dist};
-      for (int k = 0; k < 6; ++k) u[5 + k] = PlaneUse{aovs[k], size_t(kAovWidth[k]) * fout * 4, true};
+      for (int k = 0; k < 6; ++k) u[5 + k] = PlaneUse{aovs[k], size_t(kAovWidth[k]) * fout * 4, 4, false};
     }
-    if (b.aoPatch) u[11] = PlaneUse{fr.ao_patch_mask, fpix * 4, false};
+    if (b.aoPatch) u[11] = PlaneUse{fr.ao_patch_mask, fpix * 4, 0, false};
   }
   choosePlanes(planes);
   for (size_t f = 0; f < nf; ++f) {
