@@ -8,6 +8,8 @@
 #include <string>
 #include <vector>
 
+#include <cuda.h>
+
 #include "ubr_context.h"
 
 namespace ubr {
@@ -161,6 +163,34 @@ ubr_status workspaceGet(Context* c, int slot, size_t least, void** out, size_t* 
   }
   *bytes = least;
   return scratchGet(c, slot, least, out);
+}
+
+bool deviceHolds(int device, const void* ptr, size_t bytes) {
+  // from the driver: the runtime's pointer attributes have no extent
+  using Get = CUresult(CUDAAPI*)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+  static const Get get = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &fn, 12000, cudaEnableDefault, &found) !=
+            cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<Get>(fn);
+  }();
+  if (!get) return false;
+  CUpointer_attribute what[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                 CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  unsigned int type = 0;
+  int ordinal = -1;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  void* values[4] = {&type, &ordinal, &start, &size};
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(ptr);
+  if (get(4, what, values, at) != CUDA_SUCCESS) return false;
+  return type == CU_MEMORYTYPE_DEVICE && ordinal == device && at >= start && at - start <= size &&
+         bytes <= size - (at - start);
 }
 
 }  // namespace ubr

@@ -25,14 +25,17 @@ struct PlaneUse {
 
 // A plane is written in place unless its memory meets another plane's, or it
 // starts between two of the kernels' elements (a copy takes any address, a
-// kernel's store there is a fault).
-inline void choosePlanes(std::vector<PlaneUse>& planes) {
+// kernel's store there is a fault), or ours(ptr, bytes) does not know it as
+// memory of the device in its whole length (a copy to other memory works, or
+// fails with an error; a kernel's store would be a fault).
+template <class Ours>
+void choosePlanes(std::vector<PlaneUse>& planes, Ours&& ours) {
   std::vector<PlaneUse*> by;
   by.reserve(planes.size());
   auto at = [](const PlaneUse* u) { return reinterpret_cast<uintptr_t>(u->ptr); };
   for (PlaneUse& u : planes) {
     const bool some = u.ptr && u.bytes;
-    u.inPlace = some && u.align && at(&u) % u.align == 0;
+    u.inPlace = some && u.align && at(&u) % u.align == 0 && ours(u.ptr, u.bytes);
     if (some) by.push_back(&u);
   }
   std::sort(by.begin(), by.end(), [&](const PlaneUse* a, const PlaneUse* b) { return at(a) < at(b); });

@@ -112,6 +112,11 @@ T* scratchT(Context* c, int slot, size_t count, ubr_status& st) {
   return static_cast<T*>(ptr);
 }
 
+// Whether [ptr, ptr + bytes) lies within one allocation on `device`.  Kernels
+// write a caller's memory only where this holds: a copy or memset checks what
+// it is given and fails with an error, a kernel's store faults.
+bool deviceHolds(int device, const void* ptr, size_t bytes);
+
 // Frame parameters and light table of a render description (camera basis,
 // lights, AO / fog / gamma settings), validated.
 ubr_status makeParams(Context* c, const ubr_render_desc& d, Params& p, std::vector<LightD>& lights);
