@@ -860,7 +860,13 @@ ubr_status adjoint(Context* c, const Scene* sc, const ubr_render_desc& d, const 
   // no packed sums, and whatever workspace the context can lend
   const size_t pixBytes = 4 + 48 + size_t(p.aoSamples) * 8 + size_t(p.nLights);
   const size_t hitBytes = (size_t(npix) * sizeof(float2) + kAdjAlign) / kAdjAlign * kAdjAlign;
-  const size_t accBytes = (gCol || gCen || gRad) ? size_t(nSph) * 32 : 0;
+  // the caller's arrays get the packed sums spread over them at the end where
+  // the device holds them whole; any others are cleared here and added to (the
+  // clearing finds arrays it cannot write, with an error)
+  const bool spread = !dev || ((!gCol || deviceHolds(c->device, gCol, 3 * nSph * sizeof(float))) &&
+                               (!gCen || deviceHolds(c->device, gCen, 3 * nSph * sizeof(float))) &&
+                               (!gRad || deviceHolds(c->device, gRad, nSph * sizeof(float))));
+  const size_t accBytes = spread && (gCol || gCen || gRad) ? size_t(nSph) * 32 : 0;
   const size_t accPad = (accBytes + kAdjAlign - 1) / kAdjAlign * kAdjAlign;
   size_t wsBytes = kAdjHeader + std::min<size_t>(size_t(npix) * pixBytes, std::max(kAdjBytes, pixBytes));
   void* ws = nullptr;
