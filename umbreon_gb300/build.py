@@ -29,7 +29,7 @@ INCLUDE = ROOT / "include"
 ORACLE = ROOT / "oracle"
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-CU_SOURCES = ["api.cu", "scene_build.cu", "render.cu", "gi.cu", "adjoint.cu"]
+CU_SOURCES = ["api.cu", "context.cu", "scene_build.cu", "render.cu", "gi.cu", "adjoint.cu"]
 HOST_SOURCES = ["umbreon.cpp", "pov/sdl.cpp", "pov/pov_scene_reader.cpp", "pov/mesh2_reader.cpp"]
 
 
