@@ -388,7 +388,13 @@ typedef struct ubr_frame {
 /* Context: one GPU, one CUDA stream, one device arena.  Scenes and frame
  * scratch are allocated stream-ordered from the context's own memory pool;
  * memory released by ubr_scene_release or scratch growth stays in that pool
- * for reuse until ubr_context_destroy. */
+ * for reuse until ubr_context_destroy.  Scratch blocks of 96 MB and more, and
+ * (without an arena cap) one block of 48 to 512 MB that the planes of a first
+ * frame of its size are cut from, come from cudaMalloc instead: they go back to
+ * the device when a larger frame replaces them, by cudaFree, which waits for
+ * the work of every stream of the device.  Scratch is kept until then,
+ * workspaces of the GI gather (at most 1 GiB) and of the adjoint (its hits, 32
+ * bytes a sphere and at most 256 MB) among it. */
 typedef struct ubr_context ubr_context;
 typedef struct ubr_scene ubr_scene;
 

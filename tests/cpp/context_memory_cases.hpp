@@ -1,0 +1,83 @@
+// Frames of growing sizes, as a render asks for its scratch: fixed small blocks
+// (counters, a table), blocks that grow with the pixels, and blocks that only
+// some frames ask for.
+using Plan = std::vector<ScratchNeed>;
+
+static Plan frame(size_t npix, bool aov) {
+  Plan p;
+  for (int slot : {16, 18, 23, 24, 27, 28}) p.push_back({slot, 16 * npix});
+  for (int slot : {17, 19, 20, 21, 22, 25, 26}) p.push_back({slot, 4 * npix});
+  if (aov)
+    for (int slot : {70, 71, 72}) p.push_back({slot, 16 * npix});
+  return p;
+}
+
+static void render(Context& c, const Plan& plan) {
+  ++c.call;
+  scratchReserve(&c, plan);
+  void* p;
+  for (int slot : {33, 34, 37, 32}) check(scratchGet(&c, slot, 64 + 16, &p) == UBR_OK, "a counter");
+  for (const ScratchNeed& n : plan) check(scratchGet(&c, n.slot, n.bytes, &p, n.slack) == UBR_OK, "a plane");
+  consistent(c);
+}
+
+static void slabs() {
+  const size_t mib = size_t(1) << 20;
+  // a first frame in one allocation, then larger ones: the first one's memory
+  // goes back, whatever small blocks were taken with it
+  Context& c = fresh(0);
+  render(c, frame(700000, true));
+  check(c.slab.ptr != nullptr, "the first frame's scratch is one allocation");
+  const size_t first = fake::held;
+  check(first < blocks(c) + 8 * mib, "little beyond the blocks is held");
+  render(c, frame(700000, true));
+  check(fake::held == first, "the same frame again takes nothing");
+  render(c, frame(1400000, true));
+  check(fake::held < blocks(c) + 8 * mib, "the first allocation went back");
+  render(c, frame(2400000, false));
+  check(fake::held < blocks(c) + 8 * mib, "it goes back with blocks the new frame does not ask for");
+  render(c, frame(20000000, false));  // more than one allocation of this kind holds
+  check(fake::held < blocks(c) + 8 * mib, "and where the new frame takes its blocks one by one");
+  render(c, frame(700000, true));
+  check(fake::held < blocks(c) + 8 * mib, "a small frame after it");
+  // blocks that are large enough already are not allocated for again
+  Context& d = fresh(0);
+  render(d, frame(600000, false));
+  void* p;
+  ++d.call;
+  for (int slot : {70, 71, 72}) check(scratchGet(&d, slot, 64 * mib, &p) == UBR_OK, "a block on its own");
+  const size_t before = fake::held;
+  render(d, frame(1000000, true));
+  check(fake::held < before + size_t(1.3 * 124 * 1000000) + 8 * mib - size_t(1.2 * 124 * 600000), "only what grows");
+  // a block that outgrows the allocation leaves room that others take
+  Context& g = fresh(0);
+  render(g, frame(800000, true));
+  check(scratchGet(&g, 16, 40 * mib, &p) == UBR_OK, "a block that grows on its own");
+  consistent(g);
+  const size_t grown = fake::held;
+  check(scratchGet(&g, 30, 12 * mib, &p) == UBR_OK, "a new block");
+  consistent(g);
+  check(fake::held == grown, "in the room that was left");
+  // an allocation that nothing was cut from
+  Context& h = fresh(0);
+  ++h.call;
+  scratchReserve(&h, frame(800000, false));
+  render(h, frame(900000, false));
+  check(fake::held < blocks(h) + 8 * mib, "goes back at the next one");
+  // no allocation for all: the blocks one by one
+  Context& i = fresh(0);
+  fake::limit = 100 * mib;
+  render(i, frame(500000, false));
+  // random sizes
+  Context& e = fresh(0);
+  unsigned x = 1;
+  for (int k = 0; k < 300; ++k) {
+    x = x * 1664525u + 1013904223u;
+    render(e, frame(1000 + (x >> 8) % 3000000, (x >> 5) & 1));
+    check(fake::held < blocks(e) + 8 * mib, "little beyond the blocks is held");
+  }
+}
+
+static void cases() {
+  slabs();
+}

@@ -194,8 +194,7 @@ ubr_status ubr_context_destroy(ubr_context* c) {
   }
   x.sceneHandles.clear();
   for (DevBuf& b : x.scratch) devFree(&x, b);
-  for (Slab& sl : x.slabs)
-    if (sl.ptr) cudaFree(sl.ptr);
+  if (x.slab.ptr) cudaFree(x.slab.ptr);  // nothing was cut from it
   if (x.pool) {
     cudaStreamSynchronize(x.stream);
     cudaMemPoolDestroy(x.pool);

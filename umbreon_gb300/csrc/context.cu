@@ -35,24 +35,49 @@ ubr_status devAlloc(Context* c, DevBuf& b, size_t bytes, bool direct) {
   return UBR_OK;
 }
 
+// A block of the slab, or null where none fits (first fit).
+static void* slabCut(Slab& s, size_t bytes) {
+  for (auto it = s.free.begin(); it != s.free.end(); ++it) {
+    if (it->second < bytes) continue;
+    void* p = static_cast<char*>(s.ptr) + it->first;
+    it->first += bytes;
+    it->second -= bytes;
+    if (it->second == 0) s.free.erase(it);
+    return p;
+  }
+  return nullptr;
+}
+
+static void slabDrop(Slab& s) {
+  cudaFree(s.ptr);
+  s = Slab{};
+}
+
+static void slabGive(Slab& s, void* p, size_t bytes) {
+  const size_t at = size_t(static_cast<char*>(p) - static_cast<char*>(s.ptr));
+  auto it = std::lower_bound(s.free.begin(), s.free.end(), std::make_pair(at, size_t(0)));
+  it = s.free.insert(it, {at, bytes});
+  if (it + 1 != s.free.end() && it->first + it->second == (it + 1)->first) {
+    it->second += (it + 1)->second;
+    s.free.erase(it + 1);
+  }
+  if (it != s.free.begin() && (it - 1)->first + (it - 1)->second == it->first) {
+    (it - 1)->second += it->second;
+    s.free.erase(it);
+  }
+  if (s.free[0].second == s.bytes) slabDrop(s);
+}
+
 void devFree(Context* c, DevBuf& b) {
   if (b.ptr) {
-    if (b.slab) {
-      Slab& s = c->slabs[size_t(b.slab) - 1];
-      if (--s.live == 0) {
-        cudaFree(s.ptr);
-        s = Slab{};
-      }
-    } else if (b.direct) {
-      cudaFree(b.ptr);
-    } else {
-      cudaFreeAsync(b.ptr, c->stream);
-    }
+    if (b.slab) slabGive(c->slab, b.ptr, b.bytes);
+    else if (b.direct) cudaFree(b.ptr);
+    else cudaFreeAsync(b.ptr, c->stream);
     c->arenaUsed -= b.bytes;
   }
   b.ptr = nullptr;
   b.bytes = 0;
-  b.slab = 0;
+  b.slab = false;
 }
 
 // Scratch blocks from this size on come from cudaMalloc: a new pool grows by
@@ -60,6 +85,9 @@ void devFree(Context* c, DevBuf& b) {
 // takes 60-110 us at any size, and a block of the scratch lives as long as its
 // context.  Scenes stay in the pool, which hands freed blocks on in 2 us.
 constexpr size_t kDirectBytes = size_t(96) << 20;
+
+static size_t withSlack(size_t bytes) { return bytes + bytes / 4; }
+static size_t slabPadded(size_t bytes) { return (bytes + 255) / 256 * 256; }
 
 ubr_status scratchGet(Context* c, int i, size_t bytes, void** out, bool slack) {
   if (size_t(i) >= c->scratch.size()) c->scratch.resize(size_t(i) + 1);
@@ -69,24 +97,21 @@ ubr_status scratchGet(Context* c, int i, size_t bytes, void** out, bool slack) {
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cudaFail(c, e, "cudaStreamSynchronize");
     devFree(c, b);
-    const size_t grown = slack ? bytes + bytes / 4 : bytes;
-    const size_t padded = (grown + 255) / 256 * 256;
-    if (!c->slabs.empty()) {
-      Slab& s = c->slabs.back();
-      if (s.ptr && s.used + padded <= s.bytes) {
-        b.ptr = static_cast<char*>(s.ptr) + s.used;
-        b.bytes = padded;
-        b.slab = int(c->slabs.size());
-        s.used += padded;
-        ++s.live;
-        c->arenaUsed += padded;
-        *out = b.ptr;
-        return UBR_OK;
-      }
+    const size_t grown = slack ? withSlack(bytes) : bytes;
+    // small blocks stay out of the slab: many never grow, and one of them would
+    // hold all of it
+    void* cut = grown >= kSlabBlock ? slabCut(c->slab, slabPadded(grown)) : nullptr;
+    if (cut) {
+      b.ptr = cut;
+      b.bytes = slabPadded(grown);
+      b.slab = true;
+      c->arenaUsed += b.bytes;
+    } else {
+      ubr_status st = devAlloc(c, b, grown, grown >= kDirectBytes);
+      if (st != UBR_OK) return st;
     }
-    ubr_status st = devAlloc(c, b, grown, grown >= kDirectBytes);
-    if (st != UBR_OK) return st;
   }
+  b.call = c->call;
   *out = b.ptr;
   return UBR_OK;
 }
@@ -95,19 +120,29 @@ ubr_status scratchGet(Context* c, int i, size_t bytes, void** out, bool slack) {
 // the pool, 65 us whenever it has to grow (by 32 MB at least) and 0.8 us per MB;
 // the slab is one cudaMalloc, worth it from about two growths on (first GI
 // frames: 640x480 pt1 791 -> 726 us, 955x198 pt1 700 -> 598).
-void scratchReserve(Context* c, size_t bytes) {
-  if (c->arenaCap != 0 || bytes < (size_t(48) << 20) || bytes > kSlabBytes) return;
+void scratchReserve(Context* c, const std::vector<ScratchNeed>& plan) {
+  if (c->slab.ptr) {
+    if (cudaStreamSynchronize(c->stream) != cudaSuccess) return;  // the next scratchGet reports it
+    for (DevBuf& b : c->scratch)
+      if (b.slab && b.call != c->call) devFree(c, b);
+    if (c->slab.ptr && c->slab.free.size() == 1 && c->slab.free[0].second == c->slab.bytes) slabDrop(c->slab);
+    if (c->slab.ptr) return;  // this call uses blocks of it already
+  }
+  size_t want = 0;
+  for (const ScratchNeed& n : plan) {
+    const size_t has = size_t(n.slot) < c->scratch.size() ? c->scratch[size_t(n.slot)].bytes : 0;
+    const size_t grown = n.slack ? withSlack(n.bytes) : n.bytes;
+    if (has < n.bytes && grown >= kSlabBlock) want += slabPadded(grown);
+  }
+  if (c->arenaCap != 0 || want < kSlabLeast || want > kSlabBytes) return;
   void* p = nullptr;
-  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+  if (cudaMalloc(&p, want) != cudaSuccess) {
     cudaGetLastError();
     return;
   }
-  // a slab nothing was cut from serves no one any more
-  if (!c->slabs.empty() && c->slabs.back().ptr && c->slabs.back().live == 0) {
-    cudaFree(c->slabs.back().ptr);
-    c->slabs.back() = Slab{};
-  }
-  c->slabs.push_back(Slab{p, bytes, 0, 0});
+  c->slab.ptr = p;
+  c->slab.bytes = want;
+  c->slab.free = {{0, want}};
 }
 
 ubr_status workspaceMin(Context* c, void** out, size_t* bytes) {

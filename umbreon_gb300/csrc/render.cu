@@ -22,6 +22,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <vector>
 
 #include "frame_planes.h"
@@ -2260,6 +2261,7 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
                      uint64_t* progress) {
   const size_t nf = jobs.size();
   if (nf == 0) return UBR_OK;
+  ++c->call;
   const bool batch = nf > 1;
   std::vector<FrameDesc> fds(nf);
   std::vector<LightD> lights;
@@ -2318,25 +2320,62 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
   // per-slot buffers hold a full frame, or one chunk of fine samples
   const uint32_t nslot = std::max(npix, k2);
   if (!batch && !adaptive && (c->scratch.size() <= 18 || c->scratch[18].bytes < size_t(npix) * sizeof(float4))) {
-    // the context's first frame of this size: its scratch in one allocation,
-    // by what is asked for below (an estimate: what does not fit is allocated
-    // on its own)
-    const size_t perPix = 52 + 40 + (secondary ? 60 + size_t(R) + (enhanced ? 4 * size_t(aoStride) : 0) : 0) +
-                          (aov ? 48 : 0) + (p1.gi ? 48 + 16 : 0) + (p1.pt2Refl ? 48 : 0) + (d0.edge_gbuffer ? 36 : 0);
-    size_t want = size_t(npix) * perPix + size_t(nout) * (16 + (aov ? 96 : 0)) + (size_t(64) << 10);
-    size_t work = 0;
+    // the context's first frame of this size: its scratch in one allocation, by
+    // what is asked for below (what is left out is allocated on its own)
+    std::vector<ScratchNeed> plan;
+    auto per = [&](size_t n, size_t bytes, std::initializer_list<int> slots) {
+      for (int slot : slots) plan.push_back({slot, n * bytes + 16});  // as scratchT
+    };
+    per(npix, 16, {16, 18});
+    per(npix, 4, {17, 19, 20, 21, 22});
+    per(nslot, 16, {23, 24});
+    per(nslot, 4, {25, 26});
+    per(nout, 16, {35});
+    if (secondary) {
+      per(nslot, 16, {27, 28, 146});
+      per(nslot, 8, {29});
+      per(nslot, 4, {36});
+      per(nslot, R, {30});
+      if (enhanced) per(nslot, 4 * size_t(aoStride), {31});
+    }
+    if (aov) {
+      per(npix, 16, {70, 71, 72});
+      per(nout, 48, {73});
+      if (d0.denoiser != 0) {
+        per(nout, 12, {108, 109});
+        per(nout, 4, {110, 111});
+        per(nout, 1, {107});
+      }
+    }
+    if (d0.edge_gbuffer) {
+      per(npix, 4, {98, 99, 101});
+      per(npix, 12, {100});
+    }
     if (p1.gi) {
-      int div = d0.pt1_gather_div < 0 ? p1.ss : d0.pt1_gather_div == 0 ? (d0.pt1_half_res ? 2 : 1) : d0.pt1_gather_div;
-      div = std::max(1, div);
+      const int div = std::max(1, d0.pt1_gather_div < 0    ? p1.ss
+                                  : d0.pt1_gather_div == 0 ? (d0.pt1_half_res ? 2 : 1)
+                                                           : d0.pt1_gather_div);
       const size_t nlo = size_t((p1.W + div - 1) / div) * size_t((p1.H + div - 1) / div);
-      want += nlo * (64 + 42 + 60) + (div > 1 ? size_t(npix) * 22 : 0);
+      per(npix, 16, {112, 113, 114, 116});
+      if (p1.pt2Refl) per(npix, 16, {141, 142});
+      if (div > 1) {
+        per(nlo, 16, {117, 118, 119, 120});
+        per(npix, 4, {126});
+        per(npix, 1, {147});
+        if (d0.pt1_edge_patch) per(npix, 16, {128});
+      }
+      if (d0.pt1_denoise) {
+        per(nlo, 1, {121});
+        per(nlo, 16, {122, 123});
+        per(nlo, 4, {124, 125});
+      }
       GiP est{};
       est.bounces = d0.gi_bounces;
       est.pt2 = d0.gi_integrator == 2;
-      est.em = jobs[0].scene->emit;
-      work = giGatherBytes(est, p1.nLights, false, nlo, d0.pt1_spp);
+      if (est.pt2 && d0.pt2_emissive && d0.pt2_emissive_nee) est.em = jobs[0].scene->emit;
+      plan.push_back({149, giGatherBytes(est, p1.nLights, false, nlo, d0.pt1_spp), false});
     }
-    scratchReserve(c, want + want / 4 + work);
+    scratchReserve(c, plan);
   }
   Bufs b{};
   b.accum = scratchT<float4>(c, 16, npix, st);

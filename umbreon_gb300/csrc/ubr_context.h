@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "gi.cuh"
@@ -18,14 +19,16 @@ struct DevBuf {
   void* ptr = nullptr;
   size_t bytes = 0;
   bool direct = false;  // from cudaMalloc, not from the context's pool
-  int slab = 0;         // > 0: part of the context's slab of that number
+  bool slab = false;    // cut from the context's slab
+  uint64_t call = 0;    // scratch: the call that asked for it last
 };
 
-// One cudaMalloc that several scratch blocks are cut from (scratchReserve).
+// One cudaMalloc that a frame's large scratch blocks are cut from
+// (scratchReserve); given back with the last of them.
 struct Slab {
   void* ptr = nullptr;
-  size_t bytes = 0, used = 0;
-  int live = 0;  // blocks cut from it and not yet freed
+  size_t bytes = 0;
+  std::vector<std::pair<size_t, size_t>> free;  // (offset, bytes) by offset, neighbours merged
 };
 
 struct Context {
@@ -42,7 +45,8 @@ struct Context {
   std::string lastError;
   // frame scratch, reused across frames
   std::vector<DevBuf> scratch;
-  std::vector<Slab> slabs;
+  Slab slab;
+  uint64_t call = 0;         // number of the running call (scratch blocks it uses carry it)
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   std::vector<cudaEvent_t> pev;  // profiling events, created on first use
   void* pinned = nullptr;    // small pinned host block for counters
@@ -89,11 +93,18 @@ void devFree(Context* c, DevBuf& b);
 // `slack` is false)
 ubr_status scratchGet(Context* c, int i, size_t bytes, void** out, bool slack = true);
 
-// Memory for the scratch blocks that the next scratchGet calls grow, `bytes` in
-// all: one allocation instead of one each.  Nothing under an arena cap, for
-// little, above kSlabBytes, or when it fails.
-void scratchReserve(Context* c, size_t bytes);
-constexpr size_t kSlabBytes = size_t(512) << 20;
+// Memory for the scratch blocks of a frame, before it asks for them: one
+// allocation for the large blocks of the plan that have to grow, instead of one
+// each.  The blocks of the last such allocation that this call
+// has not asked for are given back first, so a context holds one at a time.
+// None under an arena cap, for little, above kSlabBytes, or when it fails.
+struct ScratchNeed {
+  int slot;
+  size_t bytes;
+  bool slack = true;  // as scratchGet's
+};
+void scratchReserve(Context* c, const std::vector<ScratchNeed>& plan);
+constexpr size_t kSlabBytes = size_t(512) << 20, kSlabLeast = size_t(48) << 20, kSlabBlock = size_t(1) << 16;
 
 // A workspace of a pass that runs in chunks.  *bytes: what it uses well on
 // entry, what it got on exit (at least `least`).  Scratch slot `slot`, or,
