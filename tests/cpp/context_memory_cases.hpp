@@ -78,6 +78,65 @@ static void slabs() {
   }
 }
 
+static void workspaces() {
+  const size_t kib = 1024, mib = 1024 * kib;
+  void* p;
+  size_t n;
+  // under a cap that leaves room: all that is wanted, counted
+  Context& c = fresh(1024 * mib);
+  ++c.call;
+  n = 300 * mib;
+  check(workspaceGet(&c, kGatherSlot, 10 * kib, nullptr, 0, &p, &n) == UBR_OK && n == 300 * mib, "all it wants");
+  check(p == c.scratch[kGatherSlot].ptr && c.arenaUsed == 300 * mib, "of its own, counted");
+  scratchDone(&c, kGatherSlot);
+  consistent(c);
+  // ... and it does not stand in the way of what comes later, in this call or the next
+  check(scratchGet(&c, 16, 640 * mib, &p) == UBR_OK, "a block of the same call");
+  check(c.scratch[kGatherSlot].ptr == nullptr, "the workspace made room");
+  ++c.call;
+  n = 400 * mib;
+  check(workspaceGet(&c, kAdjointSlot, 10 * kib, nullptr, 0, &p, &n) == UBR_OK && n == 400 * mib, "lent");
+  check(p == c.scratch[16].ptr, "the block of the call before");
+  n = 2000 * mib;
+  check(workspaceGet(&c, kAdjointSlot, 10 * kib, nullptr, 0, &p, &n) == UBR_OK && n == 800 * mib, "lent whole");
+  check(scratchGet(&c, 20, 700 * mib, &p) == UBR_OK, "scratch of an earlier call makes room");
+  check(c.scratch[16].ptr == nullptr, "it went");
+  check(scratchGet(&c, 21, 200 * mib, &p) == UBR_OUT_OF_MEMORY, "this call's own does not");
+  check(c.scratch[20].ptr != nullptr, "and stays");
+  consistent(c);
+  // what a cap leaves, where that is more than what is lent
+  Context& d = fresh(64 * mib);
+  ++d.call;
+  check(scratchGet(&d, 23, 16 * mib, &p) == UBR_OK, "a plane");
+  void* const plane = p;
+  n = 100 * mib;
+  check(workspaceGet(&d, kGatherSlot, 10 * kib, plane, 16 * mib, &p, &n) == UBR_OK && n == 44 * mib, "what is left");
+  check(d.arenaUsed == 64 * mib, "the cap in full");
+  n = 100 * mib;
+  const int before = fake::calls;
+  check(workspaceGet(&d, kGatherSlot, 10 * kib, plane, 16 * mib, &p, &n) == UBR_OK && n == 44 * mib, "kept");
+  check(fake::calls == before, "not taken again");
+  check(scratchGet(&d, 24, 40 * mib, &p) == UBR_OUT_OF_MEMORY, "a workspace in use stays");
+  scratchDone(&d, kGatherSlot);
+  check(scratchGet(&d, 24, 44 * mib, &p) == UBR_OK && d.scratch[24].bytes == 44 * mib,
+        "and goes when its work is queued; no slack where the cap has no room for it");
+  n = 100 * mib;
+  check(workspaceGet(&d, kGatherSlot, 10 * kib, plane, 16 * mib, &p, &n) == UBR_OK && p == plane && n == 16 * mib,
+        "what is lent where the cap leaves less");
+  // without a cap: its own, and what is lent where the device refuses
+  Context& e = fresh(0);
+  ++e.call;
+  n = 100 * mib;
+  check(workspaceGet(&e, kGatherSlot, 10 * kib, plane, 16 * mib, &p, &n) == UBR_OK && p != plane && n == 100 * mib,
+        "its own");
+  fake::limit = 120 * mib;
+  n = 200 * mib;
+  check(workspaceGet(&e, kGatherSlot, 10 * kib, plane, 16 * mib, &p, &n) == UBR_OK && p == plane && n == 16 * mib,
+        "lent where the device has no more");
+  consistent(e);
+}
+
 static void cases() {
   slabs();
+  workspaces();
 }

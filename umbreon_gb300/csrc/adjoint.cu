@@ -824,6 +824,7 @@ ubr_status adjointCheck(Context* c, const Scene& sc, const ubr_render_desc& d, c
 }  // namespace
 
 ubr_status adjoint(Context* c, const Scene* sc, const ubr_render_desc& d, const float* dColor, ubr_grads& g) {
+  ++c->call;
   Params p;
   std::vector<LightD> lights;
   ubr_status st = makeParams(c, d, p, lights);
@@ -856,8 +857,9 @@ ubr_status adjoint(Context* c, const Scene* sc, const ubr_render_desc& d, const 
   }
   if (st != UBR_OK) return st;
   // one block: the primary hits, the packed gradient sums and a chunk's
-  // workspace; under an arena cap, or where it does not fit, the hits alone,
-  // no packed sums, and whatever workspace the context can lend
+  // workspace; where an arena cap leaves less or it does not fit, the hits
+  // alone and whatever workspace the context has, with the sums in it if they
+  // leave at least as much for the chunk
   const size_t pixBytes = 4 + 48 + size_t(p.aoSamples) * 8 + size_t(p.nLights);
   const size_t hitBytes = (size_t(npix) * sizeof(float2) + kAdjAlign) / kAdjAlign * kAdjAlign;
   // the caller's arrays get the packed sums spread over them at the end where
@@ -871,13 +873,23 @@ ubr_status adjoint(Context* c, const Scene* sc, const ubr_render_desc& d, const 
   size_t wsBytes = kAdjHeader + std::min<size_t>(size_t(npix) * pixBytes, std::max(kAdjBytes, pixBytes));
   void* ws = nullptr;
   void* block = nullptr;
-  if (c->arenaCap == 0 && scratchGet(c, 150, hitBytes + accPad + wsBytes, &block) == UBR_OK) {
+  const size_t all = hitBytes + accPad + wsBytes;
+  const size_t own = size_t(kAdjointSlot) < c->scratch.size() ? c->scratch[kAdjointSlot].bytes : 0;
+  if ((own >= all || arenaHolds(c, all - own)) && scratchGet(c, kAdjointSlot, all, &block, c->arenaCap == 0) == UBR_OK) {
     ws = static_cast<char*>(block) + hitBytes + accPad;
     if (accBytes) b.acc = reinterpret_cast<float4*>(static_cast<char*>(block) + hitBytes);
   } else {
     cudaGetLastError();
     if ((st = scratchGet(c, 60, hitBytes, &block)) != UBR_OK) return st;
-    if ((st = workspaceGet(c, 150, kAdjHeader + pixBytes, &ws, &wsBytes)) != UBR_OK) return st;
+    size_t got = accPad + wsBytes;
+    const size_t least = kAdjHeader + pixBytes;
+    if ((st = workspaceGet(c, kAdjointSlot, least, nullptr, 0, &ws, &got)) != UBR_OK) return st;
+    if (accBytes && got >= accPad + std::max(least, accPad)) {
+      b.acc = reinterpret_cast<float4*>(ws);
+      ws = static_cast<char*>(ws) + accPad;
+      got -= accPad;
+    }
+    wsBytes = std::min(wsBytes, got);
   }
   float2* hit = static_cast<float2*>(block);
   cudaEventRecord(c->ev[0], s);

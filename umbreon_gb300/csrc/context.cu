@@ -19,10 +19,34 @@ ubr_status cudaFail(Context* c, cudaError_t e, const char* what) {
   return setError(c, e == cudaErrorMemoryAllocation ? UBR_OUT_OF_MEMORY : UBR_CUDA_ERROR, m);
 }
 
+bool arenaHolds(const Context* c, size_t bytes) {
+  return !c->arenaCap || bytes <= c->arenaCap - c->arenaUsed;
+}
+
+// Makes room for `bytes` under the arena cap: scratch that the running call has
+// not asked for goes, workspaces first, then the largest.  Frees are ordered
+// after the work in flight, and a captured graph's key holds the scratch that
+// its launches use, so it is captured again when they have moved.
+static void releaseIdle(Context* c, size_t bytes) {
+  while (!arenaHolds(c, bytes)) {
+    int pick = -1;
+    auto rank = [&](int i) {
+      const bool workspace = i == kGatherSlot || i == kAdjointSlot;
+      return std::make_pair(workspace, c->scratch[size_t(i)].bytes);
+    };
+    for (int i = 0; i < int(c->scratch.size()); ++i) {
+      const DevBuf& b = c->scratch[size_t(i)];
+      if (b.ptr && b.call != c->call && (pick < 0 || rank(i) > rank(pick))) pick = i;
+    }
+    if (pick < 0) return;
+    devFree(c, c->scratch[size_t(pick)]);
+  }
+}
+
 ubr_status devAlloc(Context* c, DevBuf& b, size_t bytes, bool direct) {
   if (bytes == 0) bytes = 16;
-  if (c->arenaCap && c->arenaUsed + bytes > c->arenaCap)
-    return setError(c, UBR_OUT_OF_MEMORY, "device arena cap exceeded");
+  if (!arenaHolds(c, bytes)) releaseIdle(c, bytes);
+  if (!arenaHolds(c, bytes)) return setError(c, UBR_OUT_OF_MEMORY, "device arena cap exceeded");
   void* p = nullptr;
   // stream-ordered from the context's pool: after the first frames a scene
   // build or a scratch growth reuses pooled memory instead of cudaMalloc
@@ -108,6 +132,8 @@ ubr_status scratchGet(Context* c, int i, size_t bytes, void** out, bool slack) {
       c->arenaUsed += b.bytes;
     } else {
       ubr_status st = devAlloc(c, b, grown, grown >= kDirectBytes);
+      // what the cap has no room for with the slack it may have without
+      if (st == UBR_OUT_OF_MEMORY && c->arenaCap && bytes < grown) st = devAlloc(c, b, bytes, bytes >= kDirectBytes);
       if (st != UBR_OK) return st;
     }
   }
@@ -152,27 +178,44 @@ ubr_status workspaceMin(Context* c, void** out, size_t* bytes) {
   return UBR_OK;
 }
 
-ubr_status workspaceGet(Context* c, int slot, size_t least, void** out, size_t* bytes) {
-  if (c->arenaCap == 0) {
-    if (scratchGet(c, slot, *bytes, out) == UBR_OK) return UBR_OK;
+void scratchDone(Context* c, int slot) {
+  if (size_t(slot) < c->scratch.size()) c->scratch[size_t(slot)].call = 0;
+}
+
+ubr_status workspaceGet(Context* c, int slot, size_t least, void* lent, size_t lentBytes, void** out, size_t* bytes) {
+  if (size_t(slot) >= c->scratch.size()) c->scratch.resize(size_t(slot) + 1);
+  const size_t want = *bytes, own = c->scratch[size_t(slot)].bytes;
+  // the largest block that the running call does not use
+  for (size_t k = 0; k < c->scratch.size(); ++k) {
+    const DevBuf& b = c->scratch[k];
+    if (int(k) == slot || !b.ptr || b.call == c->call || b.bytes <= lentBytes) continue;
+    lent = b.ptr;
+    lentBytes = b.bytes;
+  }
+  // a block of its own: all it wants, or what the cap leaves where that is more
+  // than there is without (by a quarter, lest it grow a little in every call)
+  const size_t room = c->arenaCap ? c->arenaCap - c->arenaUsed + own : want, fit = std::min(want, room);
+  if (own >= want || fit == want || (fit >= least && fit > lentBytes && fit > own + own / 4)) {
+    *bytes = std::min(want, std::max(own, fit));
+    if (scratchGet(c, slot, *bytes, out, false) == UBR_OK) return UBR_OK;
     cudaGetLastError();
   }
-  const DevBuf* lend = nullptr;
-  for (int k = 16; k <= 31 && size_t(k) < c->scratch.size(); ++k)
-    if (c->scratch[size_t(k)].ptr && (!lend || c->scratch[size_t(k)].bytes > lend->bytes)) lend = &c->scratch[size_t(k)];
-  if (lend && lend->bytes >= std::max(least, kWorkspaceMin)) {
-    *out = lend->ptr;
-    *bytes = std::min(*bytes, lend->bytes);
+  if (c->scratch[size_t(slot)].bytes >= std::max(least, lentBytes)) {
+    *bytes = c->scratch[size_t(slot)].bytes;
+    return scratchGet(c, slot, *bytes, out, false);
+  }
+  if (lentBytes >= least) {
+    *out = lent;
+    *bytes = std::min(want, lentBytes);
     return UBR_OK;
   }
   if (least <= kWorkspaceMin) {
-    const size_t want = *bytes;
     const ubr_status st = workspaceMin(c, out, bytes);
     *bytes = std::min(*bytes, std::max(want, least));
     return st;
   }
   *bytes = least;
-  return scratchGet(c, slot, least, out);
+  return scratchGet(c, slot, least, out, false);
 }
 
 }  // namespace ubr

@@ -1856,6 +1856,7 @@ static size_t gatherSlotBytes(const GiP& g, int nLights, bool area) {
   return 16 + (lean ? 48 : 64) + (g.bounces > 1 ? 32 + 64 : 0) + nl * (area ? 21 : 5) + (g.pt2 && g.em.n > 0 ? 8 : 0) + (g.rsv ? 32 : 0);
 }
 constexpr size_t kWaveHeader = 256, kWaveAlign = 256, kWaveArrays = 20;
+constexpr size_t kCarryBytes = size_t(kCarryF4) * 16 * 32;  // windows run one group at a time
 // A chunk: enough rays that its first and last wave of blocks weigh little, in
 // a workspace of the size of a frame's own buffers (0.3 GB with two lights):
 // 2^20 slots are 8 % slower on the pt2 default frame, 2^24 1.5 % faster.
@@ -1868,7 +1869,13 @@ size_t giGatherBytes(const GiP& g, int nLights, bool area, uint64_t n, int spp) 
   const uint64_t slots = (n + P - 1) / P * iters * 32u;
   const size_t sb = gatherSlotBytes(g, nLights, area);
   const uint64_t cap = std::min<uint64_t>(kWaveSlots, kWaveBytes / sb);
-  return std::max(kGatherMin, kWaveHeader + kWaveArrays * kWaveAlign + size_t(std::min(slots, cap)) * sb);
+  return std::max(giGatherLeast(g, nLights, area),
+                  kWaveHeader + kWaveArrays * kWaveAlign + size_t(std::min(slots, cap)) * sb);
+}
+
+size_t giGatherLeast(const GiP& g, int nLights, bool area) {
+  // one warp of slots and what a window carries on
+  return kWaveHeader + kWaveArrays * kWaveAlign + kCarryBytes + 32u * gatherSlotBytes(g, nLights, area);
 }
 
 cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, const LightD* lights, int nLights,
@@ -1883,12 +1890,11 @@ cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, con
   const uint32_t P = 32u >> w.logLanes;
   w.itEnd = std::max(1, (w.spp + (1 << w.logLanes) - 1) >> w.logLanes);
   const size_t sb = gatherSlotBytes(g, nLights, area);
-  const size_t carryBytes = size_t(kCarryF4) * 16 * 32;  // windows run one group at a time
   const size_t room = std::min<size_t>(wsBytes - kWaveHeader - kWaveArrays * kWaveAlign, kWaveSlots * sb);
   uint64_t groupsFit = room / (size_t(w.itEnd) * 32u * sb);
   w.iters = w.itEnd;
   if (groupsFit == 0) {
-    w.iters = int(std::max<size_t>(1, (room - carryBytes) / (32u * sb)));
+    w.iters = int(std::max<size_t>(1, (room - kCarryBytes) / (32u * sb)));
     groupsFit = 1;
   }
   cudaError_t e = cudaMemsetAsync(w.ctr, 0, 4 * sizeof(uint32_t), s);
@@ -1942,7 +1948,7 @@ cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, con
   w.vis = reinterpret_cast<uint8_t*>(take(size_t(slotCap) * nl));
   if (emit) w.rng = reinterpret_cast<uint2*>(take(size_t(slotCap) * 8));
   if (g.rsv) w.cand = reinterpret_cast<float4*>(take(size_t(slotCap) * 32));
-  if (w.iters < w.itEnd) w.carry = reinterpret_cast<float4*>(take(carryBytes));
+  if (w.iters < w.itEnd) w.carry = reinterpret_cast<float4*>(take(kCarryBytes));
   const int itWindow = w.iters;
   for (uint64_t g0 = 0; g0 < groups; g0 += perChunk) {
     w.p0 = uint32_t(g0 * P);

@@ -100,10 +100,10 @@ void giGBuffer(int km, cudaStream_t s, const Params& p, const DScene& sc, int w,
 // The gather over a grid (list null: its eligible points, listed in listBuf of
 // n; the others get E = 0) or over the points of a list (listCount of them, on
 // the device).  Runs in chunks that fit the workspace ws of wsBytes, at least
-// kGatherMin; giGatherBytes is what n points use well.  Reads the number
+// giGatherLeast; giGatherBytes is what n points use well.  Reads the number
 // of points back (hostCount, pinned) when they may need more than one chunk.
 // area: some light's shadow rays are jittered (pt2, radius > 0).
-constexpr size_t kGatherMin = size_t(1) << 16;
+size_t giGatherLeast(const GiP& g, int nLights, bool area);
 size_t giGatherBytes(const GiP& g, int nLights, bool area, uint64_t n, int spp);
 cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, const LightD* lights, int nLights,
                      bool area, const GiGrid& grid, const uint32_t* list, const uint32_t* listCount, uint32_t n, int spp,

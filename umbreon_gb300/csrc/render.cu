@@ -2373,7 +2373,7 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
       est.bounces = d0.gi_bounces;
       est.pt2 = d0.gi_integrator == 2;
       if (est.pt2 && d0.pt2_emissive && d0.pt2_emissive_nee) est.em = jobs[0].scene->emit;
-      plan.push_back({149, giGatherBytes(est, p1.nLights, false, nlo, d0.pt1_spp), false});
+      plan.push_back({kGatherSlot, giGatherBytes(est, p1.nLights, false, nlo, d0.pt1_spp), false});
     }
     scratchReserve(c, plan);
   }
@@ -2981,30 +2981,21 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
       return UBR_OK;
     };
     // the gather of `n` points of a grid or list.  Its workspace is context
-    // scratch of its own; under an arena cap, or where that allocation fails,
-    // the hit records of the finished layers (16 B per hi-res pixel) or, for a
-    // frame of few pixels, a small block outside the cap
+    // scratch of its own; where an arena cap leaves little or the allocation
+    // fails, the hit records of the finished layers (16 B per hi-res pixel) or
+    // another block that is idle
     auto gather = [&](const GiP& gg, const GiGrid& gr, const uint32_t* list, const uint32_t* cnt, uint32_t n, int nspp,
                       float4* E) -> ubr_status {
       // (a list names the points on the device: room for a sixteenth of the
       // grid, about what edges and noise take, and more chunks past that)
-      const size_t want = giGatherBytes(gg, nL, area, list ? n / 16 + 32 : n, nspp);
+      size_t bytes = giGatherBytes(gg, nL, area, list ? n / 16 + 32 : n, nspp);
       void* ws = nullptr;
-      size_t bytes = want;
-      if (c->arenaCap == 0 && scratchGet(c, 149, want, &ws, false) != UBR_OK) {
-        cudaGetLastError();
-        ws = nullptr;
-      }
-      if (!ws) {
-        ws = b.hitA;
-        bytes = size_t(nslot) * sizeof(float4);
-        if (bytes < kWorkspaceMin) {
-          const ubr_status ms = workspaceMin(c, &ws, &bytes);
-          if (ms != UBR_OK) return ms;
-        }
-      }
+      const ubr_status wst = workspaceGet(c, kGatherSlot, giGatherLeast(gg, nL, area), b.hitA,
+                                          size_t(nslot) * sizeof(float4), &ws, &bytes);
+      if (wst != UBR_OK) return wst;
       // the eligible points of a grid are listed in the first queue buffer
       UBR_CUDA(c, giGather(km, s, gg, s1, lt, nL, area, gr, list, cnt, n, nspp, E, q0, ws, bytes, hostCount + 8, &kernels));
+      scratchDone(c, kGatherSlot);
       return UBR_OK;
     };
     // the gather over a grid, with pt2's adaptive refinement (pt2_adaptive.hpp:
@@ -3463,6 +3454,7 @@ ubr_status finishQuery(Context* c, const unsigned long long* stats) {
 
 ubr_status occludedBatch(Context* c, const Scene* sc, const float* segs, uint64_t n, float eps, uint8_t* out,
                          int32_t memory) {
+  ++c->call;
   if (n == 0) return UBR_OK;
   if (!segs || !out) return setError(c, UBR_INVALID_ARGUMENT, "occluded_batch: NULL buffer");
   ubr_status st = UBR_OK;
@@ -3489,6 +3481,7 @@ ubr_status occludedBatch(Context* c, const Scene* sc, const float* segs, uint64_
 ubr_status occludedFilteredBatch(Context* c, const Scene* sc, const float* segs, uint64_t n, float eps,
                                  float grazeCos, float coplanar, const uint32_t* offs, const int32_t* faces,
                                  uint8_t* out, int32_t memory) {
+  ++c->call;
   if (n == 0) return UBR_OK;
   if (!segs || !out) return setError(c, UBR_INVALID_ARGUMENT, "occluded_filtered_batch: NULL buffer");
   if ((offs == nullptr) != (faces == nullptr))

@@ -1378,6 +1378,7 @@ int bitsFor(uint32_t n) {
 
 ubr_status buildScene(Context* c, const ubr_scene_desc& d, Scene** out) {
   const auto t0 = std::chrono::steady_clock::now();
+  ++c->call;
   ubr_status st = validate(c, d);
   if (st != UBR_OK) return st;
   // host staging of the flattened tables, reused by this thread's next build

@@ -106,13 +106,23 @@ struct ScratchNeed {
 void scratchReserve(Context* c, const std::vector<ScratchNeed>& plan);
 constexpr size_t kSlabBytes = size_t(512) << 20, kSlabLeast = size_t(48) << 20, kSlabBlock = size_t(1) << 16;
 
+// Whether the arena cap leaves `bytes` (always without a cap).
+bool arenaHolds(const Context* c, size_t bytes);
+
 // A workspace of a pass that runs in chunks.  *bytes: what it uses well on
-// entry, what it got on exit (at least `least`).  Scratch slot `slot`, or,
-// under an arena cap and where that allocation fails, memory the context holds
-// already: the largest frame buffer that is idle outside a render (slots
-// 16..31), or a small block outside the cap (workspaceMin).
+// entry, what it got on exit (at least `least`).  Scratch slot `slot`: all it
+// wants, or what the arena cap leaves; where that is little or the allocation
+// fails, memory that the context holds already, a block the running call does
+// not use or what it lends (`lent`, may be null); else a small block outside the
+// cap (workspaceMin).  A workspace does not stand in the way of other calls:
+// where the cap would refuse an allocation, scratch that the running call has
+// not asked for is released first.
+constexpr int kGatherSlot = 149, kAdjointSlot = 150;
 ubr_status workspaceMin(Context* c, void** out, size_t* bytes);
-ubr_status workspaceGet(Context* c, int slot, size_t least, void** out, size_t* bytes);
+ubr_status workspaceGet(Context* c, int slot, size_t least, void* lent, size_t lentBytes, void** out, size_t* bytes);
+// The running call has queued its last work on this block: other calls of this
+// one's allocations may release it (ordered after that work).
+void scratchDone(Context* c, int slot);
 constexpr size_t kWorkspaceMin = size_t(1) << 16;
 
 // typed view of scratch slot `slot` (count elements); a no-op once st != OK
