@@ -136,7 +136,50 @@ static void workspaces() {
   consistent(e);
 }
 
+static void hardCap() {
+  const size_t kib = 1024, mib = 1024 * kib;
+  void* p;
+  size_t n;
+  // a cap that leaves less than the least workspace, and nothing to lend
+  Context& c = fresh(1 * mib);
+  ++c.call;
+  check(scratchGet(&c, 16, 1 * mib - 4 * kib, &p) == UBR_OK, "nearly all of it");
+  n = 10 * mib;
+  check(workspaceGet(&c, kAdjointSlot, 5 * kib, nullptr, 0, &p, &n) == UBR_OUT_OF_MEMORY, "refused");
+  check(fake::peak <= c.arenaCap, "and the cap holds");
+  n = 10 * mib;
+  check(workspaceGet(&c, kAdjointSlot, 4 * kib, nullptr, 0, &p, &n) == UBR_OK && n == 4 * kib, "what is left");
+  check(fake::held == c.arenaCap && c.arenaUsed == c.arenaCap, "all counted");
+  consistent(c);
+  // random calls: blocks and workspaces, refused or not, stay within the cap
+  unsigned x = 7;
+  auto draw = [&](size_t most) {
+    x = x * 1664525u + 1013904223u;
+    return 1 + size_t(x >> 8) % most;
+  };
+  for (int round = 0; round < 20; ++round) {
+    Context& d = fresh(draw(2 * mib));
+    for (int k = 0; k < 100; ++k) {
+      ++d.call;
+      for (int b = int(draw(4)); b > 0; --b) {
+        n = draw(300 * kib);
+        scratchGet(&d, int(draw(12)), n, &p);
+      }
+      const size_t least = draw(20 * kib), lent = draw(2) == 1 ? draw(40 * kib) : 0;
+      char frame[1];
+      n = least + draw(600 * kib);
+      const ubr_status st = workspaceGet(&d, kGatherSlot, least, lent ? frame : nullptr, lent, &p, &n);
+      check(st != UBR_OK || n >= least, "at least what it asks for");
+      check(st == UBR_OK || lent < least, "what is lent serves");
+      if (draw(2) == 1) scratchDone(&d, kGatherSlot);
+      check(fake::peak <= d.arenaCap, "the cap is hard");
+      consistent(d);
+    }
+  }
+}
+
 static void cases() {
   slabs();
   workspaces();
+  hardCap();
 }

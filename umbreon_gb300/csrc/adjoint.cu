@@ -797,9 +797,14 @@ __global__ void k_adj_down(Params p, const float4* colorHi, float4* out, uint32_
   out[o] = make_float4(a[0] * inv, a[1] * inv, a[2] * inv, a[3] * inv);
 }
 
-// Workspace of a chunk of pixels: a header and alignment, and at most
-// kAdjBytes of queue and ray results.
-constexpr size_t kAdjAlign = 256, kAdjHeader = 8 * kAdjAlign, kAdjBytes = size_t(256) << 20;
+// Workspace of a chunk of pixels: a counter and kAdjArrays arrays of queue and
+// ray results, at most kAdjBytes of them.  They start on a block of the memory,
+// or on a float4 where an arena cap leaves room for a few pixels only.
+constexpr size_t kAdjAlign = 256, kAdjArrays = 7, kAdjBytes = size_t(256) << 20;
+constexpr size_t adjHeader(size_t align) { return (kAdjArrays + 1) * align; }
+size_t adjAlign(size_t wsBytes, size_t pixBytes) {
+  return wsBytes >= adjHeader(kAdjAlign) + 32 * pixBytes ? kAdjAlign : 16;
+}
 
 ubr_status adjointCheck(Context* c, const Scene& sc, const ubr_render_desc& d, const Params& p) {
   if (sc.primCount[kMesh] || sc.primCount[kRound] || sc.primCount[kCone])
@@ -870,7 +875,7 @@ ubr_status adjoint(Context* c, const Scene* sc, const ubr_render_desc& d, const 
                                (!gRad || deviceHolds(c->device, gRad, nSph * sizeof(float))));
   const size_t accBytes = spread && (gCol || gCen || gRad) ? size_t(nSph) * 32 : 0;
   const size_t accPad = (accBytes + kAdjAlign - 1) / kAdjAlign * kAdjAlign;
-  size_t wsBytes = kAdjHeader + std::min<size_t>(size_t(npix) * pixBytes, std::max(kAdjBytes, pixBytes));
+  size_t wsBytes = adjHeader(kAdjAlign) + std::min<size_t>(size_t(npix) * pixBytes, std::max(kAdjBytes, pixBytes));
   void* ws = nullptr;
   void* block = nullptr;
   const size_t all = hitBytes + accPad + wsBytes;
@@ -880,9 +885,9 @@ ubr_status adjoint(Context* c, const Scene* sc, const ubr_render_desc& d, const 
     if (accBytes) b.acc = reinterpret_cast<float4*>(static_cast<char*>(block) + hitBytes);
   } else {
     cudaGetLastError();
-    if ((st = scratchGet(c, 60, hitBytes, &block)) != UBR_OK) return st;
+    if ((st = scratchGet(c, 60, size_t(npix) * sizeof(float2), &block)) != UBR_OK) return st;
     size_t got = accPad + wsBytes;
-    const size_t least = kAdjHeader + pixBytes;
+    const size_t least = adjHeader(16) + pixBytes;
     if ((st = workspaceGet(c, kAdjointSlot, least, nullptr, 0, &ws, &got)) != UBR_OK) return st;
     if (accBytes && got >= accPad + std::max(least, accPad)) {
       b.acc = reinterpret_cast<float4*>(ws);
@@ -924,13 +929,14 @@ ubr_status adjoint(Context* c, const Scene* sc, const ubr_render_desc& d, const 
   k_adj_primary<<<grid, TB, 0, s>>>(p, travOf(sc->view), hit, npix, stats);
   // pixels per chunk: what the workspace's queue and ray results hold
   const uint32_t S = uint32_t(p.aoSamples), nL = uint32_t(p.nLights);
-  char* at = static_cast<char*>(ws) + kAdjAlign;
+  const size_t align = adjAlign(wsBytes, pixBytes);
+  char* at = static_cast<char*>(ws) + align;
   auto take = [&](size_t n) {
     char* q = at;
-    at += (n + kAdjAlign - 1) / kAdjAlign * kAdjAlign;
+    at += (n + align - 1) / align * align;
     return q;
   };
-  const uint32_t chunk = uint32_t(std::min<size_t>(npix, (wsBytes - kAdjHeader) / pixBytes));
+  const uint32_t chunk = uint32_t(std::min<size_t>(npix, (wsBytes - adjHeader(align)) / pixBytes));
   AdjRays r{};
   r.count = static_cast<uint32_t*>(ws);
   r.pix = reinterpret_cast<uint32_t*>(take(size_t(chunk) * 4));

@@ -207,7 +207,6 @@ ubr_status ubr_context_destroy(ubr_context* c) {
   for (cudaEvent_t& e : x.giEv)
     if (e) cudaEventDestroy(e);
   if (x.graphExec) cudaGraphExecDestroy(x.graphExec);
-  if (x.workMin) cudaFree(x.workMin);
   if (x.pinned) cudaFreeHost(x.pinned);
   if (x.ownStream && x.stream) cudaStreamDestroy(x.stream);
   delete c;

@@ -171,13 +171,6 @@ void scratchReserve(Context* c, const std::vector<ScratchNeed>& plan) {
   c->slab.free = {{0, want}};
 }
 
-ubr_status workspaceMin(Context* c, void** out, size_t* bytes) {
-  if (!c->workMin) UBR_CUDA(c, cudaMalloc(&c->workMin, kWorkspaceMin));
-  *out = c->workMin;
-  *bytes = kWorkspaceMin;
-  return UBR_OK;
-}
-
 void scratchDone(Context* c, int slot) {
   if (size_t(slot) < c->scratch.size()) c->scratch[size_t(slot)].call = 0;
 }
@@ -208,11 +201,6 @@ ubr_status workspaceGet(Context* c, int slot, size_t least, void* lent, size_t l
     *out = lent;
     *bytes = std::min(want, lentBytes);
     return UBR_OK;
-  }
-  if (least <= kWorkspaceMin) {
-    const ubr_status st = workspaceMin(c, out, bytes);
-    *bytes = std::min(*bytes, std::max(want, least));
-    return st;
   }
   *bytes = least;
   return scratchGet(c, slot, least, out, false);

@@ -1855,27 +1855,37 @@ static size_t gatherSlotBytes(const GiP& g, int nLights, bool area) {
   const bool lean = g.bounces <= 1 && !(g.pt2 && g.em.n > 0);
   return 16 + (lean ? 48 : 64) + (g.bounces > 1 ? 32 + 64 : 0) + nl * (area ? 21 : 5) + (g.pt2 && g.em.n > 0 ? 8 : 0) + (g.rsv ? 32 : 0);
 }
-constexpr size_t kWaveHeader = 256, kWaveAlign = 256, kWaveArrays = 20;
+constexpr size_t kWaveArrays = 21;  // at most, with the counters
 constexpr size_t kCarryBytes = size_t(kCarryF4) * 16 * 32;  // windows run one group at a time
+// Boundary the workspace's arrays start on: a block of the memory, or a float4
+// where an arena cap leaves room for a few warps of slots only.
+static size_t waveAlign(size_t wsBytes, size_t slotBytes) {
+  return wsBytes >= kWaveArrays * 256 + kCarryBytes + 128u * slotBytes ? 256 : 16;
+}
 // A chunk: enough rays that its first and last wave of blocks weigh little, in
 // a workspace of the size of a frame's own buffers (0.3 GB with two lights):
 // 2^20 slots are 8 % slower on the pt2 default frame, 2^24 1.5 % faster.
 constexpr uint64_t kWaveSlots = 1u << 22;
 constexpr size_t kWaveBytes = size_t(1) << 30;
 
-size_t giGatherBytes(const GiP& g, int nLights, bool area, uint64_t n, int spp) {
+// Warps of slots that follow one another per group of points.
+static uint64_t gatherIters(const GiP& g, int spp) {
   const int lg = gatherLogLanes(g, spp);
-  const uint64_t P = 32u >> lg, iters = (uint64_t(std::max(spp, 1)) + (1u << lg) - 1) >> lg;
-  const uint64_t slots = (n + P - 1) / P * iters * 32u;
-  const size_t sb = gatherSlotBytes(g, nLights, area);
-  const uint64_t cap = std::min<uint64_t>(kWaveSlots, kWaveBytes / sb);
-  return std::max(giGatherLeast(g, nLights, area),
-                  kWaveHeader + kWaveArrays * kWaveAlign + size_t(std::min(slots, cap)) * sb);
+  return (uint64_t(std::max(spp, 1)) + (1u << lg) - 1) >> lg;
 }
 
-size_t giGatherLeast(const GiP& g, int nLights, bool area) {
-  // one warp of slots and what a window carries on
-  return kWaveHeader + kWaveArrays * kWaveAlign + kCarryBytes + 32u * gatherSlotBytes(g, nLights, area);
+size_t giGatherBytes(const GiP& g, int nLights, bool area, uint64_t n, int spp) {
+  const uint64_t P = 32u >> gatherLogLanes(g, spp);
+  const uint64_t slots = (n + P - 1) / P * gatherIters(g, spp) * 32u;
+  const size_t sb = gatherSlotBytes(g, nLights, area);
+  const uint64_t cap = std::min<uint64_t>(kWaveSlots, kWaveBytes / sb);
+  return std::max(giGatherLeast(g, nLights, area, spp), kWaveArrays * 256 + size_t(std::min(slots, cap)) * sb);
+}
+
+size_t giGatherLeast(const GiP& g, int nLights, bool area, int spp) {
+  // one group's slots, or one warp of them and what a window carries on
+  const size_t warp = 32u * gatherSlotBytes(g, nLights, area);
+  return kWaveArrays * 16 + std::min<size_t>(gatherIters(g, spp) * warp, kCarryBytes + warp);
 }
 
 cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, const LightD* lights, int nLights,
@@ -1888,9 +1898,9 @@ cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, con
   w.spp = std::max(spp, 0);
   w.logLanes = gatherLogLanes(g, spp);
   const uint32_t P = 32u >> w.logLanes;
-  w.itEnd = std::max(1, (w.spp + (1 << w.logLanes) - 1) >> w.logLanes);
-  const size_t sb = gatherSlotBytes(g, nLights, area);
-  const size_t room = std::min<size_t>(wsBytes - kWaveHeader - kWaveArrays * kWaveAlign, kWaveSlots * sb);
+  w.itEnd = int(gatherIters(g, spp));
+  const size_t sb = gatherSlotBytes(g, nLights, area), align = waveAlign(wsBytes, sb);
+  const size_t room = std::min<size_t>(wsBytes - kWaveArrays * align, kWaveSlots * sb);
   uint64_t groupsFit = room / (size_t(w.itEnd) * 32u * sb);
   w.iters = w.itEnd;
   if (groupsFit == 0) {
@@ -1927,10 +1937,10 @@ cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, con
   const int maxB = g.bounces < 1 ? 1 : g.bounces;
   const uint64_t slotCap = perChunk * uint64_t(w.iters) * 32u;
   // carve the workspace
-  char* at = static_cast<char*>(ws) + kWaveHeader;
+  char* at = static_cast<char*>(ws) + align;
   auto take = [&](size_t bytes) {
     char* p = at;
-    at += (bytes + kWaveAlign - 1) / kWaveAlign * kWaveAlign;
+    at += (bytes + align - 1) / align * align;
     return p;
   };
   auto f4 = [&]() { return reinterpret_cast<float4*>(take(size_t(slotCap) * 16)); };

@@ -103,7 +103,7 @@ void giGBuffer(int km, cudaStream_t s, const Params& p, const DScene& sc, int w,
 // giGatherLeast; giGatherBytes is what n points use well.  Reads the number
 // of points back (hostCount, pinned) when they may need more than one chunk.
 // area: some light's shadow rays are jittered (pt2, radius > 0).
-size_t giGatherLeast(const GiP& g, int nLights, bool area);
+size_t giGatherLeast(const GiP& g, int nLights, bool area, int spp);
 size_t giGatherBytes(const GiP& g, int nLights, bool area, uint64_t n, int spp);
 cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, const LightD* lights, int nLights,
                      bool area, const GiGrid& grid, const uint32_t* list, const uint32_t* listCount, uint32_t n, int spp,

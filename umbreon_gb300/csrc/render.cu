@@ -2990,7 +2990,7 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
       // grid, about what edges and noise take, and more chunks past that)
       size_t bytes = giGatherBytes(gg, nL, area, list ? n / 16 + 32 : n, nspp);
       void* ws = nullptr;
-      const ubr_status wst = workspaceGet(c, kGatherSlot, giGatherLeast(gg, nL, area), b.hitA,
+      const ubr_status wst = workspaceGet(c, kGatherSlot, giGatherLeast(gg, nL, area, nspp), b.hitA,
                                           size_t(nslot) * sizeof(float4), &ws, &bytes);
       if (wst != UBR_OK) return wst;
       // the eligible points of a grid are listed in the first queue buffer

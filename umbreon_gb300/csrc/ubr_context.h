@@ -56,7 +56,6 @@ struct Context {
   std::vector<void*> sceneHandles;      // live ubr_scene handles built on this context
   cudaMemPool_t pool = nullptr;         // stream-ordered device allocations (scenes, scratch)
   void* noallocArray = nullptr;         // device address of the allocation-free query's fixed array
-  void* workMin = nullptr;              // workspace of last resort (kWorkspaceMin bytes), on first use
   cudaEvent_t giEv[7] = {};             // GI pass stage boundaries, created on first use
 };
 
@@ -113,17 +112,15 @@ bool arenaHolds(const Context* c, size_t bytes);
 // entry, what it got on exit (at least `least`).  Scratch slot `slot`: all it
 // wants, or what the arena cap leaves; where that is little or the allocation
 // fails, memory that the context holds already, a block the running call does
-// not use or what it lends (`lent`, may be null); else a small block outside the
-// cap (workspaceMin).  A workspace does not stand in the way of other calls:
-// where the cap would refuse an allocation, scratch that the running call has
-// not asked for is released first.
+// not use or what it lends (`lent`, may be null); else `least`, if the cap holds
+// that.  A workspace does not stand in the way of other calls: where the cap
+// would refuse an allocation, scratch that the running call has not asked for is
+// released first.
 constexpr int kGatherSlot = 149, kAdjointSlot = 150;
-ubr_status workspaceMin(Context* c, void** out, size_t* bytes);
 ubr_status workspaceGet(Context* c, int slot, size_t least, void* lent, size_t lentBytes, void** out, size_t* bytes);
 // The running call has queued its last work on this block: other calls of this
 // one's allocations may release it (ordered after that work).
 void scratchDone(Context* c, int slot);
-constexpr size_t kWorkspaceMin = size_t(1) << 16;
 
 // typed view of scratch slot `slot` (count elements); a no-op once st != OK
 template <class T>
