@@ -27,6 +27,7 @@
 
 #include "frame_planes.h"
 #include "gi.cuh"
+#include "occlusion_choice.h"
 #include "trace.cuh"
 
 namespace ubr {
@@ -2175,19 +2176,6 @@ uint32_t smCount(int device) {
   return uint32_t(std::max(1, sms));
 }
 
-// Whether a launch of n hits' rays (R each, n counting the misses too, as the
-// host knows it) runs the persistent kernel: binary answers, spheres and
-// cylinders only (with triangles the larger ray state costs 5-10 %), and
-// enough rays.  Ball-and-stick of 5 k atoms, one thread per ray against the
-// persistent kernel: 640x480 with 18 rays (5.5 M) 0.353 / 0.378 ms, 800x600
-// (8.6 M) 0.501 / 0.510, 1024x768 (14 M) 0.723 / 0.700, 1280x720 ss2 (66 M)
-// 2.61 / 2.26.
-constexpr uint64_t kFetchRays = 12000000;
-bool chooseFetch(int mode, int km, bool nearest, uint64_t n, uint64_t R) {
-  if (mode != 0) return mode == 2;
-  return !nearest && !(km & kMaskMesh) && n * R >= kFetchRays;
-}
-
 uint32_t gridStrideGrid(int device) {
   static int cached[64] = {};
   if (device >= 0 && device < 64 && cached[device]) return uint32_t(cached[device]);
@@ -2645,7 +2633,7 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
       mark(1, false);
       const uint64_t nr = uint64_t(n) * uint64_t(Rr);
       mark(2, true);
-      if (chooseFetch(c->traceMode, km, nearest, n, Rr))
+      if (chooseFetch(c->traceMode, (km & kMaskMesh) != 0, nearest, n, Rr))
         UBR_CUDA(c, launchOcclusionPersistent(km, count, batch, c->traceMode == 2, c->device, s, pr, s1, bt, br));
       else if (c->traceMode == 3)
         launchOcclusionGridStride(km, count, batch, gridStrideGrid(c->device), TB, s, pr, s1, bt, br);
@@ -2673,7 +2661,7 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
     mark(1, false);
     const uint64_t nr = uint64_t(nCell) * uint64_t(pCoarse.raysPerHit);
     mark(2, true);
-    if (chooseFetch(c->traceMode, km, nearest, nCell, uint64_t(pCoarse.raysPerHit)))
+    if (chooseFetch(c->traceMode, (km & kMaskMesh) != 0, nearest, nCell, uint64_t(pCoarse.raysPerHit)))
       UBR_CUDA(c, launchOcclusionPersistent(km, count, false, c->traceMode == 2, c->device, s, pCoarse, s1, bt, b));
     else if (c->traceMode == 3)
       launchOcclusionGridStride(km, count, false, gridStrideGrid(c->device), TB, s, pCoarse, s1, bt, b);
