@@ -394,9 +394,6 @@ UBR_D bool closestPhase(const TravScene& s, const Ray& r, const TriPre& pre, int
   return false;
 }
 
-// Visit st.node: test its 8 children, its hit leaves' primitives, choose the
-// next node.  Returns true when the ray is finished (any-hit found, stack
-// empty, or the step bound reached).
 // Candidate-hit filter of the stroke-edge pass's visibility rays
 // (excludeFaceFilter, embree_renderer.cpp:76-133): a hit is not an occluder
 // when it lies on one of the segment's own mesh faces (primID modulo the base
@@ -438,6 +435,9 @@ UBR_D bool filterAccept(const HitFilter& f, const Ray& r, const Hit& h, uint32_t
 // memory and pass them as `top` (nTop of them).
 constexpr int kTopNodes = 73;
 
+// Visit st.node: test its 8 children, its hit leaves' primitives, choose the
+// next node.  Returns true when the ray is finished (any-hit found, stack
+// empty, or the step bound reached).
 //
 // CULL (closest hits of rays without a short range): a pushed group keeps the
 // key of its nearest child, which is visited next, and is dropped when the

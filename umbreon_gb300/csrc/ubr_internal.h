@@ -373,10 +373,7 @@ UBR_HD void segmentAxis(f3 p0, f3 p1, f3& a, float& L) {
   a = ax * (1.0f / L);
 }
 
-// Capped cone segment (CONE_LINEAR_CURVE): frustum + flat disks at p0, p1,
-// with its unit axis `a` and length L precomputed by segmentAxis.
-// ATTR = false (any-hit queries) returns at the first valid hit and uses the
-// fused forms (as isectSphere does).
+// An early way out of the capped cone test, true only where no hit is possible.
 // Most lines that enter a segment's box pass the segment by (a bond is thin
 // and lies across its box), and a full test of one that does costs a quadratic
 // and three divisions, so a conservative test goes first: the line misses the
@@ -395,6 +392,10 @@ UBR_HD bool missesAxis(const Ray& r, f3 p0, float rad, f3 a) {
   const float k = fmaf(rad, 1.001f, 1.0e-5f * w1);
   return s > 0.0f && s * s > k * k * fmaf(nx, nx, fmaf(ny, ny, nz * nz));
 }
+// Capped cone segment (CONE_LINEAR_CURVE): frustum + flat disks at p0, p1,
+// with its unit axis `a` and length L precomputed by segmentAxis.
+// ATTR = false (any-hit queries) returns at the first valid hit and uses the
+// fused forms (as isectSphere does).
 template <bool ATTR = true>
 UBR_HD bool isectConeCurveAxis(const Ray& r, f3 p0, float r0, f3 p1, float r1, f3 a, float L, float tnear,
                                float tmax, Hit& h) {
