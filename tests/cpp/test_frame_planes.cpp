@@ -48,6 +48,32 @@ int main() {
       check(out[i].ptr == in[i].ptr && out[i].bytes == in[i].bytes, "order and extents are kept");
     }
   }
+  // known ranges answer as the driver would, asked once per allocation: blocks
+  // of 64 to 191 bytes every 192 bytes from 4096 on, some of other memory
+  for (int round = 0; round < 2000; ++round) {
+    ubr::KnownRanges known;
+    const unsigned salt = rng();
+    int asked = 0;
+    std::vector<int> met(64, 0);
+    for (int k = 0; k < 60; ++k) {
+      const uintptr_t a = 4096 + rng() % (192 * 64);
+      const size_t bytes = rng() % 200, block = (a - 4096) / 192;
+      const uintptr_t start = 4096 + 192 * block;
+      const size_t size = 64 + (salt * (unsigned(block) + 7u) >> 5) % 128;
+      const bool ours = (salt >> (block % 32)) & 1u;
+      auto ask = [&](uintptr_t& s, size_t& n) {
+        ++asked;
+        check(++met[block] == 1 || !ours || a >= start + size, "asked once for an allocation");
+        s = start;
+        n = size;
+        return ours && a < start + size;
+      };
+      if (ours && a >= start + size) met[block] -= 1;  // between the allocations: asked again
+      const bool got = known(at(a), bytes, ask);
+      check(got == (ours && a < start + size && a + bytes <= start + size), "within one allocation of ours");
+    }
+    check(asked > 0, "the driver was asked");
+  }
   if (failures) std::printf("%d failures\n", failures);
   return failures ? 1 : 0;
 }

@@ -870,9 +870,10 @@ ubr_status adjoint(Context* c, const Scene* sc, const ubr_render_desc& d, const 
   // the caller's arrays get the packed sums spread over them at the end where
   // the device holds them whole; any others are cleared here and added to (the
   // clearing finds arrays it cannot write, with an error)
-  const bool spread = !dev || ((!gCol || deviceHolds(c->device, gCol, 3 * nSph * sizeof(float))) &&
-                               (!gCen || deviceHolds(c->device, gCen, 3 * nSph * sizeof(float))) &&
-                               (!gRad || deviceHolds(c->device, gRad, nSph * sizeof(float))));
+  DeviceMemory holds(c->device);
+  const bool spread = !dev || ((!gCol || holds(gCol, 3 * nSph * sizeof(float))) &&
+                               (!gCen || holds(gCen, 3 * nSph * sizeof(float))) &&
+                               (!gRad || holds(gRad, nSph * sizeof(float))));
   const size_t accBytes = spread && (gCol || gCen || gRad) ? size_t(nSph) * 32 : 0;
   const size_t accPad = (accBytes + kAdjAlign - 1) / kAdjAlign * kAdjAlign;
   size_t wsBytes = adjHeader(kAdjAlign) + std::min<size_t>(size_t(npix) * pixBytes, std::max(kAdjBytes, pixBytes));

@@ -33,7 +33,7 @@ ubr_status occludedFilteredBatch(Context* c, const Scene* sc, const float* segs,
 ubr_status occludedBatchNoAlloc(Context* c, const Scene* sc, const float* segs, uint64_t n, float eps,
                                 uint8_t* out);
 
-bool deviceHolds(int device, const void* ptr, size_t bytes) {
+bool deviceRange(int device, const void* ptr, uintptr_t& start, size_t& size) {
   // from the driver: the runtime's pointer attributes have no extent
   using Get = CUresult(CUDAAPI*)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
   static const Get get = [] {
@@ -52,13 +52,12 @@ bool deviceHolds(int device, const void* ptr, size_t bytes) {
                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
   unsigned int type = 0;
   int ordinal = -1;
-  CUdeviceptr start = 0;
-  size_t size = 0;
-  void* values[4] = {&type, &ordinal, &start, &size};
-  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(ptr);
-  if (get(4, what, values, at) != CUDA_SUCCESS) return false;
-  return type == CU_MEMORYTYPE_DEVICE && ordinal == device && at >= start && at - start <= size &&
-         bytes <= size - (at - start);
+  CUdeviceptr base = 0;
+  size = 0;
+  void* values[4] = {&type, &ordinal, &base, &size};
+  if (get(4, what, values, reinterpret_cast<CUdeviceptr>(ptr)) != CUDA_SUCCESS) return false;
+  start = uintptr_t(base);
+  return type == CU_MEMORYTYPE_DEVICE && ordinal == device;
 }
 
 }  // namespace ubr

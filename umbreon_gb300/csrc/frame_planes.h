@@ -46,4 +46,33 @@ void choosePlanes(std::vector<PlaneUse>& planes, Ours&& ours) {
   }
 }
 
+// Allocations that a call has met, so that planes of one allocation cost one
+// question to the driver (70 ns: 8 us of a batch of 24 frames with 120 planes).
+// Not kept between calls.
+class KnownRanges {
+ public:
+  // Whether [ptr, ptr + bytes) lies within one allocation; ask(start, size)
+  // finds the one at ptr, or is false.
+  template <class Ask>
+  bool operator()(const void* ptr, size_t bytes, Ask&& ask) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(ptr);
+    for (const Range& r : ranges_)
+      if (r.holds(at)) return r.holds(at, bytes);
+    Range r{};
+    if (!ask(r.start, r.size) || !r.holds(at)) return false;
+    ranges_.push_back(r);
+    return r.holds(at, bytes);
+  }
+
+ private:
+  struct Range {
+    uintptr_t start;
+    size_t size;
+    bool holds(uintptr_t at, size_t bytes = 0) const {
+      return at >= start && at - start < size && bytes <= size - (at - start);
+    }
+  };
+  std::vector<Range> ranges_;
+};
+
 }  // namespace ubr

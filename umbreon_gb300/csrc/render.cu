@@ -2759,7 +2759,7 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
     }
     if (b.aoPatch) u[11] = PlaneUse{fr.ao_patch_mask, fpix * 4, 0, false};
   }
-  choosePlanes(planes, [&](const void* q, size_t n) { return deviceHolds(c->device, q, n); });
+  choosePlanes(planes, DeviceMemory(c->device));
   for (size_t f = 0; f < nf; ++f) {
     const ubr_frame& fr = *jobs[f].frame;
     const PlaneUse* u = &planes[f * kPlanes];

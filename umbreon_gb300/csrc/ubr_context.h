@@ -8,6 +8,7 @@
 #include <utility>
 #include <vector>
 
+#include "frame_planes.h"
 #include "gi.cuh"
 #include "ubr_internal.h"
 
@@ -130,10 +131,21 @@ T* scratchT(Context* c, int slot, size_t count, ubr_status& st) {
   return static_cast<T*>(ptr);
 }
 
-// Whether [ptr, ptr + bytes) lies within one allocation on `device`.  Kernels
+// The allocation on `device` that holds the address, as the driver knows it;
+// false for other memory.
+bool deviceRange(int device, const void* ptr, uintptr_t& start, size_t& size);
+// Whether [ptr, ptr + bytes) lies within one allocation on the device.  Kernels
 // write a caller's memory only where this holds: a copy or memset checks what
-// it is given and fails with an error, a kernel's store faults.
-bool deviceHolds(int device, const void* ptr, size_t bytes);
+// it is given and fails with an error, a kernel's store faults.  One object per
+// call: it asks the driver once per allocation.
+struct DeviceMemory {
+  explicit DeviceMemory(int device) : device(device) {}
+  bool operator()(const void* ptr, size_t bytes) {
+    return known(ptr, bytes, [&](uintptr_t& start, size_t& size) { return deviceRange(device, ptr, start, size); });
+  }
+  int device;
+  KnownRanges known;
+};
 
 // Frame parameters and light table of a render description (camera basis,
 // lights, AO / fog / gamma settings), validated.
