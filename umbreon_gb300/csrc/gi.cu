@@ -436,10 +436,10 @@ UBR_D uint32_t tilePixel4(uint32_t i, uint32_t W, uint32_t H) {
 // defaults (20 k ball-and-stick, 1920x1080 ss2: 12.1 M gather rays, 5.1 M
 // shadow rays) the gather and the edge patch take 24.8 -> 12.1 ms, on the 2 k
 // sphere 640x480 frame (8 samples per pixel) 0.57 -> 0.40 ms, with the same
-// frames bit for bit.  What bounds it now: k_gather_first is three quarters,
-// 74 % of its issue slots with 8.7 of 32 lanes (rays of one hemisphere fan end
-// at different depths); at most 64 registers (6 or 7 blocks per SM are 1-2 %
-// slower, 10 2.5 %).
+// frames bit for bit.  What bounds it now: k_gather_first is 55 % of the pt2
+// default frame, with 67 % of its issue slots used and 13 of 32 lanes per
+// instruction (rays of one hemisphere fan end at different depths); at most 64
+// registers (6 or 7 blocks per SM are 1-2 % slower, 10 2.5 %).
 
 // Workspace of a chunk.  A sample has a slot: LANES neighbouring slots hold
 // one point's consecutive samples, 32 slots (a warp) the same LANES samples

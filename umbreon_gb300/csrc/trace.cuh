@@ -1,6 +1,10 @@
 // trace.cuh -- device building blocks shared by the frame kernels and the
 // adjoint: primary rays, 8-wide BVH traversal, shading surface, sample
 // streams (tea2, cosine hemisphere, low-discrepancy AO), warp counters.
+//
+// Two times beside the code, here and in the files that include it, are those
+// of the change they stand at, measured against the code right before it; the
+// times of different changes do not chain.
 #pragma once
 
 #include "ubr_context.h"
