@@ -84,8 +84,9 @@ __host__ __device__ constexpr int lowKind(int km) { return (km & 1) ? 0 : (km & 
 __host__ __device__ constexpr int highKind(int km) { return (km & 8) ? 3 : (km & 4) ? 2 : (km & 2) ? 1 : 0; }
 
 // Test of the primitive in leaf slot `slot` whose kind is known; a round
-// segment needs its reference (`ref`, or kInvalid to load it).
-template <int KIND, bool ATTR>
+// segment needs its reference (`ref`, or kInvalid to load it).  ALONE: as
+// isectTriangle's.
+template <int KIND, bool ATTR, bool ALONE = false>
 UBR_D bool testKnown(const TravScene& s, int slot, const Ray& r, const TriPre& pre, float tnear, float tmax,
                      Hit& h, uint32_t ref) {
   const float4* g = s.leafGeo + kLeafF4 * slot;
@@ -94,7 +95,7 @@ UBR_D bool testKnown(const TravScene& s, int slot, const Ray& r, const TriPre& p
     return isectSphere<ATTR>(r, f3{q.x, q.y, q.z}, q.w, tnear, tmax, h);
   }
   if (KIND == kMesh) {
-    if (!isectTriangle(pre, __ldg(g + pre.kx), __ldg(g + pre.ky), __ldg(g + pre.kz), tnear, tmax, h)) return false;
+    if (!isectTriangle<ALONE>(pre, __ldg(g + pre.kx), __ldg(g + pre.ky), __ldg(g + pre.kz), tnear, tmax, h)) return false;
     if (ATTR) {
       const float4 x = __ldg(g), y = __ldg(g + 1), z = __ldg(g + 2);
       const f3 v0{x.x, y.x, z.x};
@@ -121,7 +122,7 @@ UBR_D bool testLeaf(const TravScene& s, int slot, const Ray& r, const TriPre& pr
   const int kind = refKind(ref);
   constexpr bool single = (KM & (KM - 1)) == 0;
   if ((KM & kMaskSphere) && (single || kind == kSphere)) return testKnown<kSphere, ATTR>(s, slot, r, pre, tnear, tmax, h, ref);
-  if ((KM & kMaskMesh) && (single || kind == kMesh)) return testKnown<kMesh, ATTR>(s, slot, r, pre, tnear, tmax, h, ref);
+  if ((KM & kMaskMesh) && (single || kind == kMesh)) return testKnown<kMesh, ATTR, single>(s, slot, r, pre, tnear, tmax, h, ref);
   if ((KM & kMaskCone) && (!(KM & kMaskRound) || kind == kCone))
     return testKnown<kCone, ATTR>(s, slot, r, pre, tnear, tmax, h, ref);
   if (KM & kMaskRound) return testKnown<kRound, ATTR>(s, slot, r, pre, tnear, tmax, h, ref);

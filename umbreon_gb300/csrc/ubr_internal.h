@@ -247,6 +247,14 @@ UBR_HD TriPre triPre(f3 d, f3 org) {
 // AO 32, 17.35 -> 14.40 ms, enhanced AO on a surface 2.10 -> 1.82 ms, 2*10^5
 // filtered segments 0.178 -> 0.149 ms.  On a hit h gets t, u, v; Ng is left to
 // the caller.
+// ALONE: for the tests of a kernel without other kinds, where the compiler
+// moved the redo's conversions out of its block and every test paid for them
+// on the slow double-precision pipe; a loop of its own keeps them in it.
+// Surface of 800 atoms alone, 800x600: primary rays 218 -> 115 us, enhanced AO
+// 16 4.03 -> 1.33 ms, pt2 gather 2.04 -> 1.09 ms, 2*10^5 filtered segments 351
+// -> 150 us.  With other kinds the block stays in place, and the loop costs
+// 1.5 % of an AOV frame.
+template <bool ALONE = false>
 UBR_HD bool isectTriangle(const TriPre& pre, const float4& X, const float4& Y, const float4& Z, float tnear,
                           float tmax, Hit& h) {
   const float A_z = Z.x - pre.org.z, B_z = Z.y - pre.org.z, C_z = Z.z - pre.org.z;
@@ -260,9 +268,30 @@ UBR_HD bool isectTriangle(const TriPre& pre, const float4& X, const float4& Y, c
   float V = Ax * Cy - Ay * Cx;
   float W = Bx * Ay - By * Ax;
   if (U == 0.0f || V == 0.0f || W == 0.0f) {
-    U = float(double(Cx) * By - double(Cy) * Bx);
-    V = float(double(Ax) * Cy - double(Ay) * Cx);
-    W = float(double(Bx) * Ay - double(By) * Ax);
+    if (ALONE) {
+      float px = Cx, py = Cy, qx = Bx, qy = By, ox = Ax, oy = Ay;
+      int n = 3;
+#ifdef __CUDA_ARCH__
+      asm volatile("" : "+r"(n));
+#endif
+#pragma unroll 1
+      for (; n > 0; --n) {  // C x B, A x C, B x A in turn
+        const float e = float(double(px) * qy - double(py) * qx), tx = ox, ty = oy;
+        ox = qx;
+        oy = qy;
+        qx = px;
+        qy = py;
+        px = tx;
+        py = ty;
+        U = V;
+        V = W;
+        W = e;
+      }
+    } else {
+      U = float(double(Cx) * By - double(Cy) * Bx);
+      V = float(double(Ax) * Cy - double(Ay) * Cx);
+      W = float(double(Bx) * Ay - double(By) * Ax);
+    }
   }
   if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return false;
   const float det = U + V + W;
