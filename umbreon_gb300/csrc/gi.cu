@@ -869,37 +869,112 @@ __global__ void __launch_bounds__(128) k_gather_emit(GiP g, DScene s, GiGrid gri
   warpCount(g.overflow, ovf);
 }
 
-// The samples of a point summed (each lane its own in order, the lanes in a
-// shuffle tree) into E = (mean radiance, share of first bounces that hit or
-// fell below the horizon); halfE gets the sum of the first spp/2.  ReSTIR (one
-// lane per point): every sample is also one candidate streamed, in sample
-// order, into the point's reservoir (pt1_gather.hpp:287-297, 451-499).
-__global__ void __launch_bounds__(128) k_gather_sum(GiP g, GiGrid grid, const uint32_t* list, GiWave w, float4* E) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t group = t >> 5, lane = t & 31u, iters = uint32_t(w.iters);
-  const bool on = group * iters * 32u < waveSlots(w);
+// The samples of a point summed by a lane, in order: radiance, the sum of the
+// first spp/2, the number of first bounces that hit or fell below the horizon,
+// and (ReSTIR, one lane per point) the reservoir that every sample's candidate
+// is streamed into (pt1_gather.hpp:287-297, 451-499).
+struct PointSum {
   f3 e{0.0f, 0.0f, 0.0f}, half{0.0f, 0.0f, 0.0f};
   float occ = 0.0f;
-  uint32_t point = 0, pix = 0;
-  bool own = false;
   uint32_t rs0 = 0, rs1 = 0x47490001u;
   double rWSum = 0.0;
   f3 rPos{0.0f, 0.0f, 0.0f}, rNrm{0.0f, 0.0f, 0.0f}, rRad{0.0f, 0.0f, 0.0f};
   float rPHat = 0.0f;
+};
+// L: a sample's radiance, and 1 for such a first bounce
+UBR_D void clampSample(const GiP& g, float4& L) {
+  if (g.clampLum > 0.0f) {
+    const float lum = 0.2126f * L.x + 0.7152f * L.y + 0.0722f * L.z;
+    if (lum > g.clampLum) {
+      const float k = g.clampLum / lum;
+      L.x *= k;
+      L.y *= k;
+      L.z *= k;
+    }
+  }
+}
+UBR_D void addSample(PointSum& p, const float4& L, int sI, int spp) {
+  p.e.x += L.x;
+  p.e.y += L.y;
+  p.e.z += L.z;
+  p.occ += L.w;
+  if (sI < spp / 2) {
+    p.half.x += L.x;
+    p.half.y += L.y;
+    p.half.z += L.z;
+  }
+}
+// Candidate (position, normal, cosine at the origin, not above 0: none) of a
+// sample: RIS weight pi * lum(L), p_hat = lum(L) cos over the cosine pdf.
+UBR_D void addCandidate(PointSum& p, const float4& L, f3 pos, f3 nrm, float cosine) {
+  float wgt = 0.0f, pHat = 0.0f;
+  if (cosine > 0.0f) {
+    pHat = lumOf(L.x, L.y, L.z) * cosine;
+    wgt = lumOf(L.x, L.y, L.z) * kPiF;
+  }
+  tea2(p.rs0, p.rs1);
+  p.rWSum += double(wgt);
+  if (wgt > 0.0f && double(u32ToUnorm(p.rs0)) * p.rWSum <= double(wgt)) {
+    p.rPos = pos;
+    p.rNrm = nrm;
+    p.rRad = ld3(L);
+    p.rPHat = pHat;
+  }
+}
+UBR_D uint32_t reservoirStream(const GiP& g, uint32_t pix) { return hashU32(pix ^ g.seedMix) ^ 0x52455354u; }
+// The lanes of a point in a shuffle tree (all lanes of the warp), and its
+// results by the first of them: E = (mean radiance, share of such first
+// bounces), halfE = the sum of the first spp/2, the reservoir.
+UBR_D void writePoint(const GiP& g, PointSum& p, bool own, uint32_t lane, int lanes, uint32_t pix, int spp, bool restir,
+                      float4* E) {
+  for (int o = lanes / 2; o > 0; o >>= 1) {
+    p.e.x += __shfl_xor_sync(0xFFFFFFFFu, p.e.x, o);
+    p.e.y += __shfl_xor_sync(0xFFFFFFFFu, p.e.y, o);
+    p.e.z += __shfl_xor_sync(0xFFFFFFFFu, p.e.z, o);
+    p.occ += __shfl_xor_sync(0xFFFFFFFFu, p.occ, o);
+    p.half.x += __shfl_xor_sync(0xFFFFFFFFu, p.half.x, o);
+    p.half.y += __shfl_xor_sync(0xFFFFFFFFu, p.half.y, o);
+    p.half.z += __shfl_xor_sync(0xFFFFFFFFu, p.half.z, o);
+  }
+  if (!own || (lane & uint32_t(lanes - 1)) != 0u) return;
+  const float invN = 1.0f / float(spp > 0 ? spp : 1);
+  E[pix] = make_float4(p.e.x * invN, p.e.y * invN, p.e.z * invN, p.occ * invN);
+  if (g.halfE) {
+    g.halfE[3 * size_t(pix)] = p.half.x;
+    g.halfE[3 * size_t(pix) + 1] = p.half.y;
+    g.halfE[3 * size_t(pix) + 2] = p.half.z;
+  }
+  if (restir) {  // W = wSum / (M p_hat(selected)), M = every candidate
+    float4* rsv = g.rsv + size_t(kRsvF4) * pix;
+    const float M = float(spp > 0 ? spp : 1);
+    const float W = (p.rPHat > 0.0f && p.rWSum > 0.0) ? float(p.rWSum / (double(M) * double(p.rPHat))) : 0.0f;
+    rsv[0] = make_float4(p.rPos.x, p.rPos.y, p.rPos.z, M);
+    rsv[1] = make_float4(p.rNrm.x, p.rNrm.y, p.rNrm.z, W);
+    rsv[2] = make_float4(p.rRad.x, p.rRad.y, p.rRad.z, 0.0f);
+  }
+}
+
+__global__ void __launch_bounds__(128) k_gather_sum(GiP g, GiGrid grid, const uint32_t* list, GiWave w, float4* E) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t group = t >> 5, lane = t & 31u, iters = uint32_t(w.iters);
+  const bool on = group * iters * 32u < waveSlots(w);
+  PointSum p;
+  uint32_t point = 0, pix = 0;
+  bool own = false;
   if (on && w.it0 > 0) {
     const float4* c = w.carry + size_t(kCarryF4) * t;
-    e = ld3(c[0]);
-    occ = c[0].w;
-    half = ld3(c[1]);
-    rPos = ld3(c[2]);
-    rPHat = c[2].w;
-    rNrm = ld3(c[3]);
-    rRad = ld3(c[4]);
-    rWSum = __hiloint2double(__float_as_int(c[5].y), __float_as_int(c[5].x));
+    p.e = ld3(c[0]);
+    p.occ = c[0].w;
+    p.half = ld3(c[1]);
+    p.rPos = ld3(c[2]);
+    p.rPHat = c[2].w;
+    p.rNrm = ld3(c[3]);
+    p.rRad = ld3(c[4]);
+    p.rWSum = __hiloint2double(__float_as_int(c[5].y), __float_as_int(c[5].x));
     own = c[1].w != 0.0f;
     pix = own ? __float_as_uint(c[3].w) : 0u;
-    rs0 = __float_as_uint(c[4].w);
-    rs1 = __float_as_uint(c[5].z);
+    p.rs0 = __float_as_uint(c[4].w);
+    p.rs1 = __float_as_uint(c[5].z);
   }
   for (uint32_t it = 0; on && it < iters; ++it) {
     const uint32_t slot = (group * iters + it) * 32u + lane;
@@ -908,83 +983,145 @@ __global__ void __launch_bounds__(128) k_gather_sum(GiP g, GiGrid grid, const ui
     if (!own) {
       own = true;
       pix = list[point];
-      rs0 = hashU32(pix ^ g.seedMix) ^ 0x52455354u;
+      p.rs0 = reservoirStream(g, pix);
     }
     float4 L = w.L[slot];
-    if (g.clampLum > 0.0f) {
-      const float lum = 0.2126f * L.x + 0.7152f * L.y + 0.0722f * L.z;
-      if (lum > g.clampLum) {
-        const float k = g.clampLum / lum;
-        L.x *= k;
-        L.y *= k;
-        L.z *= k;
-      }
-    }
-    if (w.cand) {  // RIS weight pi * lum(L): p_hat = lum(L) cos over the cosine pdf
+    clampSample(g, L);
+    if (w.cand) {
       const float4 c0 = w.cand[2 * size_t(slot)], c1 = w.cand[2 * size_t(slot) + 1];
-      float wgt = 0.0f, pHat = 0.0f;
-      if (c1.w > 0.0f) {
-        pHat = lumOf(L.x, L.y, L.z) * c1.w;
-        wgt = lumOf(L.x, L.y, L.z) * kPiF;
-      }
-      tea2(rs0, rs1);
-      rWSum += double(wgt);
-      if (wgt > 0.0f && double(u32ToUnorm(rs0)) * rWSum <= double(wgt)) {
-        rPos = ld3(c0);
-        rNrm = ld3(c1);
-        rRad = ld3(L);
-        rPHat = pHat;
-      }
+      addCandidate(p, L, ld3(c0), ld3(c1), c1.w);
     }
-    e.x += L.x;
-    e.y += L.y;
-    e.z += L.z;
-    occ += L.w;
-    if (sI < w.spp / 2) {
-      half.x += L.x;
-      half.y += L.y;
-      half.z += L.z;
-    }
+    addSample(p, L, sI, w.spp);
   }
   if (w.it0 + w.iters < w.itEnd) {
     if (!on) return;
     float4* c = w.carry + size_t(kCarryF4) * t;
-    c[0] = make_float4(e.x, e.y, e.z, occ);
-    c[1] = make_float4(half.x, half.y, half.z, own ? 1.0f : 0.0f);
-    c[2] = make_float4(rPos.x, rPos.y, rPos.z, rPHat);
-    c[3] = make_float4(rNrm.x, rNrm.y, rNrm.z, __uint_as_float(pix));
-    c[4] = make_float4(rRad.x, rRad.y, rRad.z, __uint_as_float(rs0));
-    c[5] = make_float4(__int_as_float(__double2loint(rWSum)), __int_as_float(__double2hiint(rWSum)),
-                       __uint_as_float(rs1), 0.0f);
+    c[0] = make_float4(p.e.x, p.e.y, p.e.z, p.occ);
+    c[1] = make_float4(p.half.x, p.half.y, p.half.z, own ? 1.0f : 0.0f);
+    c[2] = make_float4(p.rPos.x, p.rPos.y, p.rPos.z, p.rPHat);
+    c[3] = make_float4(p.rNrm.x, p.rNrm.y, p.rNrm.z, __uint_as_float(pix));
+    c[4] = make_float4(p.rRad.x, p.rRad.y, p.rRad.z, __uint_as_float(p.rs0));
+    c[5] = make_float4(__int_as_float(__double2loint(p.rWSum)), __int_as_float(__double2hiint(p.rWSum)),
+                       __uint_as_float(p.rs1), 0.0f);
     return;
   }
-  const int lanes = 1 << w.logLanes;
-  for (int o = lanes / 2; o > 0; o >>= 1) {
-    e.x += __shfl_xor_sync(0xFFFFFFFFu, e.x, o);
-    e.y += __shfl_xor_sync(0xFFFFFFFFu, e.y, o);
-    e.z += __shfl_xor_sync(0xFFFFFFFFu, e.z, o);
-    occ += __shfl_xor_sync(0xFFFFFFFFu, occ, o);
-    half.x += __shfl_xor_sync(0xFFFFFFFFu, half.x, o);
-    half.y += __shfl_xor_sync(0xFFFFFFFFu, half.y, o);
-    half.z += __shfl_xor_sync(0xFFFFFFFFu, half.z, o);
-  }
   // lane 0 of a point has its first sample: it always owns one
-  if (!own || (lane & uint32_t(lanes - 1)) != 0u) return;
-  const float invN = 1.0f / float(w.spp > 0 ? w.spp : 1);
-  E[pix] = make_float4(e.x * invN, e.y * invN, e.z * invN, occ * invN);
-  if (g.halfE) {
-    g.halfE[3 * size_t(pix)] = half.x;
-    g.halfE[3 * size_t(pix) + 1] = half.y;
-    g.halfE[3 * size_t(pix) + 2] = half.z;
+  writePoint(g, p, own, lane, 1 << w.logLanes, pix, w.spp, w.cand != nullptr, E);
+}
+
+// One sample's path from its draw to its last shadow ray: radiance, and 1 when
+// the first bounce hit something or fell below the horizon; its ReSTIR candidate
+// (cosine -1: none).
+template <int KM>
+UBR_D float4 gatherPath(const GiP& g, const DScene& s, const LightD* lights, int nLights, const GatherOrigin& o, f3 wi,
+                        int sI, f3& candPos, f3& candN, float& candCos, uint32_t& rays, uint32_t& nee, uint32_t& ovf) {
+  const int maxB = g.bounces < 1 ? 1 : g.bounces;
+  const bool emitNee = g.pt2 && g.em.n > 0;
+  const TravScene ts = travOf(s);
+  uint32_t s0 = o.seed, s1 = uint32_t(sI + g.sampleOffset);
+  tea2(s0, s1);
+  const bool horizonOk = dot(wi, o.Ng) > 0.0f;
+  const float cos0 = dot(wi, o.N);
+  f3 org = o.O, thr{1.0f, 1.0f, 1.0f}, L{0.0f, 0.0f, 0.0f};
+  float tnear = o.eps, occ = horizonOk ? 0.0f : 1.0f;
+  candPos = f3{0.0f, 0.0f, 0.0f};
+  candN = neg(wi);
+  candCos = horizonOk ? cos0 : -1.0f;
+  for (int bnc = 1; horizonOk && bnc <= maxB; ++bnc) {
+    Hit h;
+    traverse<false, KM, false, false, true>(ts, Ray{org, wi, tnear, g.maxDist}, h, ovf, nullptr, false);
+    ++rays;
+    if (h.ref == kInvalid) {
+      const f3 env = giEnvironment(g, wi);
+      L.x += thr.x * env.x;
+      L.y += thr.y * env.y;
+      L.z += thr.z * env.z;
+      // escaped: the candidate sits 1e7 along the segment
+      if (bnc == 1) candPos = f3{o.O.x + wi.x * 1.0e7f, o.O.y + wi.y * 1.0e7f, o.O.z + wi.z * 1.0e7f};
+      break;
+    }
+    if (bnc == 1) occ = 1.0f;
+    Vertex v;
+    if (!evalVertex<KM>(s, lights, nLights, h, org, wi, g.pt2 && g.emissive, g.pt2 ? &s0 : nullptr,
+                        g.pt2 ? &s1 : nullptr, v, nee, ovf)) {
+      // absorbed by an outline: a zero-radiance candidate at the hit
+      if (bnc == 1) candPos = f3{org.x + wi.x * h.t, org.y + wi.y * h.t, org.z + wi.z * h.t};
+      break;
+    }
+    if (bnc == 1) {
+      candPos = v.P;
+      candN = v.N;
+    }
+    float emW = 1.0f;
+    if (emitNee && bnc == 1) emW = emissiveHitWeight(g.em, refKind(h.ref), refPrim(h.ref), org, wi, h.t, cos0, h.Ng);
+    L.x += thr.x * (v.rad.x + emW * v.emitted.x);
+    L.y += thr.y * (v.rad.y + emW * v.emitted.y);
+    L.z += thr.z * (v.rad.z + emW * v.emitted.z);
+    if (bnc == maxB) break;
+    thr.x *= v.alb.x;
+    thr.y *= v.alb.y;
+    thr.z *= v.alb.z;
+    if (bnc >= 2) {
+      tea2(s0, s1);
+      float pc = fmaxf(thr.x, fmaxf(thr.y, thr.z));
+      pc = fminf(0.95f, fmaxf(0.05f, pc));
+      if (u32ToUnorm(s0) >= pc) break;
+      const float inv = 1.0f / pc;
+      thr.x *= inv;
+      thr.y *= inv;
+      thr.z *= inv;
+    }
+    tea2(s0, s1);
+    wi = cosineSampleHemisphere(u32ToUnorm(s0), u32ToUnorm(s1), frameFromNormal(v.N));
+    tnear = selfIntersectEps(v.P, wi, h.t);
+    org = f3{v.P.x + v.N.x * tnear, v.P.y + v.N.y * tnear, v.P.z + v.N.z * tnear};
   }
-  if (w.cand) {  // W = wSum / (M p_hat(selected)), M = every candidate
-    float4* rsv = g.rsv + size_t(kRsvF4) * pix;
-    const float M = float(w.spp > 0 ? w.spp : 1);
-    const float W = (rPHat > 0.0f && rWSum > 0.0) ? float(rWSum / (double(M) * double(rPHat))) : 0.0f;
-    rsv[0] = make_float4(rPos.x, rPos.y, rPos.z, M);
-    rsv[1] = make_float4(rNrm.x, rNrm.y, rNrm.z, W);
-    rsv[2] = make_float4(rRad.x, rRad.y, rRad.z, 0.0f);
+  if (emitNee) {
+    const f3 e = emissiveNee<KM>(g.em, s, o.P, o.N, o.Ng, o.tEps, s0, s1, ovf);
+    ++nee;
+    L.x += e.x;
+    L.y += e.y;
+    L.z += e.z;
   }
+  return make_float4(L.x, L.y, L.z, occ);
+}
+
+// The gather in one kernel, a lane walking its samples' paths one after the
+// other, for few samples (giGatherWhole).  Over n points of a grid (list null;
+// points that are not eligible get 0) or the first *listCount of a list of n.
+template <int KM>
+__global__ void __launch_bounds__(128, 8) k_gather_whole(GiP g, DScene s, const LightD* lights, int nLights, GiGrid grid,
+                                                         const uint32_t* list, const uint32_t* listCount, uint32_t n,
+                                                         int spp, int logLanes, float4* E) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = t >> logLanes;
+  const int lanes = 1 << logLanes;
+  const bool own = i < (listCount ? min(n, *listCount) : n);
+  uint32_t rays = 0, nee = 0, ovf = 0, pix = 0;
+  bool eligible = false;
+  PointSum p;
+  if (own) {
+    pix = list            ? list[i]
+          : logLanes == 0 ? tilePixel4(i, uint32_t(grid.W), uint32_t(grid.H))
+                          : quadPixel(i, uint32_t(grid.W), uint32_t(grid.H));
+    eligible = grid.ne[pix].w != 0.0f;
+  }
+  if (eligible) {
+    const GatherOrigin o = gatherOrigin(g, grid, pix);
+    p.rs0 = reservoirStream(g, pix);
+    for (int sI = int(t) & (lanes - 1); sI < spp; sI += lanes) {
+      f3 candPos, candN;
+      float candCos;
+      float4 L = gatherPath<KM>(g, s, lights, nLights, o, gatherDirection(g, grid, o, pix, spp, sI), sI, candPos, candN,
+                                candCos, rays, nee, ovf);
+      clampSample(g, L);
+      if (g.rsv) addCandidate(p, L, candPos, candN, candCos);
+      addSample(p, L, sI, spp);
+    }
+  }
+  writePoint(g, p, own, t, lanes, pix, spp, g.rsv && eligible, E);
+  warpCount(&g.stats[0], rays);
+  warpCount(&g.stats[1], nee);
+  warpCount(g.overflow, ovf);
 }
 
 // tracePt1GBuffer (pt1_gbuffer.hpp:83-196): one primary ray per point of a
@@ -1866,12 +2003,37 @@ static size_t waveAlign(size_t wsBytes, size_t slotBytes) {
 // a workspace of the size of a frame's own buffers (0.3 GB with two lights):
 // 2^20 slots are 8 % slower on the pt2 default frame, 2^24 1.5 % faster.
 constexpr uint64_t kWaveSlots = 1u << 22;
+// Samples of eligible points up to which the gather runs in one kernel: the
+// wavefront's six launches (four more per bounce, and the list and its count
+// first) are 80 to 200 us whatever they hold, one kernel 40 to 150.  Both sides
+// at 8 samples a point, wavefront / one kernel: 2 k spheres 57 k samples 91 / 57
+// us, 138 k 109 / 77, 354 k 159 / 149, 707 k 239 / 264; a surface with spheres
+// 51 k 172 / 141, 124 k 183 / 170, 317 k 268 / 319; 20 k ball-and-stick, whose
+// wavefront postpones its tests, 20 k 194 / 188, 49 k 195 / 211, 126 k 241 / 322.
+// Three bounces and more are worth twice that (4 bounces, ball-and-stick 77 k
+// 686 / 531, spheres 544 k 404 / 355).
+static uint64_t wholeSamples(int km, const GiP& g) {
+  const uint64_t one = km == kMaskSphere ? 1u << 18 : postponesTests(km) ? 1u << 15 : 1u << 17;
+  return g.bounces > 2 ? 2 * one : one;
+}
 constexpr size_t kWaveBytes = size_t(1) << 30;
 
 // Warps of slots that follow one another per group of points.
 static uint64_t gatherIters(const GiP& g, int spp) {
   const int lg = gatherLogLanes(g, spp);
   return (uint64_t(std::max(spp, 1)) + (1u << lg) - 1) >> lg;
+}
+
+// Not where a lane walks more than a few paths one after the other (32 samples a
+// point: 57 k 90 / 149, 553 k 196 / 266).
+static bool shortLanes(const GiP& g, int spp) { return spp <= 8 && gatherIters(g, spp) <= 2; }
+
+// Points that may be eligible count half where the rule is strict: molecules
+// cover a fifth to a half of their frames.  A few points need no workspace,
+// whatever an arena cap leaves.
+bool giGatherWhole(int km, const GiP& g, uint64_t n, int spp) {
+  const uint64_t samples = n * uint64_t(std::max(spp, 1));
+  return samples <= 1024 || (shortLanes(g, spp) && samples <= wholeSamples(km, g) * (postponesTests(km) ? 2 : 1));
 }
 
 size_t giGatherBytes(const GiP& g, int nLights, bool area, uint64_t n, int spp) {
@@ -1893,10 +2055,20 @@ cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, con
                      float4* E, uint32_t* listBuf, void* ws, size_t wsBytes, uint32_t* hostCount,
                      uint32_t* launches) {
   if (n == 0) return cudaSuccess;
+  const int logLanes = gatherLogLanes(g, spp);
+  auto whole = [&](const uint32_t* pts, const uint32_t* ptsCount, uint32_t points) {
+    byKind(km, [&](auto K) {
+      k_gather_whole<decltype(K)::value><<<blocks(uint64_t(points) << logLanes, 128), 128, 0, s>>>(
+          g, sc, lights, nLights, grid, pts, ptsCount, points, spp, logLanes, E);
+    });
+    ++*launches;
+    return cudaGetLastError();
+  };
+  if (giGatherWhole(km, g, n, spp)) return whole(list, listCount, n);
   GiWave w{};
   w.ctr = static_cast<uint32_t*>(ws);
   w.spp = std::max(spp, 0);
-  w.logLanes = gatherLogLanes(g, spp);
+  w.logLanes = logLanes;
   const uint32_t P = 32u >> w.logLanes;
   w.itEnd = int(gatherIters(g, spp));
   const size_t sb = gatherSlotBytes(g, nLights, area), align = waveAlign(wsBytes, sb);
@@ -1921,15 +2093,14 @@ cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, con
     pts = listBuf;
   }
   if (e != cudaSuccess) return e;
-  // more than one chunk of the listed points at most: read how many there are
-  uint32_t count = n;
-  if ((uint64_t(n) + P - 1) / P > groupsFit || w.iters < w.itEnd) {
-    e = cudaMemcpyAsync(hostCount, w.ctr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return e;
-    count = std::min(n, *hostCount);
-    if (count == 0) return cudaGetLastError();
-  }
+  // how many points there are: a launch for slots that hold none takes 1.2 ns a
+  // block, and the wavefront has several per bounce
+  e = cudaMemcpyAsync(hostCount, w.ctr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return e;
+  const uint32_t count = std::min(n, *hostCount);
+  if (count == 0) return cudaGetLastError();
+  if (shortLanes(g, spp) && uint64_t(count) * uint64_t(w.spp) <= wholeSamples(km, g)) return whole(pts, w.ctr, count);
   const uint64_t groups = (uint64_t(count) + P - 1) / P;
   const uint64_t chunks = (groups + groupsFit - 1) / groupsFit;
   const uint64_t perChunk = (groups + chunks - 1) / chunks;  // equal chunks: no short last one

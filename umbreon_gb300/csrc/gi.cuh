@@ -99,10 +99,12 @@ void giGBuffer(int km, cudaStream_t s, const Params& p, const DScene& sc, int w,
                float4* ng, unsigned long long* stats, unsigned long long* overflow);
 // The gather over a grid (list null: its eligible points, listed in listBuf of
 // n; the others get E = 0) or over the points of a list (listCount of them, on
-// the device).  Runs in chunks that fit the workspace ws of wsBytes, at least
-// giGatherLeast; giGatherBytes is what n points use well.  Reads the number
-// of points back (hostCount, pinned) when they may need more than one chunk.
+// the device).  Where giGatherWhole holds for n, in one kernel and without a
+// workspace; else the number of points is read back (hostCount, pinned), and
+// more of them run as a wavefront in chunks that fit the workspace ws of
+// wsBytes, at least giGatherLeast; giGatherBytes is what n points use well.
 // area: some light's shadow rays are jittered (pt2, radius > 0).
+bool giGatherWhole(int km, const GiP& g, uint64_t n, int spp);
 size_t giGatherLeast(const GiP& g, int nLights, bool area, int spp);
 size_t giGatherBytes(const GiP& g, int nLights, bool area, uint64_t n, int spp);
 cudaError_t giGather(int km, cudaStream_t s, const GiP& g, const DScene& sc, const LightD* lights, int nLights,

@@ -2361,7 +2361,8 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
       est.bounces = d0.gi_bounces;
       est.pt2 = d0.gi_integrator == 2;
       if (est.pt2 && d0.pt2_emissive && d0.pt2_emissive_nee) est.em = jobs[0].scene->emit;
-      plan.push_back({kGatherSlot, giGatherBytes(est, p1.nLights, false, nlo, d0.pt1_spp), false});
+      if (!giGatherWhole(km, est, nlo, d0.pt1_spp))
+        plan.push_back({kGatherSlot, giGatherBytes(est, p1.nLights, false, nlo, d0.pt1_spp), false});
     }
     scratchReserve(c, plan);
   }
@@ -2978,9 +2979,11 @@ ubr_status runFrames(Context* c, const std::vector<Job>& jobs, ubr_frame* total,
       // grid, about what edges and noise take, and more chunks past that)
       size_t bytes = giGatherBytes(gg, nL, area, list ? n / 16 + 32 : n, nspp);
       void* ws = nullptr;
-      const ubr_status wst = workspaceGet(c, kGatherSlot, giGatherLeast(gg, nL, area, nspp), b.hitA,
-                                          size_t(nslot) * sizeof(float4), &ws, &bytes);
-      if (wst != UBR_OK) return wst;
+      if (!giGatherWhole(km, gg, n, nspp)) {
+        const ubr_status wst = workspaceGet(c, kGatherSlot, giGatherLeast(gg, nL, area, nspp), b.hitA,
+                                            size_t(nslot) * sizeof(float4), &ws, &bytes);
+        if (wst != UBR_OK) return wst;
+      }
       // the eligible points of a grid are listed in the first queue buffer
       UBR_CUDA(c, giGather(km, s, gg, s1, lt, nL, area, gr, list, cnt, n, nspp, E, q0, ws, bytes, hostCount + 8, &kernels));
       scratchDone(c, kGatherSlot);
