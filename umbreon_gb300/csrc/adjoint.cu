@@ -16,7 +16,7 @@
 //                   shadeLocal (shading.hpp:76-192), the AO estimators
 //                   (ambient_occlusion.hpp:33-57, 171-267) and the sphere hit
 //                   (t, P, N, self-intersection epsilon)
-// and k_adj_background for the rest.  When the assumed gamma is not 1, a
+// and, in k_adj_surface, the background.  When the assumed gamma is not 1, a
 // forward pass of k_adj_shade over the same rays and k_adj_down give the
 // downsampled value the gamma derivative needs.
 // Visibility (which sphere a ray hits, each shadow bit, each AO sample's
@@ -70,7 +70,7 @@ struct AdjBufs {
   float* gRadius;           // per input sphere
   float4* acc;              // per input sphere: (centre, radius) (colour, -) sums, or null: the arrays above
   double* gGlobal;          // kGlobals
-  unsigned long long* stats;  // 0 samples, 1 rays, 2 overflow
+  unsigned long long* stats;  // 0 samples, 1 rays, 2 overflow, 3 a chunk's queue length
   uint32_t flags;
 };
 
@@ -268,13 +268,17 @@ UBR_D AdjHit adjHit(const Params& p, const DScene& s, int px, int py, float2 hr)
 
 // The chunk's hit samples that need shading, with what their secondary rays
 // start from.  With `all` every hit sample (the forward pass of the gamma
-// derivative), else those whose gradient is not zero.
+// derivative), else those whose gradient is not zero.  BACKGROUND: the others
+// too, as k_adj_background<true> does in a launch of its own (4 us of a small
+// frame's 60, and the hits are read once).
+template <bool BACKGROUND>
 __global__ void __launch_bounds__(128) k_adj_surface(Params p, DScene s, AdjBufs b, AdjRays r, uint32_t i0, uint32_t n,
                                                      int all) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   bool take = false;
-  uint32_t i = 0;
+  uint32_t i = 0, used = 0;
   AdjHit h;
+  float4 bg = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (k < n) {
     i = tiledPixel(i0 + k, uint32_t(p.W), uint32_t(p.H));
     const int px = int(i % uint32_t(p.W)), py = int(i / uint32_t(p.W));
@@ -284,7 +288,16 @@ __global__ void __launch_bounds__(128) k_adj_surface(Params p, DScene s, AdjBufs
       float4 g;
       take = all || sampleGradient(p, b, i, px, py, ref, g);
       if (take) h = adjHit(p, s, px, py, hr);
+    } else if (BACKGROUND) {
+      used = sampleGradient(p, b, i, px, py, kInvalid, bg) ? 1 : 0;
+      if (!used) bg = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
+  }
+  if (BACKGROUND) {
+    const float cov = p.transparentBg ? 0.0f : 1.0f;
+    const float G[3] = {bg.x * cov, bg.y * cov, bg.z * cov};
+    addGlobals<3>(b.gGlobal + gBg, G);
+    warpCount(&b.stats[0], used);
   }
   int off;
   const int q = warpPushBase(take, r.count, off) + off;
@@ -797,11 +810,11 @@ __global__ void k_adj_down(Params p, const float4* colorHi, float4* out, uint32_
   out[o] = make_float4(a[0] * inv, a[1] * inv, a[2] * inv, a[3] * inv);
 }
 
-// Workspace of a chunk of pixels: a counter and kAdjArrays arrays of queue and
-// ray results, at most kAdjBytes of them.  They start on a block of the memory,
+// Workspace of a chunk of pixels: kAdjArrays arrays of queue and ray
+// results, at most kAdjBytes of them.  They start on a block of the memory,
 // or on a float4 where an arena cap leaves room for a few pixels only.
-constexpr size_t kAdjAlign = 256, kAdjArrays = 7, kAdjBytes = size_t(256) << 20;
-constexpr size_t adjHeader(size_t align) { return (kAdjArrays + 1) * align; }
+constexpr size_t kAdjAlign = 256, kAdjArrays = 6, kAdjBytes = size_t(256) << 20;
+constexpr size_t adjHeader(size_t align) { return kAdjArrays * align; }
 size_t adjAlign(size_t wsBytes, size_t pixBytes) {
   return wsBytes >= adjHeader(kAdjAlign) + 32 * pixBytes ? kAdjAlign : 16;
 }
@@ -931,7 +944,7 @@ ubr_status adjoint(Context* c, const Scene* sc, const ubr_render_desc& d, const 
   // pixels per chunk: what the workspace's queue and ray results hold
   const uint32_t S = uint32_t(p.aoSamples), nL = uint32_t(p.nLights);
   const size_t align = adjAlign(wsBytes, pixBytes);
-  char* at = static_cast<char*>(ws) + align;
+  char* at = static_cast<char*>(ws);
   auto take = [&](size_t n) {
     char* q = at;
     at += (n + align - 1) / align * align;
@@ -939,7 +952,8 @@ ubr_status adjoint(Context* c, const Scene* sc, const ubr_render_desc& d, const 
   };
   const uint32_t chunk = uint32_t(std::min<size_t>(npix, (wsBytes - adjHeader(align)) / pixBytes));
   AdjRays r{};
-  r.count = static_cast<uint32_t*>(ws);
+  r.count = reinterpret_cast<uint32_t*>(stats + 3);  // cleared with the counters
+  bool cleared = true;
   r.pix = reinterpret_cast<uint32_t*>(take(size_t(chunk) * 4));
   r.a = reinterpret_cast<float4*>(take(size_t(chunk) * 16));
   r.b = reinterpret_cast<float4*>(take(size_t(chunk) * 16));
@@ -948,8 +962,11 @@ ubr_status adjoint(Context* c, const Scene* sc, const ubr_render_desc& d, const 
   r.shadow = reinterpret_cast<uint8_t*>(take(size_t(chunk) * nL));
   const uint64_t raysPer = uint64_t(S) + (p.shadowsActive ? nL : 0u);
   auto traceChunk = [&](uint32_t i0, uint32_t n, bool all) -> ubr_status {
-    UBR_CUDA(c, cudaMemsetAsync(r.count, 0, sizeof(uint32_t), s));
-    k_adj_surface<<<(n + TB - 1) / TB, TB, 0, s>>>(p, sc->view, b, r, i0, n, all ? 1 : 0);
+    if (!cleared) UBR_CUDA(c, cudaMemsetAsync(r.count, 0, sizeof(uint32_t), s));
+    cleared = false;
+    const uint32_t gs = (n + TB - 1) / TB;
+    if (needFwd) k_adj_surface<false><<<gs, TB, 0, s>>>(p, sc->view, b, r, i0, n, all ? 1 : 0);
+    else k_adj_surface<true><<<gs, TB, 0, s>>>(p, sc->view, b, r, i0, n, all ? 1 : 0);
     const uint32_t g = uint32_t((uint64_t(n) * raysPer + TB - 1) / TB);
     if (g > 0) {
       if (p.aoEnhanced) k_adj_rays<true><<<g, TB, 0, s>>>(p, sc->view, b, r);
@@ -968,7 +985,7 @@ ubr_status adjoint(Context* c, const Scene* sc, const ubr_render_desc& d, const 
     traced = chunk >= npix;
     k_adj_down<<<(nout + 255) / 256, 256, 0, s>>>(p, colorHi, outFwd, nout);
   }
-  k_adj_background<true><<<grid, TB, 0, s>>>(p, b, npix);
+  if (needFwd) k_adj_background<true><<<grid, TB, 0, s>>>(p, b, npix);
   for (uint32_t i0 = 0; i0 < npix; i0 += chunk) {
     const uint32_t n = std::min(chunk, npix - i0);
     if (!traced && (st = traceChunk(i0, n, false)) != UBR_OK) return st;
