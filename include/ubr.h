@@ -402,8 +402,9 @@ typedef struct ubr_context_desc {
   uint32_t abi_version;
   int32_t device;              /* CUDA ordinal */
   /* 0 = grow on demand; > 0 = hard cap on the bytes of scenes and scratch.  GI
-   * gathers and adjoints run in chunks of what it leaves; the least they need is
-   * one warp of samples (3 to 15 KB) and one pixel (0.2 KB and 8 B per AO ray) */
+   * gathers of more than 1024 samples and adjoints run in chunks of what it
+   * leaves; the least they need is one warp of samples (3 to 15 KB) and one pixel
+   * (0.2 KB and 8 B per AO ray) */
   uint64_t arena_bytes;
   void* stream;                /* cudaStream_t to run on, NULL = own stream */
   /* BVH tuning (0 = library default): the most primitives a wide-BVH leaf

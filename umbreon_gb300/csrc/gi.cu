@@ -9,10 +9,10 @@
 // and glossy reflection, variance-adaptive spp, ReSTIR spatial rounds
 // (integrator/pt2/pt2_reservoir.hpp, pt2_spatial.hpp).
 //
-// The gather is a wavefront of kernels over the samples of many points; every
-// stream is a pure function of (grid index, sample index, pt1Seed), as in the
-// reference, so the oracle draws the same samples and the frames agree up to
-// traversal float order.
+// The gather is a wavefront of kernels over the samples of many points, or one
+// kernel for few; every stream is a pure function of (grid index, sample index,
+// pt1Seed), as in the reference, so the oracle draws the same samples and the
+// frames agree up to traversal float order.
 #include <algorithm>
 
 #include <cub/device/device_select.cuh>
@@ -428,8 +428,9 @@ UBR_D uint32_t tilePixel4(uint32_t i, uint32_t W, uint32_t H) {
 //   k_gather_next     one thread per path of a later bounce: closest hit
 //   k_gather_emit     (emitters) one thread per sample: emissive NEE
 //   k_gather_sum      the samples of a point, summed
-// One kernel that walks a path from its draw to its last shadow ray was bound
-// by instruction fetch (closest-hit and any-hit traversal, four intersectors
+// and, for few samples, in one kernel (k_gather_whole, giGatherWhole).
+// At many samples one kernel that walks a path from its draw to its last shadow
+// ray is bound by instruction fetch (closest-hit and any-hit traversal, four intersectors
 // and the shading in one loop: 5 stalls on a missing instruction per issue)
 // with 6.5 of 32 lanes active (a lane's shadow rays waited for the others'
 // closest hits) and spilled 780 B per thread at 64 registers.  At the pt2
